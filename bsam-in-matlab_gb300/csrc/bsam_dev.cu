@@ -233,15 +233,34 @@ Fields fields(bsam_hier h) {
   return f;
 }
 
+// how to divide by the constant d (DivC).  elo and espan: x, its quotient
+// and the remainder of the correction step (53 binary digits below x) all
+// stay normal, with a margin of two.
+DivC div_const(double d) {
+  DivC c;
+  c.d = d;
+  c.r = 1.0 / d;
+  int e;
+  const double m = std::frexp(d, &e);
+  const double rel = std::fabs(std::fma(c.r, d, -1.0));   // exact: |r d - 1| is below an ulp
+  c.ops = m == 0.5 ? 1 : rel < std::ldexp(1.0, -54) ? 3 : 5;
+  // biased exponents; the quotient's is x's minus (e - 1), give or take one
+  const int lo = std::max(57, 3 + (e - 1)), hi = std::min(2044, 2044 + (e - 1));
+  c.elo = (unsigned)lo;
+  c.espan = (unsigned)std::max(hi - lo, 0);
+  if ((e - 1 > 1000 || e - 1 < -1000) && c.ops != 1) c.elo = 2048, c.espan = 0;   // always divide
+  return c;
+}
+
 LevelD leveld(bsam_hier h, int k) {
   const LevelPlan &L = h->lev[k];
   LevelD d;
   d.patches = h->patches.p + L.p0;
   d.hx = L.hx; d.hy = L.hy;
-  d.hx2 = L.hx * L.hx; d.hy2 = L.hy * L.hy;
-  d.ihx2 = 1.0 / d.hx2; d.ihy2 = 1.0 / d.hy2;
   d.pow2 = L.pow2 ? 1 : 0;
-  d.fhx = (float)d.hx; d.fhy = (float)d.hy; d.fhx2 = (float)d.hx2; d.fhy2 = (float)d.hy2;
+  d.dx = div_const(L.hx * L.hx); d.dy = div_const(L.hy * L.hy);
+  d.fhx = (float)d.hx; d.fhy = (float)d.hy;
+  d.fhx2 = (float)(L.hx * L.hx); d.fhy2 = (float)(L.hy * L.hy);
   return d;
 }
 

@@ -88,19 +88,59 @@ struct Decomp {
   int n, nblocks;
 };
 
+// Division by a level's constant h^2, correctly rounded without a divide: a
+// double division is a chain of about nine dependent FP64 operations (556
+// cycles on GB300, one operation takes 64).  r = RN(1/d) comes from the host.
+// ops 1: d is a power of two, x r is exact.  ops 3: q = RN(x r), then
+// RN(q + r RN(x - q d)), the last two fused -- the quotient step of Markstein
+// (IBM J. Res. Dev. 34, 1990): correctly rounded if r is the correctly
+// rounded reciprocal and q is within an ulp, which holds while |r d - 1| is
+// below a quarter ulp of 1 (the host checks it per constant).  ops 5: the step
+// twice; the first brings q within an ulp for any d.  Outside the exponent
+// range [elo, elo + espan] an intermediate could leave the normal range: a
+// true division there, and the signed zero of the first product for x = 0.
+// A colour pass of a 15 x 11-based ragged level (660 cells): 4.1 us with
+// divisions, 3.6 with this; the three-level ragged solve 4.23 -> 3.95 ms.
+struct DivC {
+  double d, r;
+  int ops;
+  unsigned elo, espan;
+};
+
+__device__ __forceinline__ unsigned exp_bits(double x) { return ((unsigned)__double2hiint(x) >> 20) & 0x7ffu; }
+__device__ __forceinline__ bool is_zero(double x) {
+  return (((unsigned)__double2hiint(x) << 1) | (unsigned)__double2loint(x)) == 0u;
+}
+
+__device__ __forceinline__ double div_c(double x, const DivC &D) {
+  const double q0 = x * D.r;
+  if (D.ops == 1) return q0;
+  double q = __fma_rn(__fma_rn(-q0, D.d, x), D.r, q0);
+  if (D.ops == 5) q = __fma_rn(__fma_rn(-q, D.d, x), D.r, q);
+  if (exp_bits(x) - D.elo > D.espan) q = is_zero(x) ? q0 : x / D.d;
+  return q;
+}
+// FP32: a divide is short there (with the steps above the ragged mixed solve
+// was 2% slower)
+__device__ __forceinline__ float div_c(float x, float d) { return x / d; }
+
 struct LevelD {
   const PatchD *patches;       // this level's patches
-  double hx, hy, hx2, hy2, ihx2, ihy2;   // ihx2 = 1/hx2 (used only when exact)
+  double hx, hy;
+  DivC dx, dy;                 // division by hx^2, hy^2
   int pow2;                    // hx2 and hy2 are powers of two
   float fhx, fhy, fhx2, fhy2;  // FP32 copies for the correction cycle
 };
 
 // the level's cell sizes in the cycle's value type
-template <class T> struct LevelH {
-  T hx, hy, hx2, hy2;
+template <class T, class D2> struct LevelH {
+  T hx, hy;
+  D2 dx, dy;                   // what div_c divides by
 };
-__device__ __forceinline__ LevelH<double> level_h(const LevelD &L, double) { return {L.hx, L.hy, L.hx2, L.hy2}; }
-__device__ __forceinline__ LevelH<float> level_h(const LevelD &L, float) { return {L.fhx, L.fhy, L.fhx2, L.fhy2}; }
+__device__ __forceinline__ LevelH<double, DivC> level_h(const LevelD &L, double) { return {L.hx, L.hy, L.dx, L.dy}; }
+__device__ __forceinline__ LevelH<float, float> level_h(const LevelD &L, float) {
+  return {L.fhx, L.fhy, L.fhx2, L.fhy2};
+}
 
 // `b` is the block index within the decomposition
 __device__ __forceinline__ int find_patch(const Decomp &D, int b, int g) {
@@ -109,15 +149,20 @@ __device__ __forceinline__ int find_patch(const Decomp &D, int b, int g) {
   return p;
 }
 
-__device__ __forceinline__ double divr(double x, double h2, double ih2, int pow2) {
-  return pow2 ? x * ih2 : x / h2;
+// op2d (ebKernels.m:13-25) at one cell from its values and coefficients
+__device__ __forceinline__ double op_pre(double q, double qe, double qw, double qn, double qs, double dE, double dW,
+                                         double dN, double dS, double cc, const LevelD &L) {
+  const double feE = dE * (qe - q), feW = dW * (q - qw), fnN = dN * (qn - q), fnS = dS * (q - qs);
+  return (div_c(-(feE - feW), L.dx) - div_c(fnN - fnS, L.dy)) + cc * q;
 }
 
+// the same at interior cell (li, lj) of a padded array
 __device__ __forceinline__ double op_cell_r(const double *__restrict__ Qa, int ldq, const double *__restrict__ DeW,
                                             const double *__restrict__ DnS, double cc, int mx, int li, int lj,
                                             const LevelD &L) {
-  return L.pow2 ? op_cell<true>(Qa, ldq, DeW, DnS, cc, mx, li, lj, L.hx2, L.hy2, L.ihx2, L.ihy2)
-                : op_cell<false>(Qa, ldq, DeW, DnS, cc, mx, li, lj, L.hx2, L.hy2, L.ihx2, L.ihy2);
+  const int c = (li + 1) + (lj + 1) * ldq;
+  return op_pre(Qa[c], Qa[c + 1], Qa[c - 1], Qa[c + ldq], Qa[c - ldq], DeW[(li + 1) + lj * (mx + 1)],
+                DeW[li + lj * (mx + 1)], DnS[li + (lj + 1) * mx], DnS[li + lj * mx], cc, L);
 }
 
 // ---------------------------------------------------------------------------
@@ -555,7 +600,7 @@ __device__ __forceinline__ void cell_update(const LevelD &L, const FieldsT<T> &f
                                             T omega, int unit_omega, const CellState<T> &S) {
   if (!S.live) return;
   const T c83 = T(8.0 / 3.0), c13 = T(1.0 / 3.0);
-  const LevelH<T> H = level_h(L, T(0));
+  const auto H = level_h(L, T(0));
   const int c = S.c, ldq = S.ldq;
   const int kx = S.code & 3, ky = (S.code >> 2) & 3, sx = (S.code >> 4) & 1, sy = (S.code >> 5) & 1;
   T *__restrict__ Q = f.Q + S.q_off;
@@ -601,10 +646,10 @@ __device__ __forceinline__ void cell_update(const LevelD &L, const FieldsT<T> &f
     t = t + qn * S.dN;
     t = t + qs * S.dS;
   } else {
-    t = t + (qe * S.dE) / H.hx2;
-    t = t + (qw * S.dW) / H.hx2;
-    t = t + (qn * S.dN) / H.hy2;
-    t = t + (qs * S.dS) / H.hy2;
+    t = t + div_c(qe * S.dE, H.dx);
+    t = t + div_c(qw * S.dW, H.dx);
+    t = t + div_c(qn * S.dN, H.dy);
+    t = t + div_c(qs * S.dS, H.dy);
   }
   t = t * S.idg;
   if (unit_omega) Q[c] = t;
@@ -731,7 +776,7 @@ __global__ void __launch_bounds__(kBlock) k_relax_n(LevelD L, const RelaxChunkD 
   }
   chain_wait();
   const T c83 = T(8.0 / 3.0), c13 = T(1.0 / 3.0);
-  const LevelH<T> H = level_h(L, T(0));
+  const auto H = level_h(L, T(0));
   T *__restrict__ Q = f.Q + R.q_off;
   T qe[kN], qw[kN], qn[kN], qs[kN], fv[kN], qc[kN];
 #pragma unroll
@@ -773,10 +818,10 @@ __global__ void __launch_bounds__(kBlock) k_relax_n(LevelD L, const RelaxChunkD 
       t = t + qn[u] * dN[u];
       t = t + qs[u] * dS[u];
     } else {
-      t = t + (qe[u] * dE[u]) / H.hx2;
-      t = t + (qw[u] * dW[u]) / H.hx2;
-      t = t + (qn[u] * dN[u]) / H.hy2;
-      t = t + (qs[u] * dS[u]) / H.hy2;
+      t = t + div_c(qe[u] * dE[u], H.dx);
+      t = t + div_c(qw[u] * dW[u], H.dx);
+      t = t + div_c(qn[u] * dN[u], H.dy);
+      t = t + div_c(qs[u] * dS[u], H.dy);
     }
     t = t * idg[u];
     if (unit_omega) Q[c[u]] = t;
@@ -974,7 +1019,7 @@ __device__ __forceinline__ void dsm_cell_update(const LevelD &L, const FieldsT<T
                                                 const T *ov, const DsmRange<T> &D) {
   if (!X.live) return;
   const T c83 = T(8.0 / 3.0), c13 = T(1.0 / 3.0);
-  const LevelH<T> H = level_h(L, T(0));
+  const auto H = level_h(L, T(0));
   const int ldq = X.ldq, c = X.c;
   int kx = X.code & 3, ky = (X.code >> 2) & 3;
   const int sx = (X.code >> 4) & 1, sy = (X.code >> 5) & 1;
@@ -1011,10 +1056,10 @@ __device__ __forceinline__ void dsm_cell_update(const LevelD &L, const FieldsT<T
     t = t + qn * X.dN;
     t = t + qs * X.dS;
   } else {
-    t = t + (qe * X.dE) / H.hx2;
-    t = t + (qw * X.dW) / H.hx2;
-    t = t + (qn * X.dN) / H.hy2;
-    t = t + (qs * X.dS) / H.hy2;
+    t = t + div_c(qe * X.dE, H.dx);
+    t = t + div_c(qw * X.dW, H.dx);
+    t = t + div_c(qn * X.dN, H.dy);
+    t = t + div_c(qs * X.dS, H.dy);
   }
   t = t * X.idg;
   const uint32_t ac = dsm_addr(D, c);
@@ -1227,8 +1272,8 @@ __global__ void __launch_bounds__(kT) k_restrict_fill(LevelD L, Decomp D, Fields
 // The arithmetic is FP64 for either value type (the reflux of the mixed
 // form stays FP64).
 template <class T>
-__device__ __forceinline__ double face_corr(const PatchD &P, const FieldsT<T> &f, int fc, int j, double hc2,
-                                            double ihc2, int pow2, bool qc_inner) {
+__device__ __forceinline__ double face_corr(const PatchD &P, const FieldsT<T> &f, int fc, int j,
+                                            const DivC &hc2, bool qc_inner) {
   const int mx = P.mx, my = P.my, cmx = mx >> 1, cmy = my >> 1;
   const int ldq = mx + 2, ldc = cmx + 2;
   const T *Q = f.Q + P.q_off, *QC = f.QC + P.qc_off;
@@ -1273,7 +1318,7 @@ __device__ __forceinline__ double face_corr(const PatchD &P, const FieldsT<T> &f
       break;
     }
   }
-  return divr(v, hc2, ihc2, pow2);
+  return div_c(v, hc2);
 }
 
 // gather-form corrections of one target coarse cell: contributions in the
@@ -1288,8 +1333,7 @@ __device__ __forceinline__ double add_corrections(double v, const CorrCSR &C, in
   for (int i = C.beg[t]; i < C.beg[t + 1]; ++i) {
     const int it = C.item[i];
     const int fc = it & 3;
-    v = v + face_corr(Lf.patches[it >> 2], f, fc, C.jj[i], fc < 2 ? Lc.hx2 : Lc.hy2, fc < 2 ? Lc.ihx2 : Lc.ihy2,
-                      Lc.pow2, qc_inner);
+    v = v + face_corr(Lf.patches[it >> 2], f, fc, C.jj[i], fc < 2 ? Lc.dx : Lc.dy, qc_inner);
   }
   return v;
 }
@@ -1305,14 +1349,6 @@ __device__ __forceinline__ double add_corrections(double v, const CorrCSR &C, in
 //   [.., +nb_tgt)           F_target = F_target + corrections (ebCoarseLoad.m:37-45)
 // QC ring values are read from the parent's Q through the window table, so
 // the three ranges are independent.
-// op2d at one cell from preloaded face coefficients (same operation order
-// as op_cell)
-__device__ __forceinline__ double op_pre(double q, double qe, double qw, double qn, double qs, double dE, double dW,
-                                         double dN, double dS, double cc, const LevelD &L) {
-  const double feE = dE * (qe - q), feW = dW * (q - qw), fnN = dN * (qn - q), fnS = dS * (q - qs);
-  return (divr(-(feE - feW), L.hx2, L.ihx2, L.pow2) - divr(fnN - fnS, L.hy2, L.ihy2, L.pow2)) + cc * q;
-}
-
 // the three item kinds of the coarse load (kChain as restrict_item)
 template <class T, bool kChain>
 __device__ __forceinline__ void load_ring_item(const FieldsT<T> &f, const int *__restrict__ ring,
