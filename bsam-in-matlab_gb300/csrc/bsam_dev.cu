@@ -190,6 +190,9 @@ struct bsam_hier_s {
   DBuf<InstRes> instres;           // per-instance residual reduction plan
   DBuf<SlotRange> sranges;
   DBuf<CoarsestD> coarsest;        // one coarsest operator per instance
+  bool all_pow2 = false;           // every level's h^2 is a power of two
+  int nres = 0;                    // residual tasks; rtasks' rest refreshes QC
+  DBuf<unsigned long long> norms;  // per instance: max |r|, max |FTrue| as bit patterns
   int nrtasks = 0, nslots = 0, npartials = 0, hist_stride = 0;
   ResAcc *acc_host = nullptr;      // ninst entries (pageable: freeing pinned memory synchronises the device)
   int *active_host = nullptr;      // ninst entries
@@ -243,12 +246,13 @@ DivC div_const(double d) {
   int e;
   const double m = std::frexp(d, &e);
   const double rel = std::fabs(std::fma(c.r, d, -1.0));   // exact: |r d - 1| is below an ulp
+  c.kexp = (1 - e) * (1 << 20);
   c.ops = m == 0.5 ? 1 : rel < std::ldexp(1.0, -54) ? 3 : 5;
   // biased exponents; the quotient's is x's minus (e - 1), give or take one
   const int lo = std::max(57, 3 + (e - 1)), hi = std::min(2044, 2044 + (e - 1));
   c.elo = (unsigned)lo;
   c.espan = (unsigned)std::max(hi - lo, 0);
-  if ((e - 1 > 1000 || e - 1 < -1000) && c.ops != 1) c.elo = 2048, c.espan = 0;   // always divide
+  if (e - 1 > 1000 || e - 1 < -1000) c.elo = 2048, c.espan = 0;   // always divide
   return c;
 }
 
@@ -710,13 +714,19 @@ void launch_coarse_load(bsam_hier h, int k) {
   const int ntgt = h->opts.mass_correction ? L.ct_n : 0;
   Launch l(h, K_LOAD, 50.0 * tscale<T>() * (double)L.ncells, k);
   const int *ri = (const int *)(h->ninst > 1 ? h->ring_inst.p : nullptr);
-  if (D.nblocks < spread_limit(h)) {   // spread the footprint's FP64 work over more SMs
-    auto nb = [](int n) { return (n + 63) / 64; };
-    launch_k(h, k_load<T, 64>, nb(L.ring_n) + nb(D.n) + nb(ntgt), 64, leveld(h, k), leveld(h, k - 1), D,
-             fields_t<T>(h), (const int *)h->ring.p, ri, L.ring_off, L.ring_n, corr_csr(h, L), ntgt);
+  const bool spread = D.nblocks < spread_limit(h);   // the footprint's FP64 work over more SMs
+  const int kt = spread ? 64 : kBlock;
+  auto nb = [&](int n) { return (n + kt - 1) / kt; };
+  auto go = [&](auto kern) {
+    launch_k(h, kern, nb(L.ring_n) + nb(D.n) + nb(ntgt), kt, leveld(h, k), leveld(h, k - 1), D, fields_t<T>(h),
+             (const int *)h->ring.p, ri, L.ring_off, L.ring_n, corr_csr(h, L), ntgt);
+  };
+  if (L.pow2 && h->lev[k - 1].pow2) {
+    if (spread) go(k_load<T, true, 64>);
+    else go(k_load<T, true>);
   } else {
-    launch_k(h, k_load<T>, nblk(L.ring_n) + D.nblocks + nblk(ntgt), kBlock, leveld(h, k), leveld(h, k - 1), D,
-             fields_t<T>(h), (const int *)h->ring.p, ri, L.ring_off, L.ring_n, corr_csr(h, L), ntgt);
+    if (spread) go(k_load<T, false, 64>);
+    else go(k_load<T, false>);
   }
 }
 
@@ -843,29 +853,68 @@ void launch_filldown(bsam_hier h, bool top_fill = false) {
 
 bool mixed(bsam_hier h) { return h->opts.precision == 1; }
 
+// the WHILE / IF conditions that the end of a residual sets (none outside
+// graphs)
+struct LoopCond {
+  cudaGraphConditionalHandle c0 = 0, c1 = 0;
+  int n = 0;
+};
+
+// QC's ring and interior as the reference's residual leaves them
+void launch_qc_refresh(bsam_hier h) {
+  const int n = h->nrtasks - h->nres;
+  if (n <= 0 || !h->opts.mass_correction) return;
+  h->launch_count++;
+  k_qc_refresh<<<(unsigned)((n + kBlock / 32 - 1) / (kBlock / 32)), kBlock, 0, h->stream>>>(
+      h->patches.p, h->rtasks.p + h->nres, n, fields(h), h->ring.p);
+}
+
 // ebCompResidual (ebCompResidual.m:15-85): one launch over every level of
-// every instance, then the per-instance reduction and stop test (mode 0:
-// before the first V-cycle, 1: after one, 2: report only).  The mixed form
-// also stores r (FP32) as the right-hand side of the next correction cycle.
-void launch_residual(bsam_hier h, int mode) {
+// every instance, then the per-instance end: RES_START before the first
+// V-cycle (norms of r and of the source), RES_STEP after one, RES_REPORT an
+// eager call (L2 too, QC refreshed), RES_RHS only r itself, the right-hand
+// side of the mixed form's next correction cycle (stored as FP32 by every
+// mode of that form).
+enum { RES_START = 0, RES_STEP = 1, RES_REPORT = 2, RES_RHS = 3 };
+
+void launch_residual(bsam_hier h, int mode, const LoopCond &c = LoopCond()) {
   double bytes = 0;
   for (int k = 1; k <= h->nlev; ++k) bytes += 41.0 * (double)h->lev[k].ncells;
+  float *rout = mixed(h) ? h->F32.p : (float *)nullptr;
+  if (mode == RES_START) cudaMemsetAsync(h->norms.p, 0, sizeof(unsigned long long) * h->norms.n, h->stream);
   {
     Launch l(h, K_RESID, bytes);
-    const int g256 = (h->nrtasks + kBlock / 32 - 1) / (kBlock / 32);
-    if (g256 < spread_limit(h))
-      launch_k(h, k_residual<64>, (h->nrtasks + 1) / 2, 64, (const LevelX *)h->levelx.p, (const PatchD *)h->patches.p,
-               (const ResTask *)h->rtasks.p, h->nrtasks, fields(h), (const int *)h->ring.p, h->slots.p, h->nslots,
-               h->opts.mass_correction, mixed(h) ? h->F32.p : (float *)nullptr);
-    else
-      launch_k(h, k_residual<>, g256, kBlock, (const LevelX *)h->levelx.p, (const PatchD *)h->patches.p,
-               (const ResTask *)h->rtasks.p, h->nrtasks, fields(h), (const int *)h->ring.p, h->slots.p, h->nslots,
-               h->opts.mass_correction, mixed(h) ? h->F32.p : (float *)nullptr);
+    const int g256 = (h->nres + kBlock / 32 - 1) / (kBlock / 32);
+    unsigned long long *nm = mode == RES_RHS ? nullptr : h->norms.p;
+    auto go = [&](auto kern, int grid, int block) {
+      launch_k(h, kern, grid, block, (const LevelX *)h->levelx.p, (const PatchD *)h->patches.p,
+               (const ResTask *)h->rtasks.p, h->nres, fields(h), h->slots.p, h->nslots, nm,
+               mode == RES_START ? 1 : 0, h->opts.mass_correction, rout);
+    };
+    const bool small = g256 < spread_limit(h);
+    const int g64 = (h->nres + 1) / 2;
+    if (mode == RES_REPORT) {
+      if (small) go(k_residual<true, false, 64>, g64, 64);
+      else go(k_residual<true, false>, g256, kBlock);
+    } else if (h->all_pow2) {
+      if (small) go(k_residual<false, true, 64>, g64, 64);
+      else go(k_residual<false, true>, g256, kBlock);
+    } else {
+      if (small) go(k_residual<false, false, 64>, g64, 64);
+      else go(k_residual<false, false>, g256, kBlock);
+    }
   }
+  if (mode == RES_RHS) return;
   Launch l(h, K_RESID, 0);
-  launch_k(h, k_residual_final, h->ninst, kFinal, (const InstRes *)h->instres.p, (const SlotRange *)h->sranges.p,
-           (const double *)h->slots.p, h->nslots, h->acc.p, h->active.p, h->iters.p, h->hist.p, h->hist_stride, mode,
-           (const int *)h->crange.p, h->nlev, h->act_mode == kActChunk ? h->cact.p : nullptr);
+  if (mode == RES_REPORT) {
+    launch_k(h, k_residual_final, h->ninst, kFinal, (const InstRes *)h->instres.p, (const SlotRange *)h->sranges.p,
+             (const double *)h->slots.p, h->nslots, h->acc.p);
+    launch_qc_refresh(h);
+  } else {
+    launch_k(h, k_solve_step, 1, kStep, (const InstRes *)h->instres.p, h->ninst, h->norms.p, h->acc.p, h->active.p,
+             h->iters.p, h->hist.p, h->hist_stride, mode, (const int *)h->crange.p, h->nlev,
+             h->act_mode == kActChunk ? h->cact.p : nullptr, c.c0, c.c1, c.n);
+  }
 }
 
 // Ghost fills of several levels in one launch (k_ghost_spans); `lv` lists
@@ -970,7 +1019,7 @@ void reset_force(bsam_hier h) {
 // residual, Q += E in FP64, restriction and ghost fill in FP64, FP64
 // residual.  The FP64 body expects F = FTrue off the footprints
 // (reset_force before the first iteration).
-int launch_iteration(bsam_hier h, int mode) {
+int launch_iteration(bsam_hier h, int mode, const LoopCond &cond = LoopCond()) {
   if (mixed(h)) {
     CK(cudaMemsetAsync(h->E.p, 0, sizeof(float) * h->E.n, h->stream));
     // the finest level's closing fill of E is left out: nothing reads the
@@ -998,7 +1047,7 @@ int launch_iteration(bsam_hier h, int mode) {
                (const int *)h->active.p);
     }
     launch_consistent(h, fold);
-    launch_residual(h, mode);
+    launch_residual(h, mode, cond);
     CK(cudaGetLastError());
     return BSAM_OK;
   }
@@ -1007,7 +1056,7 @@ int launch_iteration(bsam_hier h, int mode) {
                    (h->opts.npost <= 0 || relax_form<double>(h, h->nlev) != 0);
   launch_vcycle(h, h->nlev, top);
   launch_filldown(h, top);
-  launch_residual(h, mode);
+  launch_residual(h, mode, cond);
   CK(cudaGetLastError());
   return BSAM_OK;
 }
@@ -1206,7 +1255,7 @@ int build_graph(bsam_hier h) {
   if (h->gexec) return BSAM_OK;
   CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
   const int64_t before = h->launch_count;
-  int rc = launch_iteration(h, 1);
+  int rc = launch_iteration(h, RES_STEP);
   cudaGraph_t g = nullptr;
   cudaError_t e = cudaStreamEndCapture(h->stream, &g);
   if (rc) return rc;
@@ -1244,7 +1293,7 @@ bool host_loop() {
 }
 
 // ebSolveCycles' loop as one graph: a conditional WHILE node whose body is
-// one iteration followed by k_any_active, which sets the condition from the
+// one iteration, whose last kernel (k_solve_step) sets the condition from the
 // instances' stop tests.  A solve is then one graph launch and one read of
 // the results, with no host round trip per V-cycle.  Returns false (and the
 // per-iteration graph is used) when the runtime cannot build it.
@@ -1271,9 +1320,8 @@ bool build_while_graph(bsam_hier h) {
          cudaSuccess;
     if (ok) {
       const int64_t before = h->launch_count;
-      const int rc = launch_iteration(h, 1);
+      const int rc = launch_iteration(h, RES_STEP, LoopCond{cond, cond, 1});
       h->kernels_per_cycle = h->launch_count - before;
-      launch_k(h, k_any_active, 1, kBlock, (const int *)h->active.p, h->ninst, cond, cond, 0);
       cudaGraph_t out = nullptr;
       ok = cudaStreamEndCapture(h->stream, &out) == cudaSuccess && rc == BSAM_OK;
       h->launch_count = before;
@@ -1354,21 +1402,19 @@ bool build_solve_graph(bsam_hier h) {
     if (ok) {
       if (!mixed(h)) reset_force(h);
       for (int k = 1; k <= h->nlev; ++k) launch_fill(h, k);
-      launch_residual(h, 0);
-      launch_k(h, k_any_active, 1, kBlock, (const int *)h->active.p, h->ninst, wcond, icond, mixed(h) ? 1 : 0);
+      launch_residual(h, RES_START, LoopCond{wcond, icond, mixed(h) ? 2 : 1});
       h->preamble_kernels = h->launch_count - before;
       if (mixed(h))
         ok = add_conditional(h, helper, icond, cudaGraphCondTypeIf, [h]() {
           launch_consistent(h);
-          launch_residual(h, 2);
+          launch_residual(h, RES_RHS);
           return cudaGetLastError() == cudaSuccess ? BSAM_OK : BSAM_ERR_CUDA;
         });
       if (ok)
         ok = add_conditional(h, helper, wcond, cudaGraphCondTypeWhile, [h, wcond]() {
-          const int rc = launch_iteration(h, 1);
-          launch_k(h, k_any_active, 1, kBlock, (const int *)h->active.p, h->ninst, wcond, wcond, 0);
-          return rc;
+          return launch_iteration(h, RES_STEP, LoopCond{wcond, wcond, 1});
         });
+      if (ok) launch_qc_refresh(h);
     }
     cudaGraph_t g = nullptr;
     const bool ended = cudaStreamEndCapture(h->stream, &g) == cudaSuccess;
@@ -1859,6 +1905,7 @@ int do_upload(bsam_hier h, const bsam_hier_desc *d) {
     L.hx = d->hs[2 * (k - 1)];
     L.hy = d->hs[2 * (k - 1) + 1];
     L.pow2 = is_pow2(L.hx * L.hx) && is_pow2(L.hy * L.hy);
+    h->all_pow2 = (k == 1 || h->all_pow2) && L.pow2;
     L.ncells = lv[LD_CELL1] - lv[LD_CELL0];
     L.col = B.make_decomp(L.p0, L.p1, 0);
     L.cell = B.make_decomp(L.p0, L.p1, 1);
@@ -1962,10 +2009,11 @@ int do_upload(bsam_hier h, const bsam_hier_desc *d) {
     h->relax_n[1].assign(d->nlev + 1, 1);
   }
   // residual plan: warp tasks, slots in instance order, level by level
-  constexpr int kTask = 32 * kResLane;
-  // (main cells, then the level's correction targets), then the QC refresh
-  // tasks of the levels above each instance's root
-  std::vector<ResTask> tasks;
+  // (main cells, then the level's correction targets); the targets' tasks,
+  // the longest, come first in the list; then the QC refresh tasks of the
+  // levels above each instance's root
+  constexpr int kTask = 128;
+  std::vector<ResTask> tasks, cells;
   std::vector<SlotRange> ranges;
   std::vector<InstRes> ir(h->ninst);
   h->inst_visible.assign(h->ninst, 0);
@@ -1978,9 +2026,9 @@ int do_upload(bsam_hier h, const bsam_hier_desc *d) {
       for (int p = L.p0; p < L.p1; ++p) {
         if (pinst[p] != i) continue;
         const int32_t *r = B.P(p);
-        const int n = r[PD_MX] * r[PD_MY];
+        const int n = r[PD_MX] * r[PD_MY], nc = r[PD_MX] * ((r[PD_MY] + kResRows - 1) / kResRows);
         for (int c = 0; c < n; ++c) h->inst_visible[i] += (d->covered[r[PD_COFF] + c] == 0);
-        for (int b0 = 0; b0 < n; b0 += kTask) tasks.push_back(ResTask{0, k, p, b0, std::min(kTask, n - b0), ns++, i, 0});
+        for (int b0 = 0; b0 < nc; b0 += 32) cells.push_back(ResTask{0, k, p, b0, std::min(32, nc - b0), ns++, i, 0});
       }
       if (k < d->nlev) {
         const LevelPlan &Lf = h->lev[k + 1];
@@ -1991,8 +2039,8 @@ int do_upload(bsam_hier h, const bsam_hier_desc *d) {
             if (t0 < 0) t0 = t;
             t1 = t + 1;
           }
-        for (int t = t0; t0 >= 0 && t < t1; t += kTask)
-          tasks.push_back(ResTask{1, k, 0, t, std::min(kTask, t1 - t), ns++, i, 0});
+        for (int t = t0; t0 >= 0 && t < t1; t += 32)
+          tasks.push_back(ResTask{1, k, 0, t, std::min(32, t1 - t), ns++, i, 0});
       }
       ranges.push_back(SlotRange{s0, ns, L.hx * L.hy});
     }
@@ -2002,6 +2050,8 @@ int do_upload(bsam_hier h, const bsam_hier_desc *d) {
     ir[i].rel_tol = h->opts.rel_tol;
     ir[i].ncell = (double)h->inst_visible[i];
   }
+  tasks.insert(tasks.end(), cells.begin(), cells.end());
+  h->nres = (int)tasks.size();
   for (int k = 2; k <= d->nlev; ++k) {
     const LevelPlan &L = h->lev[k];
     for (int p = L.p0; p < L.p1; ++p) {
@@ -2189,6 +2239,7 @@ int do_upload(bsam_hier h, const bsam_hier_desc *d) {
       (rc = h->rtasks.upload(tasks.data(), tasks.size(), s)) || (rc = h->sranges.upload(ranges.data(), ranges.size(), s)) ||
       (rc = h->instres.upload(ir.data(), ir.size(), s)) || (rc = h->coarsest.upload(cds.data(), cds.size(), s)) ||
       (rc = h->slots.alloc(3 * (size_t)h->nslots)) || (rc = h->acc.alloc(h->ninst)) ||
+      (rc = h->norms.alloc(2 * (size_t)h->ninst)) ||
       (rc = h->iters.alloc(h->ninst)) ||
       (rc = h->hist.alloc((size_t)h->ninst * h->hist_stride)))
     return rc;
@@ -2241,6 +2292,7 @@ void release(bsam_hier h) {
   h->flags.release(); h->g_type.release(); h->patches.release(); h->acc.release(); h->perim.release();
   h->rchunks.release(); h->pchunks.release(); h->cact.release(); h->crange.release(); h->levelx.release(); h->rtasks.release(); h->instres.release(); h->sranges.release();
   h->coarsest.release();
+  h->norms.release();
   h->ga_rt.release();
   delete[] h->acc_host;
   delete[] h->active_host;
@@ -2502,7 +2554,7 @@ int bsam_comp_residual(bsam_hier h, double out[5]) {
   if (!h || !out) return fail(BSAM_ERR_ARG, "null argument");
   int rc = set_device(h);
   if (rc) return rc;
-  launch_residual(h, 2);
+  launch_residual(h, RES_REPORT);
   CK(cudaGetLastError());
   return read_residual(h, out);
 }
@@ -2652,11 +2704,11 @@ int bsam_vcycle(bsam_hier h) {
   if (rc || (rc = ensure_f32(h))) return rc;
   if (mixed(h)) {   // the correction cycle's right-hand side
     launch_consistent(h);
-    launch_residual(h, 2);
+    launch_residual(h, RES_RHS);
   } else {
     reset_force(h);
   }
-  if ((rc = launch_iteration(h, 2))) return rc;
+  if ((rc = launch_iteration(h, RES_REPORT))) return rc;
   CK(cudaStreamSynchronize(h->stream));
   return BSAM_OK;
 }
@@ -2682,14 +2734,14 @@ int bsam_solve_cycles(bsam_hier h, double *res_hist, int hist_cap, int *vcycles,
   }
   if (!mixed(h)) reset_force(h);
   for (int k = 1; k <= h->nlev; ++k) launch_fill(h, k);
-  launch_residual(h, 0);
+  launch_residual(h, RES_START);
   CK(cudaGetLastError());
   if ((rc = read_state(h, &nactive))) return rc;
   if (nactive && mixed(h)) {
     // the history starts with the reference's own initial residual; the
     // first correction's right-hand side is the consistent hierarchy's
     launch_consistent(h);
-    launch_residual(h, 2);
+    launch_residual(h, RES_RHS);
   }
   // every instance iterates until its own stop test fails; a converged
   // instance of a batch is frozen (its stores are predicated off) while the
@@ -2707,6 +2759,8 @@ int bsam_solve_cycles(bsam_hier h, double *res_hist, int hist_cap, int *vcycles,
     h->graph_launches++;
     if ((rc = read_state(h, &nactive))) return rc;
   }
+  launch_qc_refresh(h);
+  CK(cudaGetLastError());
   return finish_solve(h, on_device, res_hist, hist_cap, vcycles, final_rel, visible_cells);
 }
 
@@ -2875,8 +2929,8 @@ int bsam_restore_state(bsam_hier h) {
 
 int bsam_launch_count(bsam_hier h, int64_t *count) {
   if (!h || !count) return fail(BSAM_ERR_ARG, "null argument");
-  *count = h->launch_count + h->graph_launches * h->kernels_per_cycle + h->while_bodies * (h->kernels_per_cycle + 1) +
-           h->solve_graphs * h->preamble_kernels;
+  *count = h->launch_count + h->graph_launches * h->kernels_per_cycle + h->while_bodies * h->kernels_per_cycle +
+           h->solve_graphs * (h->preamble_kernels + 1);
   return BSAM_OK;
 }
 
@@ -2947,7 +3001,7 @@ int bsam_profile_vcycles(bsam_hier h, int ncycles, int level, double ms[BSAM_NKI
   if ((rc = ensure_f32(h))) return rc;
   if (mixed(h)) {
     launch_consistent(h);
-    launch_residual(h, 2);
+    launch_residual(h, RES_RHS);
   } else {
     reset_force(h);
   }
@@ -2955,7 +3009,7 @@ int bsam_profile_vcycles(bsam_hier h, int ncycles, int level, double ms[BSAM_NKI
   h->profiling = true;
   h->profile_level = level;
   h->recs.clear();
-  for (int c = 0; c < ncycles && !rc; ++c) rc = launch_iteration(h, 2);
+  for (int c = 0; c < ncycles && !rc; ++c) rc = launch_iteration(h, RES_REPORT);
   h->profiling = false;
   cudaError_t e = cudaStreamSynchronize(h->stream);
   for (auto &r : h->recs) {

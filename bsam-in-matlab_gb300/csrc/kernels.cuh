@@ -69,17 +69,30 @@ struct FieldsT {
   const int *win, *fp;         // window gathers, footprint scatters (2 ints/cell)
   const int *active;           // per instance: 1 while its V-cycles continue (below)
 };
-// `active` is written only by k_residual_final, the last kernel of a launch
+// `active` is written only by k_solve_step, the last kernel of a launch
 // chain, and the host synchronises before the next chain (or writes it with
 // a stream-ordered copy).  Within a chain no kernel can still be in its
-// pre-wait part when k_residual_final's body runs (every kernel completes
+// pre-wait part when k_solve_step's body runs (every kernel completes
 // only after its predecessor), so kernels read `active` before
 // griddepcontrol.wait and the blocks of a frozen instance skip their loads.
 using Fields = FieldsT<double>;
 
-// FP64 view of a value of either type (a no-op for double)
-template <class T>
-__device__ __forceinline__ double dbl(T x) { return (double)x; }
+// FP64 view of a value of either type (a no-op for double).  A float is
+// widened on the integer pipe: the conversion instruction shares the FP64
+// pipe (one warp every 19 cycles per SM), and the mixed form's coarse load
+// converts as many values as it does FP64 operations.  A denormal is brought
+// to the normal range first (an exact FP32 product).
+__device__ __forceinline__ double dbl(double x) { return x; }
+__device__ __forceinline__ double dbl(float x) {
+  unsigned u = __float_as_uint(x), off = 0x38000000u;   // (1023 - 127) << 20
+  const unsigned m = u & 0x7fffffffu;
+  if (m < 0x00800000u) {
+    u = __float_as_uint(x * 16777216.0f);
+    off = m ? 0x38000000u - (24u << 20) : 0u;
+  }
+  if (m >= 0x7f800000u) off = 0x70000000u;              // infinity, NaN
+  return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + off)), (int)(u << 29));
+}
 
 // one level's work decomposition for one kind of item
 struct Decomp {
@@ -103,7 +116,7 @@ struct Decomp {
 // divisions, 3.6 with this; the three-level ragged solve 4.23 -> 3.95 ms.
 struct DivC {
   double d, r;
-  int ops;
+  int ops, kexp;               // kexp: what x / d adds to x's high word (ops 1)
   unsigned elo, espan;
 };
 
@@ -112,16 +125,43 @@ __device__ __forceinline__ bool is_zero(double x) {
   return (((unsigned)__double2hiint(x) << 1) | (unsigned)__double2loint(x)) == 0u;
 }
 
+__device__ __noinline__ double div_out_of_line(double x, double d) { return x / d; }
+
+// kPow2: the kernel's variant for levels where every constant is a power of
+// two (ops 1), which carries none of the other code
+template <bool kPow2>
 __device__ __forceinline__ double div_c(double x, const DivC &D) {
   const double q0 = x * D.r;
-  if (D.ops == 1) return q0;
+  if (kPow2 || D.ops == 1) return q0;
   double q = __fma_rn(__fma_rn(-q0, D.d, x), D.r, q0);
   if (D.ops == 5) q = __fma_rn(__fma_rn(-q, D.d, x), D.r, q);
-  if (exp_bits(x) - D.elo > D.espan) q = is_zero(x) ? q0 : x / D.d;
+  if (exp_bits(x) - D.elo > D.espan) q = is_zero(x) ? q0 : div_out_of_line(x, D.d);
   return q;
 }
+
+// The face coefficients of an operator on a power-of-two level, scaled by the
+// exact 1/h^2 on the integer pipe before they are used: (D 2^-k) dq ==
+// (D dq) 2^-k in floating point, so the operator's two divisions fall away
+// (relax_cell's packed operands rely on the same).  Coefficients whose scaled
+// exponent could leave the normal range (faces_in false for any of a cell's)
+// are multiplied instead.
+template <int kN>
+__device__ __forceinline__ bool faces_in(const double (&c)[kN], const DivC &D) {
+  bool in = true;
+#pragma unroll
+  for (int i = 0; i < kN; ++i) in = in && exp_bits(c[i]) - D.elo <= D.espan;
+  return in;
+}
+template <int kN>
+__device__ __forceinline__ void scale_faces(double (&c)[kN], const DivC &D, bool in) {
+#pragma unroll
+  for (int i = 0; i < kN; ++i)
+    c[i] = in ? __hiloint2double(__double2hiint(c[i]) + D.kexp, __double2loint(c[i])) : c[i] * D.r;
+}
+
 // FP32: a divide is short there (with the steps above the ragged mixed solve
 // was 2% slower)
+template <bool kPow2>
 __device__ __forceinline__ float div_c(float x, float d) { return x / d; }
 
 struct LevelD {
@@ -149,19 +189,30 @@ __device__ __forceinline__ int find_patch(const Decomp &D, int b, int g) {
   return p;
 }
 
-// op2d (ebKernels.m:13-25) at one cell from its values and coefficients
+// op2d (ebKernels.m:13-25) at one cell from its face fluxes (kPow2: formed
+// with scale_faces' coefficients)
+template <bool kPow2>
+__device__ __forceinline__ double op_flux(double feE, double feW, double fnN, double fnS, double cc, double q,
+                                          const LevelD &L) {
+  if (kPow2) return (-(feE - feW) - (fnN - fnS)) + cc * q;
+  return (div_c<false>(-(feE - feW), L.dx) - div_c<false>(fnN - fnS, L.dy)) + cc * q;
+}
+
+// the same from its values and (unscaled) coefficients
+template <bool kPow2>
 __device__ __forceinline__ double op_pre(double q, double qe, double qw, double qn, double qs, double dE, double dW,
                                          double dN, double dS, double cc, const LevelD &L) {
   const double feE = dE * (qe - q), feW = dW * (q - qw), fnN = dN * (qn - q), fnS = dS * (q - qs);
-  return (div_c(-(feE - feW), L.dx) - div_c(fnN - fnS, L.dy)) + cc * q;
+  return (div_c<kPow2>(-(feE - feW), L.dx) - div_c<kPow2>(fnN - fnS, L.dy)) + cc * q;
 }
 
 // the same at interior cell (li, lj) of a padded array
+template <bool kPow2 = false>
 __device__ __forceinline__ double op_cell_r(const double *__restrict__ Qa, int ldq, const double *__restrict__ DeW,
                                             const double *__restrict__ DnS, double cc, int mx, int li, int lj,
                                             const LevelD &L) {
   const int c = (li + 1) + (lj + 1) * ldq;
-  return op_pre(Qa[c], Qa[c + 1], Qa[c - 1], Qa[c + ldq], Qa[c - ldq], DeW[(li + 1) + lj * (mx + 1)],
+  return op_pre<kPow2>(Qa[c], Qa[c + 1], Qa[c - 1], Qa[c + ldq], Qa[c - ldq], DeW[(li + 1) + lj * (mx + 1)],
                 DeW[li + lj * (mx + 1)], DnS[li + (lj + 1) * mx], DnS[li + lj * mx], cc, L);
 }
 
@@ -440,7 +491,7 @@ struct __align__(16) RelaxChunkD {
 
 // how a smoother chunk learns that its instance is frozen: kActNone, one
 // instance (always live while a V-cycle runs); kActChunk, the per-chunk flag
-// array k_residual_final keeps (a batch's instances' chunks are contiguous
+// array k_solve_step keeps (a batch's instances' chunks are contiguous
 // per level)
 enum { kActNone = 0, kActChunk = 1 };
 
@@ -646,10 +697,10 @@ __device__ __forceinline__ void cell_update(const LevelD &L, const FieldsT<T> &f
     t = t + qn * S.dN;
     t = t + qs * S.dS;
   } else {
-    t = t + div_c(qe * S.dE, H.dx);
-    t = t + div_c(qw * S.dW, H.dx);
-    t = t + div_c(qn * S.dN, H.dy);
-    t = t + div_c(qs * S.dS, H.dy);
+    t = t + div_c<false>(qe * S.dE, H.dx);
+    t = t + div_c<false>(qw * S.dW, H.dx);
+    t = t + div_c<false>(qn * S.dN, H.dy);
+    t = t + div_c<false>(qs * S.dS, H.dy);
   }
   t = t * S.idg;
   if (unit_omega) Q[c] = t;
@@ -818,10 +869,10 @@ __global__ void __launch_bounds__(kBlock) k_relax_n(LevelD L, const RelaxChunkD 
       t = t + qn[u] * dN[u];
       t = t + qs[u] * dS[u];
     } else {
-      t = t + div_c(qe[u] * dE[u], H.dx);
-      t = t + div_c(qw[u] * dW[u], H.dx);
-      t = t + div_c(qn[u] * dN[u], H.dy);
-      t = t + div_c(qs[u] * dS[u], H.dy);
+      t = t + div_c<false>(qe[u] * dE[u], H.dx);
+      t = t + div_c<false>(qw[u] * dW[u], H.dx);
+      t = t + div_c<false>(qn[u] * dN[u], H.dy);
+      t = t + div_c<false>(qs[u] * dS[u], H.dy);
     }
     t = t * idg[u];
     if (unit_omega) Q[c[u]] = t;
@@ -859,8 +910,8 @@ __global__ void __launch_bounds__(kClusterBlock, 1)
                     const T *__restrict__ pack, const Rule *__restrict__ perim, T omega, int unit_omega, int nsweeps,
                     int first_fresh, const uint8_t *__restrict__ cact, int amode, GhostItems G, int g_off, int g_n,
                     double hx_, double hy_) {
-  namespace cg = cooperative_groups;
   chain_trigger();
+  namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   const int nth = (int)cl.num_blocks() * kClusterBlock;
   const int tid = (int)cl.block_rank() * kClusterBlock + threadIdx.x;
@@ -1056,10 +1107,10 @@ __device__ __forceinline__ void dsm_cell_update(const LevelD &L, const FieldsT<T
     t = t + qn * X.dN;
     t = t + qs * X.dS;
   } else {
-    t = t + div_c(qe * X.dE, H.dx);
-    t = t + div_c(qw * X.dW, H.dx);
-    t = t + div_c(qn * X.dN, H.dy);
-    t = t + div_c(qs * X.dS, H.dy);
+    t = t + div_c<false>(qe * X.dE, H.dx);
+    t = t + div_c<false>(qw * X.dW, H.dx);
+    t = t + div_c<false>(qn * X.dN, H.dy);
+    t = t + div_c<false>(qs * X.dS, H.dy);
   }
   t = t * X.idg;
   const uint32_t ac = dsm_addr(D, c);
@@ -1084,11 +1135,11 @@ __global__ void __launch_bounds__(kDsmBlock, 1)
                 const T *__restrict__ pack, const Rule *__restrict__ perim, T omega, int unit_omega, int nsweeps,
                 int first_fresh, const uint8_t *__restrict__ cact, int amode, GhostItems G, int g_off, int g_n,
                 double hx_, double hy_, int q0, int qn, int shift) {
+  chain_trigger();
   namespace cg = cooperative_groups;
   constexpr int kB = kDsmBlock;
   extern __shared__ __align__(16) unsigned char dsm_raw[];
   T *slice = reinterpret_cast<T *>(dsm_raw);
-  chain_trigger();
   cg::cluster_group cl = cg::this_cluster();
   const int C = (int)cl.num_blocks(), r = (int)cl.block_rank();
   const int S = 1 << shift;
@@ -1271,7 +1322,7 @@ __global__ void __launch_bounds__(kT) k_restrict_fill(LevelD L, Decomp D, Fields
 // (`qc_inner` true: the residual's refresh, ebCompResidual.m:32-38).
 // The arithmetic is FP64 for either value type (the reflux of the mixed
 // form stays FP64).
-template <class T>
+template <bool kPow2, class T>
 __device__ __forceinline__ double face_corr(const PatchD &P, const FieldsT<T> &f, int fc, int j,
                                             const DivC &hc2, bool qc_inner) {
   const int mx = P.mx, my = P.my, cmx = mx >> 1, cmy = my >> 1;
@@ -1318,7 +1369,7 @@ __device__ __forceinline__ double face_corr(const PatchD &P, const FieldsT<T> &f
       break;
     }
   }
-  return div_c(v, hc2);
+  return div_c<kPow2>(v, hc2);
 }
 
 // gather-form corrections of one target coarse cell: contributions in the
@@ -1327,13 +1378,13 @@ struct CorrCSR {
   const int *cell, *patch, *beg, *item, *jj;   // item = (level-local fine patch << 2) | face
 };
 
-template <class T>
+template <bool kPow2, class T>
 __device__ __forceinline__ double add_corrections(double v, const CorrCSR &C, int t, const LevelD &Lf, const LevelD &Lc,
                                                   const FieldsT<T> &f, bool qc_inner) {
   for (int i = C.beg[t]; i < C.beg[t + 1]; ++i) {
     const int it = C.item[i];
     const int fc = it & 3;
-    v = v + face_corr(Lf.patches[it >> 2], f, fc, C.jj[i], fc < 2 ? Lc.dx : Lc.dy, qc_inner);
+    v = v + face_corr<kPow2>(Lf.patches[it >> 2], f, fc, C.jj[i], fc < 2 ? Lc.dx : Lc.dy, qc_inner);
   }
   return v;
 }
@@ -1363,7 +1414,7 @@ __device__ __forceinline__ void load_ring_item(const FieldsT<T> &f, const int *_
   if (on) f.QC[dst] = f.Q[src];
 }
 
-template <class T, bool kChain>
+template <class T, bool kPow2, bool kChain>
 __device__ __forceinline__ void load_fp_item(const LevelD &L, const LevelD &Lc, const Decomp &D, const FieldsT<T> &f,
                                              int g) {
   if (g >= D.n) {
@@ -1380,19 +1431,18 @@ __device__ __forceinline__ void load_fp_item(const LevelD &L, const LevelD &Lc, 
   const int s = g - __ldg(D.beg + p);
   const int cj = s / cmx, ci = s - cj * cmx;
   const int q_off = P.q_off, c_off = P.c_off, qc_off = P.qc_off;
-  // static operands of the four fine cells (restrict2 order) and of the
-  // coarse operator
-  const T *DeW = f.DeW + P.dew_off, *DnS = f.DnS + P.dns_off, *CC = f.CC + c_off;
-  double dE[4], dW[4], dN[4], dS[4], cf[4];
+  // static operands: the 2 x 3 x-faces and 3 x 2 y-faces of the four fine
+  // cells, their reaction coefficients, and the coarse operator's
+  const T *DeW = f.DeW + P.dew_off + 2 * ci + 2 * cj * (mx + 1), *DnS = f.DnS + P.dns_off + 2 * ci + 2 * cj * mx;
+  const T *CC = f.CC + c_off + 2 * ci + 2 * cj * mx;
+  double dx[6], dy[6], cf[4];
 #pragma unroll
-  for (int t = 0; t < 4; ++t) {
-    const int li = 2 * ci + (t & 1), lj = 2 * cj + (t >> 1);
-    dE[t] = dbl(__ldg(DeW + (li + 1) + lj * (mx + 1)));
-    dW[t] = dbl(__ldg(DeW + li + lj * (mx + 1)));
-    dN[t] = dbl(__ldg(DnS + li + (lj + 1) * mx));
-    dS[t] = dbl(__ldg(DnS + li + lj * mx));
-    cf[t] = dbl(__ldg(CC + li + lj * mx));
+  for (int t = 0; t < 6; ++t) {
+    dx[t] = dbl(__ldg(DeW + t % 3 + (t / 3) * (mx + 1)));
+    dy[t] = dbl(__ldg(DnS + t % 2 + (t / 2) * mx));
   }
+#pragma unroll
+  for (int t = 0; t < 4; ++t) cf[t] = dbl(__ldg(CC + (t & 1) + (t >> 1) * mx));
   const int ldc = cmx + 2;
   const int *win = f.win + P.win_off;
   const int w = (ci + 1) + (cj + 1) * ldc;
@@ -1404,20 +1454,47 @@ __device__ __forceinline__ void load_fp_item(const LevelD &L, const LevelD &Lc, 
   const T *PDeW = f.pcoef + P.pc_off;
   const T *PDnS = PDeW + (cmx + 1) * cmy;
   const T *PCC = PDnS + cmx * (cmy + 1);
-  const double pE = dbl(__ldg(PDeW + (ci + 1) + cj * (cmx + 1))), pW = dbl(__ldg(PDeW + ci + cj * (cmx + 1)));
-  const double pN = dbl(__ldg(PDnS + ci + (cj + 1) * cmx)), pS = dbl(__ldg(PDnS + ci + cj * cmx));
+  double px[2] = {dbl(__ldg(PDeW + ci + cj * (cmx + 1))), dbl(__ldg(PDeW + (ci + 1) + cj * (cmx + 1)))};
+  double py[2] = {dbl(__ldg(PDnS + ci + cj * cmx)), dbl(__ldg(PDnS + ci + (cj + 1) * cmx))};
   const double pC = dbl(__ldg(PCC + s));
   const int dst = __ldg(f.fp + 2 * (P.fp_off + s) + 1);
+  if (kPow2) {
+    if (faces_in(dx, L.dx) && faces_in(dy, L.dy) && faces_in(px, Lc.dx) && faces_in(py, Lc.dy)) {
+      scale_faces(dx, L.dx, true);
+      scale_faces(dy, L.dy, true);
+      scale_faces(px, Lc.dx, true);
+      scale_faces(py, Lc.dy, true);
+    } else {
+      scale_faces(dx, L.dx, false);
+      scale_faces(dy, L.dy, false);
+      scale_faces(px, Lc.dx, false);
+      scale_faces(py, Lc.dy, false);
+    }
+  }
   if (kChain) chain_wait();
-  const T *Qp = f.Q + q_off;
-  const T *Fp = f.F + c_off;
-  double rf[4];
+  // the four fine cells and their eight neighbours: v[j][i], corners unused
+  const T *Qp = f.Q + q_off + 2 * ci + 2 * cj * ldq;
+  double v[4][4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      v[j][i] = (i == 0 || i == 3) && (j == 0 || j == 3) ? 0.0 : dbl(Qp[i + j * ldq]);
+  // each face's flux once: the neighbour across it forms the same one
+  double fx[2][3], fy[3][2], rf[4];
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      fx[j][i] = dx[3 * j + i] * (v[j + 1][i + 1] - v[j + 1][i]);
+      fy[i][j] = dy[2 * i + j] * (v[i + 1][j + 1] - v[i][j + 1]);
+    }
+  const T *Fp = f.F + c_off + 2 * ci + 2 * cj * mx;
 #pragma unroll
   for (int t = 0; t < 4; ++t) {
-    const int li = 2 * ci + (t & 1), lj = 2 * cj + (t >> 1);
-    const int c = (li + 1) + (lj + 1) * ldq;
-    rf[t] = dbl(Fp[li + lj * mx]) - op_pre(dbl(Qp[c]), dbl(Qp[c + 1]), dbl(Qp[c - 1]), dbl(Qp[c + ldq]),
-                                           dbl(Qp[c - ldq]), dE[t], dW[t], dN[t], dS[t], cf[t], L);
+    const int i = t & 1, j = t >> 1;
+    rf[t] = dbl(Fp[i + j * mx]) -
+            op_flux<kPow2>(fx[j][i + 1], fx[j][i], fy[j + 1][i], fy[j][i], cf[t], v[j + 1][i + 1], L);
   }
   const double rr = 0.25 * (((rf[0] + rf[1]) + rf[2]) + rf[3]);
   const T *QC = f.QC + qc_off;
@@ -1426,11 +1503,11 @@ __device__ __forceinline__ void load_fp_item(const LevelD &L, const LevelD &Lc, 
   const double qw = dbl(sw >= 0 ? f.Q[sw] : QC[w - 1]);
   const double qn = dbl(sn >= 0 ? f.Q[sn] : QC[w + ldc]);
   const double qs = dbl(ss >= 0 ? f.Q[ss] : QC[w - ldc]);
-  const double lc = op_pre(q, qe, qw, qn, qs, pE, pW, pN, pS, pC, Lc);
+  const double lc = op_flux<kPow2>(px[1] * (qe - q), px[0] * (q - qw), py[1] * (qn - q), py[0] * (q - qs), pC, q, Lc);
   f.F[dst] = T(rr + lc);
 }
 
-template <class T, bool kChain>
+template <class T, bool kPow2, bool kChain>
 __device__ __forceinline__ void load_corr_item(const LevelD &L, const LevelD &Lc, const FieldsT<T> &f, const CorrCSR &C,
                                                int n_tgt, int t) {
   const bool on = t < n_tgt && f.active[Lc.patches[C.patch[t]].inst];
@@ -1442,13 +1519,13 @@ __device__ __forceinline__ void load_corr_item(const LevelD &L, const LevelD &Lc
   // not depend on a reset of F before it; the correction cycle of the mixed
   // form adds to its own right-hand side
   const double base = sizeof(T) == sizeof(double) ? f.FTrue[cell] : dbl(f.F[cell]);
-  f.F[cell] = T(add_corrections<T>(base, C, t, L, Lc, f, false));
+  f.F[cell] = T(add_corrections<kPow2, T>(base, C, t, L, Lc, f, false));
 }
 
 // kT threads per block (kBlock, or 64 on a level whose kBlock grid leaves
 // SMs idle: a footprint cell is ~84 FP64 operations, and an SM issues about
 // two per clock); the decomposition's per-block patch table is kBlock-based
-template <class T, int kT = kBlock>
+template <class T, bool kPow2, int kT = kBlock>
 __global__ void __launch_bounds__(kT) k_load(LevelD L, LevelD Lc, Decomp D, FieldsT<T> f, const int *__restrict__ ring,
                                              const int *__restrict__ ring_inst, int ring_off, int n_ring, CorrCSR C,
                                              int n_tgt) {
@@ -1462,11 +1539,11 @@ __global__ void __launch_bounds__(kT) k_load(LevelD L, LevelD Lc, Decomp D, Fiel
   }
   b -= nb_ring;
   if (b < nb_fp) {
-    load_fp_item<T, true>(L, Lc, D, f, b * kT + threadIdx.x);
+    load_fp_item<T, kPow2, true>(L, Lc, D, f, b * kT + threadIdx.x);
     return;
   }
   b -= nb_fp;
-  load_corr_item<T, true>(L, Lc, f, C, n_tgt, b * kT + threadIdx.x);
+  load_corr_item<T, kPow2, true>(L, Lc, f, C, n_tgt, b * kT + threadIdx.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -1656,17 +1733,29 @@ __global__ void __launch_bounds__(32 * kRows) k_coarsest(const double *__restric
 // ---------------------------------------------------------------------------
 // Composite residual (ebCompResidual.m:15-85) of every level >= root, for one
 // hierarchy or every instance of a batch, in one launch.  The work is a list
-// of warp tasks, each covering up to 32 * kResLane items of ONE patch (or of
-// one instance's correction targets), so every warp belongs to one instance:
+// of warp tasks of up to 32 items of ONE patch (or of one instance's
+// correction targets), so every warp belongs to one instance:
 //   kind 0  r = FTrue - op(Q) on visible cells of a patch in the norms,
-//           correction targets excluded while the corrections are on
+//           correction targets excluded while the corrections are on; an item
+//           is kResRows cells of one column, whose inner y fluxes are formed
+//           once
 //   kind 1  r at correction targets of a level, corrections added in order,
 //           the coarse values taken as the refreshed QC holds them
+// and, in a launch of their own (k_qc_refresh), tasks of up to 128 items:
 //   kind 2  QC ring refresh of a patch (ebCompResidual.m:25)
 //   kind 3  QC interior refresh of a patch (ebCompResidual.m:32-38)
-// A residual warp reduces its values (fixed shuffle tree) into one slot;
-// k_residual_final reduces each instance's slots.  Max-norms are order-free,
-// so linf and rel do not depend on the task layout.
+// Inside a solve only the max-norms are needed (kL2 false): a warp reduces
+// them into its instance's two accumulators with a max on their bit patterns
+// (non-negative doubles order like integers); the source's norm does not
+// change between V-cycles and is only formed before the first one.  A report
+// (kL2) also reduces the squares, into one slot per task, for
+// k_residual_final.  Max-norms are order-free, so linf and rel do not depend
+// on the task layout.
+//
+// Bound by the FP64 pipe and latency: about 13 operations per cell (19 with
+// every flux formed twice, the scaling by 1/h^2 on the FP64 pipe and the
+// squares): starfish 34 us -> @RES@ us per iteration, its floor at the
+// measured FP64 rate 10 us.
 struct ResAcc {
   double out[5];        // linf, l2, fnorm, rel, ncell
 };
@@ -1693,103 +1782,146 @@ __device__ __forceinline__ double pmax(double a, double b) {
   return __longlong_as_double(m < 0 ? 0 : m);
 }
 
-// items per lane of a residual warp task (a task covers up to 32 * kResLane
-// items of one patch or one instance's targets)
-constexpr int kResLane = 4;
+constexpr int kResRows = 4;
 
 // kT threads per block (kBlock, or 64 where the kBlock grid would leave
 // SMs with unequal shares of the FP64 work)
-template <int kT = kBlock>
+template <bool kL2, bool kPow2, int kT = kBlock>
 __global__ void __launch_bounds__(kT) k_residual(const LevelX *__restrict__ X, const PatchD *__restrict__ patches,
-                                                 const ResTask *__restrict__ tasks, int ntask, Fields f,
-                                                 const int *__restrict__ ring, double *slots, int nslots,
-                                                 int mass_corr, float *__restrict__ rout) {
+                                                 const ResTask *__restrict__ tasks, int ntask, Fields f, double *slots,
+                                                 int nslots, unsigned long long *norms, int want_fn, int mass_corr,
+                                                 float *__restrict__ rout) {
   chain_trigger();
   const int w = blockIdx.x * (kT / 32) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  // a frozen instance's residual is neither reported nor needed (its QC
-  // refresh would rewrite the same values), so its warps only wait
+  // a frozen instance's residual is neither reported nor needed, so its
+  // warps only wait
   if (w >= ntask || !f.active[tasks[w].inst]) {
     chain_wait();
     return;
   }
   const ResTask T = tasks[w];
-  chain_wait();
-  if (T.kind >= 2) {
-    if (!mass_corr) return;
-    if (T.kind == 2) {
-      for (int e = lane; e < T.n; e += 32) {
-        const int i = T.a + e;
-        f.QC[__ldg(ring + 2 * i + 1)] = f.Q[__ldg(ring + 2 * i)];
-      }
-      return;
-    }
-    const PatchD &P = patches[T.a];
-    const int cmx = P.mx >> 1;
-    for (int e = lane; e < T.n; e += 32) {
-      const int s = T.b + e;
-      const int cj = s / cmx, ci = s - cj * cmx;
-      f.QC[P.qc_off + (ci + 1) + (cj + 1) * (cmx + 2)] = restrict_cell(f.Q + P.q_off, P.mx + 2, ci, cj);
-    }
-    return;
-  }
   double li = 0, sq = 0, fn = 0;
   const LevelX &Xk = X[T.level];
+  auto take = [&](double r, double ft) {
+    li = pmax(li, fabs(r));
+    if (kL2) sq = sq + r * r;
+    if (kL2 || want_fn) fn = pmax(fn, fabs(ft));
+  };
   if (T.kind == 0) {
     const PatchD &P = patches[T.a];
-    const int mx = P.mx, ldq = mx + 2;
-    const double *DeW = f.DeW + P.dew_off, *DnS = f.DnS + P.dns_off, *Qp = f.Q + P.q_off;
+    const int mx = P.mx, my = P.my, ldq = mx + 2;
+    const int i = T.b + min(lane, T.n - 1);
+    const int g = i / mx, lx = i - g * mx, lj0 = g * kResRows;
+    const int rows = lane < T.n ? min(kResRows, my - lj0) : 0;
+    const double *DeW = f.DeW + P.dew_off + lx + lj0 * (mx + 1), *DnS = f.DnS + P.dns_off + lx + lj0 * mx;
+    const int cc = P.c_off + lx + lj0 * mx;
+    // static operands before the programmatic-launch wait
+    double dE[kResRows], dW[kResRows], dN[kResRows + 1], cf[kResRows], ft[kResRows];
+    uint8_t fl[kResRows];
+    dN[0] = __ldg(DnS);
 #pragma unroll
-    for (int u = 0; u < kResLane; ++u) {
-      const int e = lane + 32 * u;
-      if (e >= T.n) break;
-      const int s = T.b + e;
-      const int lj = s / mx, lx = s - lj * mx;
-      const int cc = P.c_off + s;
-      const uint8_t fl = __ldg(f.flags + cc);
-      if ((fl & 1) || (mass_corr && (fl & 2))) continue;
-      const double ft = __ldg(f.FTrue + cc);
-      const int c = (lx + 1) + (lj + 1) * ldq;
-      const double r = ft - op_pre(Qp[c], Qp[c + 1], Qp[c - 1], Qp[c + ldq], Qp[c - ldq],
-                                   __ldg(DeW + (lx + 1) + lj * (mx + 1)), __ldg(DeW + lx + lj * (mx + 1)),
-                                   __ldg(DnS + lx + (lj + 1) * mx), __ldg(DnS + lx + lj * mx), __ldg(f.CC + cc), Xk.L);
-      li = pmax(li, fabs(r));
-      sq = sq + r * r;
-      fn = pmax(fn, fabs(ft));
-      if (rout) rout[cc] = (float)r;
+    for (int u = 0; u < kResRows; ++u) {
+      const int v = u < rows ? u : 0;
+      dE[u] = __ldg(DeW + 1 + v * (mx + 1));
+      dW[u] = __ldg(DeW + v * (mx + 1));
+      dN[u + 1] = __ldg(DnS + (v + 1) * mx);
+      cf[u] = __ldg(f.CC + cc + v * mx);
+      ft[u] = __ldg(f.FTrue + cc + v * mx);
+      fl[u] = __ldg(f.flags + cc + v * mx);
     }
-  } else if (mass_corr) {   // kind 1: targets of this level, corrections from the level above
+    if (kPow2) {
+      const DivC &Dx = Xk.L.dx, &Dy = Xk.L.dy;
+      if (__all_sync(0xffffffffu, faces_in(dE, Dx) && faces_in(dW, Dx) && faces_in(dN, Dy))) {
+        scale_faces(dE, Dx, true);
+        scale_faces(dW, Dx, true);
+        scale_faces(dN, Dy, true);
+      } else {
+        scale_faces(dE, Dx, false);
+        scale_faces(dW, Dx, false);
+        scale_faces(dN, Dy, false);
+      }
+    }
+    chain_wait();
+    const double *Q = f.Q + P.q_off + (lx + 1) + (lj0 + 1) * ldq;
+    double q = Q[0], fs = dN[0] * (q - Q[-ldq]);
+#pragma unroll
+    for (int u = 0; u < kResRows; ++u) {
+      if (u >= rows) break;
+      const double *Qu = Q + u * ldq;
+      const double qn = Qu[ldq];
+      const double feE = dE[u] * (Qu[1] - q), feW = dW[u] * (q - Qu[-1]), fnN = dN[u + 1] * (qn - q);
+      if (!((fl[u] & 1) || (mass_corr && (fl[u] & 2)))) {
+        const double r = ft[u] - op_flux<kPow2>(feE, feW, fnN, fs, cf[u], q, Xk.L);
+        take(r, ft[u]);
+        if (rout) rout[cc + u * mx] = (float)r;
+      }
+      q = qn;
+      fs = fnN;
+    }
+  } else {   // targets of this level, corrections from the level above
+    chain_wait();
+    if (!mass_corr) return;
     const LevelX &Xf = X[T.level + 1];
-    for (int u = 0; u < kResLane; ++u) {
-      const int e = lane + 32 * u;
-      if (e >= T.n) break;
-      const int g = T.b + e;
+    if (lane < T.n) {
+      const int g = T.b + lane;
       const int cell = Xf.C.cell[g];
       const PatchD &Pc = Xk.L.patches[Xf.C.patch[g]];
       const int s = cell - Pc.c_off;
       const int lj = s / Pc.mx, lx = s - lj * Pc.mx;
       const double ft = f.FTrue[cell];
-      double r = ft - op_cell_r(f.Q + Pc.q_off, Pc.mx + 2, f.DeW + Pc.dew_off, f.DnS + Pc.dns_off, f.CC[cell], Pc.mx,
+      double r = ft - op_cell_r<kPow2>(f.Q + Pc.q_off, Pc.mx + 2, f.DeW + Pc.dew_off, f.DnS + Pc.dns_off, f.CC[cell], Pc.mx,
                                 lx, lj, Xk.L);
-      r = add_corrections(r, Xf.C, g, Xf.L, Xk.L, f, true);
+      r = add_corrections<kPow2>(r, Xf.C, g, Xf.L, Xk.L, f, true);
       if (rout) rout[cell] = (float)r;
-      if (!(f.flags[cell] & 1)) {
-        li = pmax(li, fabs(r));
-        sq = sq + r * r;
-        fn = pmax(fn, fabs(ft));
-      }
+      if (!(f.flags[cell] & 1)) take(r, ft);
     }
   }
+  if (!kL2 && !norms) return;
 #pragma unroll
   for (int off = 16; off >= 1; off >>= 1) {
     li = pmax(li, __shfl_down_sync(0xffffffffu, li, off));
-    fn = pmax(fn, __shfl_down_sync(0xffffffffu, fn, off));
-    sq = sq + __shfl_down_sync(0xffffffffu, sq, off);
+    if (kL2 || want_fn) fn = pmax(fn, __shfl_down_sync(0xffffffffu, fn, off));
+    if (kL2) sq = sq + __shfl_down_sync(0xffffffffu, sq, off);
   }
-  if (lane == 0) {
+  if (lane) return;
+  if (kL2) {
     slots[T.slot] = li;
     slots[nslots + T.slot] = sq;
     slots[2 * nslots + T.slot] = fn;
+  } else {
+    // most warps find a larger value there already and leave it
+    unsigned long long *a = norms + 2 * T.inst;
+    const unsigned long long l = (unsigned long long)__double_as_longlong(li);
+    if (l > __ldcg(a)) atomicMax(a, l);
+    if (want_fn) atomicMax(a + 1, (unsigned long long)__double_as_longlong(fn));
+  }
+}
+
+// The refresh of QC's ring and interior that the reference's residual makes
+// (ebCompResidual.m:25,32-38), a function of Q alone: no kernel reads a QC
+// cell between a residual and the next restriction and ring gather, so a
+// solve runs it once, after its last V-cycle.
+__global__ void __launch_bounds__(kBlock) k_qc_refresh(const PatchD *__restrict__ patches,
+                                                       const ResTask *__restrict__ tasks, int ntask, Fields f,
+                                                       const int *__restrict__ ring) {
+  const int w = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (w >= ntask) return;
+  const ResTask T = tasks[w];
+  if (T.kind == 2) {
+    for (int e = lane; e < T.n; e += 32) {
+      const int i = T.a + e;
+      f.QC[__ldg(ring + 2 * i + 1)] = f.Q[__ldg(ring + 2 * i)];
+    }
+    return;
+  }
+  const PatchD &P = patches[T.a];
+  const int cmx = P.mx >> 1;
+  for (int e = lane; e < T.n; e += 32) {
+    const int s = T.b + e;
+    const int cj = s / cmx, ci = s - cj * cmx;
+    f.QC[P.qc_off + (ci + 1) + (cj + 1) * (cmx + 2)] = restrict_cell(f.Q + P.q_off, P.mx + 2, ci, cj);
   }
 }
 
@@ -1805,128 +1937,102 @@ struct SlotRange {
   double area;
 };
 
-// finish the residual of every instance (one block per instance): max-norms
-// over its slots, L2 per level from that level's slots in a fixed tree order
-// weighted by the cell area, rel = linf / max(fnorm, realmin).  mode 0 is
-// the residual before the first V-cycle; mode 1 follows a V-cycle of the
-// instances active during it; mode 2 only reports (an eager call).  The history and the stop test follow
-// ebSolveCycles.m:17-46: an instance stays active while it < MaxVCycles and
-// rel > RelTol.
-constexpr int kFinal = 512;
-constexpr int kFinalGroup = 8;   // levels whose L2 trees share barrier steps
-__global__ void __launch_bounds__(kFinal) k_residual_final(const InstRes *__restrict__ ir,
-                                                          const SlotRange *__restrict__ ranges, const double *slots,
-                                                          int nslots, ResAcc *acc, int *active, int *iters,
-                                                          double *hist, int hist_stride, int mode,
-                                                          const int *__restrict__ crange, int nlev, uint8_t *cact) {
+// The end of a solve's residual: per instance rel = linf / max(fnorm,
+// realmin), the history and the stop test (ebSolveCycles.m:17-46: an instance
+// stays active while it < MaxVCycles and rel > RelTol), then the condition of
+// the solve loop's WHILE node (and of `c1`, with ncond 2): 1 while any
+// instance iterates.  mode 0 is the residual before the first V-cycle; mode 1
+// follows a V-cycle of the instances active during it.  One block, a thread
+// per instance: the former pair of kernels (a tree over one slot per task,
+// then the condition) took 14 + 2 us of a starfish iteration, this one @FIN@.
+constexpr int kStep = 256;
+__global__ void __launch_bounds__(kStep) k_solve_step(const InstRes *__restrict__ ir, int ninst,
+                                                      unsigned long long *norms, ResAcc *acc, int *active, int *iters,
+                                                      double *hist, int hist_stride, int mode,
+                                                      const int *__restrict__ crange, int nlev, uint8_t *cact,
+                                                      cudaGraphConditionalHandle c0, cudaGraphConditionalHandle c1,
+                                                      int ncond) {
   chain_in();
-  const int inst = blockIdx.x;
-  const InstRes R = ir[inst];
-  __shared__ int s_write;
-  const int t = threadIdx.x;
-  // one pass over the slots: the max-norms (order-free) and, per level
-  // (range), a fixed-order tree over the threads' partial sums -- four
-  // strided partial sums per thread, then their sum; the levels of a group
-  // are reduced in the same barrier steps (each level's pairings unchanged)
-  // and summed in level order with their areas
-  double li = 0, fn = 0;
-  __shared__ double s_p[kFinalGroup][kFinal];
-  __shared__ double s_a[kFinal / 32 + 1], s_b[kFinal / 32 + 1];
-  double l2sq = 0;
-  for (int r0 = R.range0; r0 < R.range1; r0 += kFinalGroup) {
-    const int nr = min(kFinalGroup, R.range1 - r0);
-    for (int q = 0; q < nr; ++q) {
-      const int s0 = ranges[r0 + q].s0, s1 = ranges[r0 + q].s1;
-      double p0 = 0, p1 = 0, p2 = 0, p3 = 0;
-      int i = s0 + t;
-      for (; i + 3 * kFinal < s1; i += 4 * kFinal) {
-        const double a0 = slots[i], a1 = slots[i + kFinal], a2 = slots[i + 2 * kFinal], a3 = slots[i + 3 * kFinal];
-        const double b0 = slots[2 * nslots + i], b1 = slots[2 * nslots + i + kFinal];
-        const double b2 = slots[2 * nslots + i + 2 * kFinal], b3 = slots[2 * nslots + i + 3 * kFinal];
-        p0 = p0 + slots[nslots + i];
-        p1 = p1 + slots[nslots + i + kFinal];
-        p2 = p2 + slots[nslots + i + 2 * kFinal];
-        p3 = p3 + slots[nslots + i + 3 * kFinal];
-        li = pmax(li, pmax(pmax(a0, a1), pmax(a2, a3)));
-        fn = pmax(fn, pmax(pmax(b0, b1), pmax(b2, b3)));
-      }
-      for (; i < s1; i += kFinal) {
-        p0 = p0 + slots[nslots + i];
-        li = pmax(li, slots[i]);
-        fn = pmax(fn, slots[2 * nslots + i]);
-      }
-      s_p[q][t] = (p0 + p1) + (p2 + p3);
-    }
-    __syncthreads();
-    for (int off = kFinal / 2; off >= 1; off >>= 1) {
-      if (t < off)
-        for (int q = 0; q < nr; ++q) s_p[q][t] = s_p[q][t] + s_p[q][t + off];
-      __syncthreads();
-    }
-    for (int q = 0; q < nr; ++q) l2sq = l2sq + s_p[q][0] * ranges[r0 + q].area;
-    __syncthreads();
-  }
-#pragma unroll
-  for (int off = 16; off >= 1; off >>= 1) {
-    li = pmax(li, __shfl_xor_sync(0xffffffffu, li, off));
-    fn = pmax(fn, __shfl_xor_sync(0xffffffffu, fn, off));
-  }
-  if ((t & 31) == 0) {
-    s_a[t >> 5] = li;
-    s_b[t >> 5] = fn;
-  }
-  __syncthreads();
-  if (t < 32) {
-    li = t < kFinal / 32 ? s_a[t] : 0.0;
-    fn = t < kFinal / 32 ? s_b[t] : 0.0;
-#pragma unroll
-    for (int off = 16; off >= 1; off >>= 1) {
-      li = pmax(li, __shfl_xor_sync(0xffffffffu, li, off));
-      fn = pmax(fn, __shfl_xor_sync(0xffffffffu, fn, off));
-    }
-    if (t == 0) {
-      s_a[kFinal / 32] = li;
-      s_b[kFinal / 32] = fn;
-    }
-  }
-  __syncthreads();
-  const double linf = s_a[kFinal / 32];
-  double fnorm = s_b[kFinal / 32];
-  if (t == 0) {
-    int wr = -1;
+  int any = 0;
+  for (int i = threadIdx.x; i < ninst; i += kStep) {
+    if (mode != 0 && !active[i]) continue;
+    const InstRes R = ir[i];
+    const double linf = __longlong_as_double((long long)norms[2 * i]);
+    double fnorm = __longlong_as_double((long long)norms[2 * i + 1]);
+    norms[2 * i] = 0;
     fnorm = fnorm > 2.2250738585072014e-308 ? fnorm : 2.2250738585072014e-308;
     const double rel = linf / fnorm;
-    ResAcc &A = acc[inst];
-    if (mode == 2 || mode == 0 || active[inst]) {
-      A.out[0] = linf;
-      A.out[1] = sqrt(l2sq);
-      A.out[2] = fnorm;
-      A.out[3] = rel;
-      A.out[4] = R.ncell;
-    }
-    if (mode != 2 && (mode == 0 || active[inst])) {
-      int it = iters[inst];
-      if (mode == 0) it = 0;
-      else it = it + 1;
-      iters[inst] = it;
-      if (it < hist_stride) hist[(size_t)inst * hist_stride + it] = linf;
-      const int a = (it < R.max_vcycles && rel > R.rel_tol) ? 1 : 0;
-      active[inst] = a;
-      if (mode == 0 || !a) wr = a;     // every instance at the start; later only when it freezes
-    }
-    s_write = wr;
+    ResAcc &A = acc[i];
+    A.out[0] = linf;
+    A.out[2] = fnorm;
+    A.out[3] = rel;
+    A.out[4] = R.ncell;
+    const int it = mode == 0 ? 0 : iters[i] + 1;
+    iters[i] = it;
+    if (it < hist_stride) hist[(size_t)i * hist_stride + it] = linf;
+    const int a = (it < R.max_vcycles && rel > R.rel_tol) ? 1 : 0;
+    active[i] = a;
+    any |= a;
+    // the smoother's per-chunk copy of the flag, over the instance's chunk
+    // range of every level (crange: [inst][level] begin, end)
+    if (cact && (mode == 0 || !a))
+      for (int k = 0; k < nlev; ++k)
+        for (int c = crange[2 * (i * nlev + k)]; c < crange[2 * (i * nlev + k) + 1]; ++c) cact[c] = (uint8_t)a;
   }
-  // the smoother's per-chunk copy of the flag, over the instance's chunk
-  // range of every level (crange: [inst][level] begin, end)
-  if (cact) {
+  any = __syncthreads_or(any);
+  if (threadIdx.x == 0 && ncond > 0) {
+    cudaGraphSetConditional(c0, any ? 1u : 0u);
+    if (ncond > 1) cudaGraphSetConditional(c1, any ? 1u : 0u);
+  }
+}
+
+// A residual report of every instance (one block per instance): max-norms
+// over its slots, L2 per level from that level's slots in a fixed tree order
+// weighted by the cell area, rel = linf / max(fnorm, realmin).
+constexpr int kFinal = 512;
+__global__ void __launch_bounds__(kFinal) k_residual_final(const InstRes *__restrict__ ir,
+                                                          const SlotRange *__restrict__ ranges, const double *slots,
+                                                          int nslots, ResAcc *acc) {
+  chain_in();
+  const int inst = blockIdx.x, t = threadIdx.x;
+  const InstRes R = ir[inst];
+  double li = 0, fn = 0, l2sq = 0;
+  __shared__ double s_p[kFinal], s_a[kFinal], s_b[kFinal];
+  for (int r = R.range0; r < R.range1; ++r) {
+    const int s0 = ranges[r].s0, s1 = ranges[r].s1;
+    double p = 0;
+    for (int i = s0 + t; i < s1; i += kFinal) {
+      p = p + slots[nslots + i];
+      li = pmax(li, slots[i]);
+      fn = pmax(fn, slots[2 * nslots + i]);
+    }
+    s_p[t] = p;
     __syncthreads();
-    const int wr = s_write;
-    if (wr >= 0)
-      for (int k = 0; k < nlev; ++k) {
-        const int b = crange[2 * (inst * nlev + k)], e = crange[2 * (inst * nlev + k) + 1];
-        for (int c = b + t; c < e; c += kFinal) cact[c] = (uint8_t)wr;
-      }
+    for (int off = kFinal / 2; off >= 1; off >>= 1) {
+      if (t < off) s_p[t] = s_p[t] + s_p[t + off];
+      __syncthreads();
+    }
+    l2sq = l2sq + s_p[0] * ranges[r].area;
+    __syncthreads();
   }
+  s_a[t] = li;
+  s_b[t] = fn;
+  __syncthreads();
+  for (int off = kFinal / 2; off >= 1; off >>= 1) {
+    if (t < off) {
+      s_a[t] = pmax(s_a[t], s_a[t + off]);
+      s_b[t] = pmax(s_b[t], s_b[t + off]);
+    }
+    __syncthreads();
+  }
+  if (t) return;
+  const double linf = s_a[0], fnorm = s_b[0] > 2.2250738585072014e-308 ? s_b[0] : 2.2250738585072014e-308;
+  ResAcc &A = acc[inst];
+  A.out[0] = linf;
+  A.out[1] = sqrt(l2sq);
+  A.out[2] = fnorm;
+  A.out[3] = linf / fnorm;
+  A.out[4] = R.ncell;
 }
 
 // ---------------------------------------------------------------------------
@@ -1946,26 +2052,6 @@ __global__ void __launch_bounds__(kBlock) k_fp64_rate(double *out, int iters, do
 #pragma unroll
   for (int u = 0; u < 8; ++u) s = s + x[u];
   out[blockIdx.x * kBlock + threadIdx.x] = s;
-}
-
-// ---------------------------------------------------------------------------
-// Condition of the solve loop's device-side WHILE node: 1 while any instance
-// still iterates (ebSolveCycles.m:22, per instance).  One block; a single
-// thread sets the condition.
-__global__ void __launch_bounds__(kBlock) k_any_active(const int *__restrict__ active, int ninst,
-                                                       cudaGraphConditionalHandle cond,
-                                                       cudaGraphConditionalHandle cond2, int use2) {
-  chain_in();
-  __shared__ int any;
-  if (threadIdx.x == 0) any = 0;
-  __syncthreads();
-  for (int i = threadIdx.x; i < ninst; i += kBlock)
-    if (active[i]) any = 1;   // benign: every writer stores 1
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    cudaGraphSetConditional(cond, any ? 1u : 0u);
-    if (use2) cudaGraphSetConditional(cond2, any ? 1u : 0u);
-  }
 }
 
 // ---------------------------------------------------------------------------
