@@ -302,7 +302,7 @@ int sm_count() {
 
 // Every kernel goes out with programmatic stream serialization: the next
 // kernel is scheduled while the previous one drains and waits for it at its
-// griddepcontrol.wait (kernels.cuh chain_in).
+// griddepcontrol.wait (kernels.cuh chain_wait).
 template <typename... KArgs, typename... Args>
 void launch_k(bsam_hier h, void (*kern)(KArgs...), int grid, int block, Args... args) {
   if (grid <= 0) return;

@@ -12,13 +12,17 @@
 // concatenated, each patch column-major (x fastest) like the reference; the
 // solution Q and the coarse shadows QC carry their one-cell ghost frame.
 //
-// Launch chaining (programmatic dependent launch): every kernel opens with
-// griddepcontrol.launch_dependents, so the next kernel of the V-cycle is
-// scheduled while this one drains, then loads what no kernel of the solve
-// writes (patch records, coefficients, ghost rules, index tables) and only
-// then executes griddepcontrol.wait, after which it reads and writes the
-// solution state.  Every thread executes the wait before it exits, so no
-// kernel completes before its predecessor.
+// Launch chaining (programmatic dependent launch): a kernel first loads what
+// no kernel of the solve writes (patch records, coefficients, ghost rules,
+// index tables), then executes griddepcontrol.wait, after which it reads and
+// writes the solution state, and only then griddepcontrol.launch_dependents:
+// one kernel ahead is resident, and its static loads run beside this one's
+// work.  (With the trigger at entry the waiting blocks of many kernels pile
+// up, each grid's blocks go wherever those before it left room, and an
+// FP64-heavy kernel runs on part of the SMs: the starfish's second-finest
+// prolongation took 13-20 us instead of 3.9, its smoother passes 4.9 instead
+// of 3.9, an iteration 469 instead of 409 us.)  Every thread executes the
+// wait before it exits, so no kernel completes before its predecessor.
 #pragma once
 #include <cooperative_groups.h>
 #include <cstdint>
@@ -28,11 +32,9 @@
 
 namespace bsam {
 
-__device__ __forceinline__ void chain_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void chain_in() {
-  chain_trigger();
-  chain_wait();
+__device__ __forceinline__ void chain_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // a solution load; kCG: from L2 (ld.global.cg), for kernels whose blocks
@@ -400,7 +402,6 @@ __global__ void __launch_bounds__(kT) k_ghost(GhostItems G, int off, int n, T *_
                                               const T *__restrict__ bcg, double hx_, double hy_,
                                               const int *__restrict__ active, const int *__restrict__ inst_nlev,
                                               int need) {
-  chain_trigger();
   const int t = blockIdx.x * kT + threadIdx.x;
   const int i = off + t;
   // a converged instance of a batch stays frozen; a fill that follows the
@@ -431,7 +432,6 @@ template <class T, int kT = kBlock>
 __global__ void __launch_bounds__(kT) k_ghost_spans(GhostItems G, GhostSpans S, T *__restrict__ Q,
                                                     T *__restrict__ QC, const T *__restrict__ bcg,
                                                     const int *__restrict__ active) {
-  chain_trigger();
   const int t = blockIdx.x * kT + threadIdx.x;
   int off = S.off[0], b = 0, tot = 0;
   double hx = S.hx[0], hy = S.hy[0];
@@ -732,7 +732,6 @@ __global__ void __launch_bounds__(kBlock) k_relax_p(LevelD L, const RelaxChunkD 
                                                     FieldsT<T> f, const T *__restrict__ pack,
                                                     const Rule *__restrict__ perim, int m, T omega, int unit_omega,
                                                     int fresh, const uint8_t *__restrict__ cact, int amode) {
-  chain_trigger();
   constexpr int cpb = kBlock / kChunk;
   const int sub = threadIdx.x / kChunk, tc = threadIdx.x & (kChunk - 1);
   const int ngroups = (nchunks + cpb - 1) / cpb;
@@ -764,7 +763,6 @@ __global__ void __launch_bounds__(kBlock) k_relax_n(LevelD L, const RelaxChunkD 
                                                     FieldsT<T> f, const T *__restrict__ pack,
                                                     const Rule *__restrict__ perim, int m, T omega, int unit_omega,
                                                     int fresh, const uint8_t *__restrict__ cact, int amode) {
-  chain_trigger();
   constexpr int tpc = kChunk / kN;                    // threads per chunk
   const int ch = blockIdx.x * (kBlock / tpc) + threadIdx.x / tpc;
   const int t0 = threadIdx.x % tpc;
@@ -889,7 +887,6 @@ __global__ void __launch_bounds__(kT, (sizeof(T) == 4 ? 8 : 5) * (kBlock / kT))
     k_relax(LevelD L, const RelaxChunkD *__restrict__ chunks, int nchunks, FieldsT<T> f, const T *__restrict__ pack,
             const Rule *__restrict__ perim, int m, T omega, int unit_omega, int fresh,
             const uint8_t *__restrict__ cact, int amode) {
-  chain_trigger();
   relax_cell<T, kPow2, true>(L, chunks, nchunks, f, pack, perim, m, omega, unit_omega, fresh, cact, amode,
                              blockIdx.x * (kT / kChunk) + threadIdx.x / kChunk, threadIdx.x & (kChunk - 1));
 }
@@ -910,7 +907,6 @@ __global__ void __launch_bounds__(kClusterBlock, 1)
                     const T *__restrict__ pack, const Rule *__restrict__ perim, T omega, int unit_omega, int nsweeps,
                     int first_fresh, const uint8_t *__restrict__ cact, int amode, GhostItems G, int g_off, int g_n,
                     double hx_, double hy_) {
-  chain_trigger();
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   const int nth = (int)cl.num_blocks() * kClusterBlock;
@@ -1135,7 +1131,6 @@ __global__ void __launch_bounds__(kDsmBlock, 1)
                 const T *__restrict__ pack, const Rule *__restrict__ perim, T omega, int unit_omega, int nsweeps,
                 int first_fresh, const uint8_t *__restrict__ cact, int amode, GhostItems G, int g_off, int g_n,
                 double hx_, double hy_, int q0, int qn, int shift) {
-  chain_trigger();
   namespace cg = cooperative_groups;
   constexpr int kB = kDsmBlock;
   extern __shared__ __align__(16) unsigned char dsm_raw[];
@@ -1236,7 +1231,6 @@ __device__ __forceinline__ void restrict_item(const LevelD &L, const Decomp &D, 
 // SMs idle
 template <class T, int kT = kBlock>
 __global__ void __launch_bounds__(kT) k_restrict(LevelD L, Decomp D, FieldsT<T> f, int to_parent) {
-  chain_trigger();
   restrict_item<T, true>(L, D, f, to_parent, blockIdx.x * kT + threadIdx.x);
 }
 
@@ -1265,7 +1259,6 @@ __global__ void __launch_bounds__(kT) k_restrict_fill(LevelD L, Decomp D, Fields
                                                      const int *__restrict__ inst_nlev, int need, int f_off, int f_n,
                                                      int nb_f, int f_ring, double fhx, double fhy, int z_lo,
                                                      int z_n) {
-  chain_trigger();
   if ((int)blockIdx.x < nb_r) {
     restrict_item<T, true>(L, D, f, to_parent, blockIdx.x * kT + threadIdx.x);
     return;
@@ -1529,7 +1522,6 @@ template <class T, bool kPow2, int kT = kBlock>
 __global__ void __launch_bounds__(kT) k_load(LevelD L, LevelD Lc, Decomp D, FieldsT<T> f, const int *__restrict__ ring,
                                              const int *__restrict__ ring_inst, int ring_off, int n_ring, CorrCSR C,
                                              int n_tgt) {
-  chain_trigger();
   const int nb_ring = (n_ring + kT - 1) / kT;
   const int nb_fp = (D.n + kT - 1) / kT;
   int b = blockIdx.x;
@@ -1638,7 +1630,6 @@ __device__ __forceinline__ void prolong_item(const LevelD &L, const Decomp &D, c
 
 template <class T, int kT = kBlock>
 __global__ void __launch_bounds__(kT) k_prolong(LevelD L, Decomp D, FieldsT<T> f, int correct) {
-  chain_trigger();
   prolong_item<T, true>(L, D, f, correct, blockIdx.x * kT + threadIdx.x);
 }
 
@@ -1652,7 +1643,6 @@ __global__ void __launch_bounds__(kT) k_fill_prolong(GhostItems G, int g_off, in
                                                     FieldsT<T> f, int correct, WindowGhosts<T> W,
                                                     const int *__restrict__ active,
                                                     const int *__restrict__ inst_nlev) {
-  chain_trigger();
   if ((int)blockIdx.x < nb_g) {
     const int t = blockIdx.x * kT + threadIdx.x;
     const int i = g_off + t;
@@ -1725,7 +1715,6 @@ template <class T, int kRows = 1>
 __global__ void __launch_bounds__(32 * kRows) k_coarsest(const double *__restrict__ Ainv,
                                                          const double *__restrict__ bcRhs,
                                                          const CoarsestD *__restrict__ cd, FieldsT<T> f) {
-  chain_trigger();
   const CoarsestD D = cd[blockIdx.y];
   coarsest_row<T, true>(Ainv, bcRhs, D, f, blockIdx.x * kRows + (int)(threadIdx.x >> 5), threadIdx.x & 31);
 }
@@ -1791,7 +1780,6 @@ __global__ void __launch_bounds__(kT) k_residual(const LevelX *__restrict__ X, c
                                                  const ResTask *__restrict__ tasks, int ntask, Fields f, double *slots,
                                                  int nslots, unsigned long long *norms, int want_fn, int mass_corr,
                                                  float *__restrict__ rout) {
-  chain_trigger();
   const int w = blockIdx.x * (kT / 32) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   // a frozen instance's residual is neither reported nor needed, so its
@@ -1952,7 +1940,7 @@ __global__ void __launch_bounds__(kStep) k_solve_step(const InstRes *__restrict_
                                                       const int *__restrict__ crange, int nlev, uint8_t *cact,
                                                       cudaGraphConditionalHandle c0, cudaGraphConditionalHandle c1,
                                                       int ncond) {
-  chain_in();
+  chain_wait();
   int any = 0;
   for (int i = threadIdx.x; i < ninst; i += kStep) {
     if (mode != 0 && !active[i]) continue;
@@ -1993,7 +1981,7 @@ constexpr int kFinal = 512;
 __global__ void __launch_bounds__(kFinal) k_residual_final(const InstRes *__restrict__ ir,
                                                           const SlotRange *__restrict__ ranges, const double *slots,
                                                           int nslots, ResAcc *acc) {
-  chain_in();
+  chain_wait();
   const int inst = blockIdx.x, t = threadIdx.x;
   const InstRes R = ir[inst];
   double li = 0, fn = 0, l2sq = 0;
@@ -2059,7 +2047,6 @@ __global__ void __launch_bounds__(kBlock) k_fp64_rate(double *out, int iters, do
 // batch, one thread per cell over every patch of every level (a single
 // hierarchy copies the whole array instead).
 __global__ void __launch_bounds__(kBlock) k_freset(Decomp D, const PatchD *__restrict__ patches, Fields f) {
-  chain_trigger();
   const int g = blockIdx.x * kBlock + threadIdx.x;
   if (g >= D.n) {
     chain_wait();
@@ -2082,7 +2069,6 @@ __global__ void __launch_bounds__(kBlock) k_freset(Decomp D, const PatchD *__res
 // cells of every patch of the active instances.
 __global__ void __launch_bounds__(kBlock) k_update(Decomp D, const PatchD *__restrict__ patches, double *Q,
                                                    const float *__restrict__ E, const int *__restrict__ active) {
-  chain_trigger();
   const int g = blockIdx.x * kBlock + threadIdx.x;
   if (g >= D.n) {
     chain_wait();
@@ -2113,7 +2099,6 @@ __global__ void __launch_bounds__(kBlock) k_update(Decomp D, const PatchD *__res
 template <int kT = kBlock>
 __global__ void __launch_bounds__(kT) k_restrict_update(LevelD L, Decomp D, Fields f, const float *__restrict__ E,
                                                        int nb_r, Decomp Du, const PatchD *__restrict__ patches) {
-  chain_trigger();
   if ((int)blockIdx.x < nb_r) {
     const int g = blockIdx.x * kT + threadIdx.x;
     if (g >= D.n) {
@@ -2170,7 +2155,7 @@ __global__ void __launch_bounds__(kT) k_restrict_update(LevelD L, Decomp D, Fiel
 // BDF2 f + (2 Uo - 0.5 Uoo)/Dt, in that operation order; f null is f = 0.
 __global__ void __launch_bounds__(kBlock) k_history(Decomp D, const PatchD *__restrict__ patches, const double *Q,
                                                     double *Uo, double *Uoo, int rotate) {
-  chain_in();
+  chain_wait();
   const int g = blockIdx.x * kBlock + threadIdx.x;
   if (g >= D.n) return;
   const int p = find_patch(D, blockIdx.x, g);
@@ -2195,7 +2180,7 @@ __global__ void __launch_bounds__(kBlock) k_history(Decomp D, const PatchD *__re
 __global__ void __launch_bounds__(kBlock) k_uoo_transfer(LevelD L, Decomp D, const int *__restrict__ fp,
                                                          const int *__restrict__ src_old,
                                                          const double *__restrict__ uoo_old, double *uoo) {
-  chain_in();
+  chain_wait();
   const int g = blockIdx.x * kBlock + threadIdx.x;
   if (g >= D.n) return;
   const int p = find_patch(D, blockIdx.x, g);
@@ -2222,7 +2207,7 @@ __global__ void __launch_bounds__(kBlock) k_uoo_transfer(LevelD L, Decomp D, con
 __global__ void __launch_bounds__(kBlock) k_prhs(Decomp D, const PatchD *__restrict__ patches, double *FTrue,
                                                  const double *__restrict__ fsrc, const double *__restrict__ Uo,
                                                  const double *__restrict__ Uoo, double dt, int bdf2) {
-  chain_in();
+  chain_wait();
   const int g = blockIdx.x * kBlock + threadIdx.x;
   if (g >= D.n) return;
   const int p = find_patch(D, blockIdx.x, g);
@@ -2331,7 +2316,7 @@ __global__ void __launch_bounds__(kBlock) k_tag_buffer(const uint8_t *__restrict
 
 // FP32 copy of an FP64 array (coefficient copies of the mixed form)
 __global__ void __launch_bounds__(kBlock) k_to_f32(const double *__restrict__ a, float *__restrict__ b, long long n) {
-  chain_in();
+  chain_wait();
   for (long long i = blockIdx.x * (long long)kBlock + threadIdx.x; i < n; i += (long long)gridDim.x * kBlock)
     b[i] = (float)a[i];
 }
@@ -2340,7 +2325,7 @@ __global__ void __launch_bounds__(kBlock) k_to_f32(const double *__restrict__ a,
 // Composite sums over visible cells (ebCompositeMean.m, ebMassCheck.m lhs):
 // per-block partials of sum(u), sum(C u - FTrue), sum(|FTrue|)
 __global__ void __launch_bounds__(kBlock) k_sums(LevelD L, Decomp D, Fields f, double *partials) {
-  chain_in();
+  chain_wait();
   const int g = blockIdx.x * kBlock + threadIdx.x;
   double su = 0, sm = 0, sa = 0, nv = 0;
   if (g < D.n) {
