@@ -70,6 +70,8 @@ struct FieldsT {
   const uint8_t *flags;        // bit0 covered by a finer level, bit1 correction target
   const int *win, *fp;         // window gathers, footprint scatters (2 ints/cell)
   const int *active;           // per instance: 1 while its V-cycles continue (below)
+  int lsh;                     // the launch's (finer) level lives at Q + lsh: 0, or its second copy
+                               // between the two relaxations of the tile form (tile.cuh)
 };
 // `active` is written only by k_solve_step, the last kernel of a launch
 // chain, and the host synchronises before the next chain (or writes it with
@@ -305,6 +307,7 @@ __device__ __forceinline__ void ghost_item(const GhostItems &G, int i, int8_t ty
 struct GhostAlt {
   const int *a, *b, *c;        // operand slots (d and e are parent cells: never restricted)
   const int2 *rt;              // (first fine cell in Q, fine row stride)
+  int sh;                      // where the finer level lives (FieldsT::lsh)
 };
 
 struct GhostPrep {
@@ -342,7 +345,7 @@ template <class T, bool kCG, bool kAlt>
 __device__ __forceinline__ T ghost_operand(const T *Q, int code, const GhostAlt *A) {
   if (kAlt && code < 0) {
     const int2 r = __ldg(A->rt + (-1 - code));
-    const T *q = Q + r.x;
+    const T *q = Q + r.x + A->sh;
     return T(0.25) * (((ld_sol<kCG>(q) + ld_sol<kCG>(q + 1)) + ld_sol<kCG>(q + r.y)) + ld_sol<kCG>(q + r.y + 1));
   }
   return ld_sol<kCG>(Q + code);
@@ -370,6 +373,38 @@ __device__ __forceinline__ T ghost_value(const GhostPrep &P, const T *Q, const T
   const T qd = ld_sol<kCG>(Q + P.d), qe = ld_sol<kCG>(Q + P.e);
   const T g = P.g >= 0 ? bcg[P.g] : T(0);
   return ghost_formula<T>(P.ty, qa, qb, qc, qd, qe, g, P.nb, hx, hy);
+}
+
+// A level's own fill where the level lives at Q + sh: operands inside the
+// level's range [lo, lo + n) of Q and the ghosts move by sh, parent cells
+// (and a ring refresh's) do not.  kZero: parent cells hold 0 (k_restrict_fill).
+struct GhostHome {
+  int lo, n, sh;
+};
+template <class T, bool kZero>
+__device__ __forceinline__ void ghost_apply_home(const GhostItems &G, const GhostPrep &P, int i, T *Q, T *QC,
+                                                 const T *bcg, T hx, T hy, const GhostHome &M, bool zero) {
+  auto op = [&](int j) -> T {
+    if ((unsigned)(j - M.lo) < (unsigned)M.n) return Q[j + M.sh];
+    return kZero && zero ? T(0) : Q[j];
+  };
+  auto value = [&](const GhostPrep &R) -> T {
+    return ghost_formula<T>(R.ty, op(R.a), op(R.b), op(R.c), op(R.d), op(R.e), R.g >= 0 ? bcg[R.g] : T(0), R.nb, hx,
+                            hy);
+  };
+  if (P.ty == G_RING) {
+    QC[P.dst] = Q[P.a];
+    return;
+  }
+  T v;
+  if (P.ty == G_PHYS_CORNER) {
+    const int r1 = G.a[i], r2 = G.b[i];
+    const T v1 = value(ghost_prep(G, r1, G.type[r1], 0)), v2 = value(ghost_prep(G, r2, G.type[r2], 0));
+    v = (v1 + v2) - op(G.c[i]);
+  } else {
+    v = value(P);
+  }
+  Q[P.dst + M.sh] = v;
 }
 
 template <class T, bool kCG = false, bool kAlt = false>
@@ -401,7 +436,7 @@ template <class T, int kT = kBlock>
 __global__ void __launch_bounds__(kT) k_ghost(GhostItems G, int off, int n, T *__restrict__ Q, T *__restrict__ QC,
                                               const T *__restrict__ bcg, double hx_, double hy_,
                                               const int *__restrict__ active, const int *__restrict__ inst_nlev,
-                                              int need) {
+                                              int need, GhostHome M) {
   const int t = blockIdx.x * kT + threadIdx.x;
   const int i = off + t;
   // a converged instance of a batch stays frozen; a fill that follows the
@@ -413,7 +448,7 @@ __global__ void __launch_bounds__(kT) k_ghost(GhostItems G, int off, int n, T *_
   if (!skip) P = ghost_prep(G, i, G.type[i], G.dst[i]);
   chain_wait();
   if (skip) return;
-  ghost_apply<T>(G, i, P, Q, QC, bcg, T(hx_), T(hy_));
+  ghost_apply_home<T, false>(G, P, i, Q, QC, bcg, T(hx_), T(hy_), M, false);
 }
 
 // Ghost fills of several levels in one launch: span s holds the items
@@ -1222,7 +1257,7 @@ __device__ __forceinline__ void restrict_item(const LevelD &L, const Decomp &D, 
   const int cj = s / cmx, ci = s - cj * cmx;
   const int dst = to_parent ? __ldg(f.fp + 2 * (P.fp_off + s)) : 0;
   if (kChain) chain_wait();
-  const T R = restrict_cell<T>(f.Q + q_off, ldq, ci, cj);
+  const T R = restrict_cell<T>(f.Q + q_off + f.lsh, ldq, ci, cj);
   f.QC[qc_off + (ci + 1) + (cj + 1) * (cmx + 2)] = R;
   if (to_parent) f.Q[dst] = R;
 }
@@ -1248,7 +1283,7 @@ __global__ void __launch_bounds__(kT) k_restrict(LevelD L, Decomp D, FieldsT<T> 
 // with f_ring.  The host allows it on a level whose fill reads no cell the
 // restriction or the parent's fill writes, and whose ghost cells the
 // parent's fill does not read.  In the FP32 correction cycle it runs on
-// every level in the zero-parent form (z_n > 0): the correction starts at 0
+// every level in the zero-parent form (f_zero): the correction starts at 0
 // and level k-1 is first written by this very launch, so every parent-level
 // operand of level k's pre-smoothing fill is 0, which the items use instead
 // of reading cells the launch may be writing.
@@ -1257,8 +1292,8 @@ __global__ void __launch_bounds__(kT) k_restrict_fill(LevelD L, Decomp D, Fields
                                                      GhostItems G, GhostAlt A, int g_off, int g_n, double hx_,
                                                      double hy_, const int *__restrict__ active,
                                                      const int *__restrict__ inst_nlev, int need, int f_off, int f_n,
-                                                     int nb_f, int f_ring, double fhx, double fhy, int z_lo,
-                                                     int z_n) {
+                                                     int nb_f, int f_ring, double fhx, double fhy, GhostHome M,
+                                                     int f_zero) {
   if ((int)blockIdx.x < nb_r) {
     restrict_item<T, true>(L, D, f, to_parent, blockIdx.x * kT + threadIdx.x);
     return;
@@ -1273,27 +1308,7 @@ __global__ void __launch_bounds__(kT) k_restrict_fill(LevelD L, Decomp D, Fields
     if (!skip) P = ghost_prep(G, i, ty, G.dst[i]);
     chain_wait();
     if (skip) return;
-    if (z_n <= 0) {
-      ghost_apply<T>(G, i, P, f.Q, f.QC, f.bcg, T(fhx), T(fhy));
-      return;
-    }
-    // zero-parent form: an operand outside level k's range [z_lo, z_lo + z_n)
-    // is a parent-level cell, which holds 0 here (below) -- the value it had
-    // before this launch's restriction and parent fill wrote any of them
-    const T hx = T(fhx), hy = T(fhy);
-    auto op = [&](int n) -> T { return (unsigned)(n - z_lo) < (unsigned)z_n ? f.Q[n] : T(0); };
-    auto rule = [&](int j) -> T {
-      const GhostPrep R = ghost_prep(G, j, G.type[j], 0);
-      return ghost_formula<T>(R.ty, op(R.a), op(R.b), op(R.c), op(R.d), op(R.e), R.g >= 0 ? f.bcg[R.g] : T(0),
-                              R.nb, hx, hy);
-    };
-    if (P.ty == G_PHYS_CORNER) {
-      const T v1 = rule(G.a[i]), v2 = rule(G.b[i]);
-      f.Q[P.dst] = (v1 + v2) - op(G.c[i]);
-    } else {
-      f.Q[P.dst] = ghost_formula<T>(P.ty, op(P.a), op(P.b), op(P.c), op(P.d), op(P.e),
-                                    P.g >= 0 ? f.bcg[P.g] : T(0), P.nb, hx, hy);
-    }
+    ghost_apply_home<T, true>(G, P, i, f.Q, f.QC, f.bcg, T(fhx), T(fhy), M, f_zero != 0);
     return;
   }
   const int t = ((int)blockIdx.x - nb_r - nb_f) * kT + threadIdx.x;
@@ -1320,7 +1335,7 @@ __device__ __forceinline__ double face_corr(const PatchD &P, const FieldsT<T> &f
                                             const DivC &hc2, bool qc_inner) {
   const int mx = P.mx, my = P.my, cmx = mx >> 1, cmy = my >> 1;
   const int ldq = mx + 2, ldc = cmx + 2;
-  const T *Q = f.Q + P.q_off, *QC = f.QC + P.qc_off;
+  const T *Q = f.Q + P.q_off + f.lsh, *QC = f.QC + P.qc_off;
   const int *win = f.win + P.win_off;
   const T *DeW = f.DeW + P.dew_off, *DnS = f.DnS + P.dns_off, *cfd = f.cfd + P.cfd_off;
   auto q = [&](int i) { return dbl(Q[i]); };
@@ -1466,7 +1481,7 @@ __device__ __forceinline__ void load_fp_item(const LevelD &L, const LevelD &Lc, 
   }
   if (kChain) chain_wait();
   // the four fine cells and their eight neighbours: v[j][i], corners unused
-  const T *Qp = f.Q + q_off + 2 * ci + 2 * cj * ldq;
+  const T *Qp = f.Q + q_off + f.lsh + 2 * ci + 2 * cj * ldq;
   double v[4][4];
 #pragma unroll
   for (int j = 0; j < 4; ++j)
@@ -1613,7 +1628,7 @@ __device__ __forceinline__ void prolong_item(const LevelD &L, const Decomp &D, c
   const T f21 = (((9 * C + 3 * Wp) + 3 * Sm) + E[0][2]) / 16;
   const T f12 = (((9 * C + 3 * Wm) + 3 * Sp) + E[2][0]) / 16;
   const T f22 = (((9 * C + 3 * Wp) + 3 * Sp) + E[2][2]) / 16;
-  T *Q = f.Q + q_off;
+  T *Q = f.Q + q_off + f.lsh;
   const int c = (2 * a + 1) + (2 * b + 1) * ldq;
   if (correct) {
     Q[c] = Q[c] + f11;
@@ -1743,7 +1758,7 @@ __global__ void __launch_bounds__(32 * kRows) k_coarsest(const double *__restric
 //
 // Bound by the FP64 pipe and latency: about 13 operations per cell (19 with
 // every flux formed twice, the scaling by 1/h^2 on the FP64 pipe and the
-// squares): starfish 34 us -> @RES@ us per iteration, its floor at the
+// squares): starfish 34 us -> 18 us per iteration, its floor at the
 // measured FP64 rate 10 us.
 struct ResAcc {
   double out[5];        // linf, l2, fnorm, rel, ncell
@@ -1932,7 +1947,8 @@ struct SlotRange {
 // instance iterates.  mode 0 is the residual before the first V-cycle; mode 1
 // follows a V-cycle of the instances active during it.  One block, a thread
 // per instance: the former pair of kernels (a tree over one slot per task,
-// then the condition) took 14 + 2 us of a starfish iteration, this one @FIN@.
+// then the condition) and the turn of the loop took 21 us of a starfish
+// iteration, now 7, six of them the loop's own.
 constexpr int kStep = 256;
 __global__ void __launch_bounds__(kStep) k_solve_step(const InstRes *__restrict__ ir, int ninst,
                                                       unsigned long long *norms, ResAcc *acc, int *active, int *iters,

@@ -269,15 +269,17 @@ int bsam_launch_count(bsam_hier h, int64_t *count);
 /* The smoother's launch form per level as the autotuner chose it at the
  * first solve, levels 1..nlev in cells_per_thread[0..nlev-1], for
  * precision 0 (FP64 cycle) or 1 (FP32 correction cycle): 1, 2 or 4 colour
- * cells updated per thread, one launch per colour pass; 3 for one launch
+ * cells updated per thread, one launch per colour pass (1 also where a
+ * launch runs a whole relaxation's passes on tiles of the level, one colour
+ * cell per thread and pass); 3 for one launch
  * per pass of resident blocks that walk the level's chunks, the next
  * chunks' operands in flight during each update; 0 for the whole relaxation
  * (every pass and the closing ghost fill) in one launch of a single
  * thread-block cluster; 5 for the same with the level's solution held in
  * the cluster's distributed shared memory (levels whose Q range fits it);
  * -1 where that cycle has not run yet.  The choice never changes a result
- * bit; BSAM_RELAX_N=0|1|2|3|4|5 in the environment forces one form (5 where
- * it fits, else 1).  No reference counterpart (ebRelaxLevel.m has one loop
+ * bit; BSAM_RELAX_N=0|1|2|3|4|5|6 in the environment forces one form (5, and
+ * 6 for the tiles, where it fits, else 1).  No reference counterpart (ebRelaxLevel.m has one loop
  * order).                                                                 */
 int bsam_relax_tuning(bsam_hier h, int precision, int32_t *cells_per_thread, int cap);
 
