@@ -915,25 +915,28 @@ void launch_relax(bsam_hier h, int k, int nsweeps, bool first_fresh = false, boo
         }
         continue;
       }
-      // one chunk per block, the FP64 work over more SMs; the FP32 pass has
-      // little arithmetic, and fewer, larger blocks schedule faster once the
-      // level fills the SMs (starfish FP32 iteration 337 -> 326 us)
-      const int lim = sizeof(T) == sizeof(float) ? sm_count() : spread_limit(h);
-      if (grid < lim) {
-        if (L.pow2)
-          launch_k(h, k_relax<T, true, kChunk>, L.rc_n, kChunk, ld, ch, L.rc_n, f, pk, (const Rule *)h->perim.p, m,
-                   (T)h->opts.omega, unit, fresh, ca, am);
-        else
-          launch_k(h, k_relax<T, false, kChunk>, L.rc_n, kChunk, ld, ch, L.rc_n, f, pk, (const Rule *)h->perim.p, m,
-                   (T)h->opts.omega, unit, fresh, ca, am);
-        continue;
+      // smaller blocks where the kBlock grid would leave SMs idle or unevenly
+      // loaded.  FP64: 128 threads, few enough blocks to schedule and enough
+      // threads to share a rule list (starfish levels 4-7, us per pass with
+      // 64 / 128 / 256 threads: 2.84 / 2.40 / 2.57, 2.90 / 2.45 / 2.57,
+      // 3.54 / 3.22 / 3.42, 6.20 / 5.90 / 6.22).  The FP32 pass has little
+      // arithmetic, and fewer, larger blocks schedule faster once the level
+      // fills the SMs.
+      constexpr bool f32 = sizeof(T) == sizeof(float);
+      constexpr int kSmall = f32 ? kChunk : 2 * kChunk;
+      const bool small = grid < (f32 ? sm_count() : spread_limit(h));
+      const int kt = small ? kSmall : kBlock, g = (L.rc_n + kt / kChunk - 1) / (kt / kChunk);
+      auto go = [&](auto kern) {
+        launch_k(h, kern, g, kt, ld, ch, L.rc_n, f, pk, (const Rule *)h->perim.p, m, (T)h->opts.omega, unit, fresh, ca,
+                 am);
+      };
+      if (L.pow2) {
+        if (small) go(k_relax<T, true, kSmall>);
+        else go(k_relax<T, true>);
+      } else {
+        if (small) go(k_relax<T, false, kSmall>);
+        else go(k_relax<T, false>);
       }
-      if (L.pow2)
-        launch_k(h, k_relax<T, true>, grid, kBlock, ld, ch, L.rc_n, f, pk, (const Rule *)h->perim.p, m,
-                 (T)h->opts.omega, unit, fresh, ca, am);
-      else
-        launch_k(h, k_relax<T, false>, grid, kBlock, ld, ch, L.rc_n, f, pk, (const Rule *)h->perim.p, m,
-                 (T)h->opts.omega, unit, fresh, ca, am);
     }
   if (!defer_fill) launch_fill<T>(h, k);
 }
