@@ -321,6 +321,14 @@ Decomp decomp(bsam_hier h, const DecompH &D) {
 
 inline int nblk(int n) { return (n + kBlock - 1) / kBlock; }
 
+// levels of at least this many cells keep the FP64 pipe busy: their kernels
+// form products on the integer pipe (mul_int_pipe).  Smaller levels wait for
+// latency, where the multiply instruction is the shorter one.  FP64 smoother,
+// us per pass without / with: 16,384 cells 2.06 / 1.89, 33,668: 2.57 / 2.40,
+// 114,756: 3.15 / 2.78, 379,536: 5.87 / 5.19, 262,144 (one patch): 4.82 /
+// 3.59, 1,048,576: 11.8 / 9.06; but 4,096: 1.72 / 1.88, 11,328: 2.40 / 2.40.
+constexpr int64_t kIntMinCells = 16384;
+
 // kernels whose kBlock grid has fewer blocks than this run with 64-thread
 // (or one-chunk) blocks: an SM issues about two FP64 operations per clock,
 // so spreading a level's FP64 work over more SMs shortens the launch.  A
@@ -810,7 +818,14 @@ void launch_relax_tiles(bsam_hier h, int k, int nsweeps, bool first_fresh, bool 
   const int nl = ((nsweeps + kTileGroups - 1) / kTileGroups) | 1;
   const int unit = h->opts.omega == 1.0 ? 1 : 0;
   const T om = (T)h->opts.omega;
-  const size_t smem = tile_smem<T>(P.win_cap, P.cap, P.nf_cap);
+  // FP64: a block's passes share its SM's pipe with any other block there, so
+  // the blocks of a grid that covers a good part of the SMs ask for as much
+  // shared memory as spreads them evenly (starfish -1.4%; a handful of blocks
+  // only pays for the larger request: a 1,024-cell solve +2%)
+  size_t smem = tile_smem<T>(P.win_cap, P.cap, P.nf_cap);
+  const int per_sm = (P.ntiles + sm_count() - 1) / sm_count();
+  if (sizeof(T) == sizeof(double) && 4 * P.ntiles >= sm_count())
+    smem = std::max(smem, (size_t)std::min(kTileMaxBytes, 224 * 1024 / per_sm - 2048));
   T *a = f.Q, *b = f.Q + h->n_q;
   if (back) std::swap(a, b);
   for (int l = 0, done = 0; l < nl; ++l, std::swap(a, b)) {
@@ -930,6 +945,18 @@ void launch_relax(bsam_hier h, int k, int nsweeps, bool first_fresh = false, boo
         launch_k(h, kern, g, kt, ld, ch, L.rc_n, f, pk, (const Rule *)h->perim.p, m, (T)h->opts.omega, unit, fresh, ca,
                  am);
       };
+      if constexpr (!f32) {
+        if (L.ncells >= kIntMinCells) {
+          if (L.pow2) {
+            if (small) go(k_relax<T, true, kSmall, true>);
+            else go(k_relax<T, true, kBlock, true>);
+          } else {
+            if (small) go(k_relax<T, false, kSmall, true>);
+            else go(k_relax<T, false, kBlock, true>);
+          }
+          continue;
+        }
+      }
       if (L.pow2) {
         if (small) go(k_relax<T, true, kSmall>);
         else go(k_relax<T, true>);
@@ -1016,12 +1043,18 @@ void launch_coarse_load(bsam_hier h, int k, int home = 0) {
     launch_k(h, kern, nb(L.ring_n) + nb(D.n) + nb(ntgt), kt, leveld(h, k), leveld(h, k - 1), D, fields_at<T>(h, home),
              (const int *)h->ring.p, ri, L.ring_off, L.ring_n, corr_csr(h, L), ntgt);
   };
-  if (L.pow2 && h->lev[k - 1].pow2) {
-    if (spread) go(k_load<T, true, 64>);
-    else go(k_load<T, true>);
+  auto pick = [&](auto pow2, auto ints) {
+    constexpr bool p2 = decltype(pow2)::value, in = decltype(ints)::value;
+    if (spread) go(k_load<T, p2, in, 64>);
+    else go(k_load<T, p2, in>);
+  };
+  const bool p2 = L.pow2 && h->lev[k - 1].pow2;
+  if (L.ncells >= kIntMinCells) {
+    if (p2) pick(std::true_type{}, std::true_type{});
+    else pick(std::false_type{}, std::true_type{});
   } else {
-    if (spread) go(k_load<T, false, 64>);
-    else go(k_load<T, false>);
+    if (p2) pick(std::true_type{}, std::false_type{});
+    else pick(std::false_type{}, std::false_type{});
   }
 }
 
@@ -1181,15 +1214,23 @@ void launch_residual(bsam_hier h, int mode, const LoopCond &c = LoopCond()) {
     };
     const bool small = g256 < spread_limit(h);
     const int g64 = (h->nres + 1) / 2;
+    auto pick = [&](auto l2, auto pow2, auto ints) {
+      constexpr bool a = decltype(l2)::value, p2 = decltype(pow2)::value, in = decltype(ints)::value;
+      if (small) go(k_residual<a, p2, in, 64>, g64, 64);
+      else go(k_residual<a, p2, in>, g256, kBlock);
+    };
+    const std::true_type y{};
+    const std::false_type n{};
+    const bool ints = h->n_cells >= kIntMinCells;
     if (mode == RES_REPORT) {
-      if (small) go(k_residual<true, false, 64>, g64, 64);
-      else go(k_residual<true, false>, g256, kBlock);
+      if (h->all_pow2) pick(y, y, y);
+      else pick(y, n, y);
     } else if (h->all_pow2) {
-      if (small) go(k_residual<false, true, 64>, g64, 64);
-      else go(k_residual<false, true>, g256, kBlock);
+      if (ints) pick(n, y, y);
+      else pick(n, y, n);
     } else {
-      if (small) go(k_residual<false, false, 64>, g64, 64);
-      else go(k_residual<false, false>, g256, kBlock);
+      if (ints) pick(n, n, y);
+      else pick(n, n, n);
     }
   }
   if (mode == RES_RHS) return;

@@ -46,6 +46,50 @@ __device__ __forceinline__ T ld_sol(const T *p) {
   else return *p;
 }
 
+// A double product on the integer pipe, correctly rounded (to nearest, ties to
+// even): the 53-bit significands' product from four 32-bit multiply-adds,
+// one bit of normalisation, rounding by a carry.  Operands that are zero,
+// denormal, infinite or NaN and results near the ends of the exponent range
+// take the multiply instruction.  GB300 starts a warp's FP64 operation every
+// 19 cycles per SM and four warps' integer operations every cycle, so a
+// kernel bound by the FP64 pipe gains from moving products over: the
+// smoother's update (five products, four additions) ran at 55.9 G/s with
+// none, 99.0 with four and 104.1 with five of its products formed this way.
+__device__ __noinline__ double mul_fp64_pipe(double a, double b) { return a * b; }
+__device__ __forceinline__ double mul_int_pipe(double a, double b) {
+  const unsigned ah = (unsigned)__double2hiint(a), al = (unsigned)__double2loint(a);
+  const unsigned bh = (unsigned)__double2hiint(b), bl = (unsigned)__double2loint(b);
+  // significands: a's in 53 bits, b's at the top of 64
+  const unsigned a1 = (ah & 0xfffffu) | 0x100000u;
+  const unsigned b1 = __funnelshift_l(bl, (bh & 0xfffffu) | 0x100000u, 11), b0 = bl << 11;
+  const uint64_t p = (uint64_t)al * b0;
+  const uint64_t t = (uint64_t)al * b1 + (p >> 32);
+  const uint64_t u = (uint64_t)a1 * b0 + (uint32_t)t;
+  const uint64_t hi = (uint64_t)a1 * b1 + (t >> 32) + (u >> 32);   // in [2^51, 2^53)
+  const unsigned hh = (unsigned)(hi >> 32), hl = (unsigned)hi, l1 = (unsigned)u, l0 = (unsigned)p;
+  const unsigned n = (~hh >> 20) & 1u;                             // below 2^52: one bit more
+  const unsigned h1 = __funnelshift_l(hl, hh, n), h0 = __funnelshift_l(l1, hl, n), r = __funnelshift_l(l0, l1, n);
+  const unsigned rest = r | ((l0 << n) ? 1u : 0u);                 // what is cut off, its tail as one bit
+  uint64_t m = ((uint64_t)h1 << 32) | h0;
+  m += ((uint64_t)rest + 0x7fffffffu + (h0 & 1u)) >> 32;
+  const unsigned ea = ah & 0x7ff00000u, eb = bh & 0x7ff00000u;
+  const unsigned e = ea + eb - (1023u << 20) - (n << 20);          // the result's exponent field minus one
+  double q = __hiloint2double((int)(((unsigned)(m >> 32) + e) ^ ((ah ^ bh) & 0x80000000u)), (int)(unsigned)m);
+  const bool in = ea - 0x00100000u < 0x7fe00000u && eb - 0x00100000u < 0x7fe00000u && (int)e >= 0x00100000 &&
+                  (int)e < 0x7fd00000;
+  if (!in) q = mul_fp64_pipe(a, b);
+  return q;
+}
+// the product on the pipe of choice
+template <bool kInt>
+__device__ __forceinline__ double mul_on(double a, double b) {
+  return kInt ? mul_int_pipe(a, b) : a * b;
+}
+template <bool kInt>
+__device__ __forceinline__ float mul_on(float a, float b) {
+  return a * b;
+}
+
 // per-patch metadata on the device
 struct PatchD {
   int mx, my, par0, level;
@@ -133,9 +177,9 @@ __device__ __noinline__ double div_out_of_line(double x, double d) { return x / 
 
 // kPow2: the kernel's variant for levels where every constant is a power of
 // two (ops 1), which carries none of the other code
-template <bool kPow2>
+template <bool kPow2, bool kInt = false>
 __device__ __forceinline__ double div_c(double x, const DivC &D) {
-  const double q0 = x * D.r;
+  const double q0 = mul_on<kInt>(x, D.r);
   if (kPow2 || D.ops == 1) return q0;
   double q = __fma_rn(__fma_rn(-q0, D.d, x), D.r, q0);
   if (D.ops == 5) q = __fma_rn(__fma_rn(-q, D.d, x), D.r, q);
@@ -165,7 +209,7 @@ __device__ __forceinline__ void scale_faces(double (&c)[kN], const DivC &D, bool
 
 // FP32: a divide is short there (with the steps above the ragged mixed solve
 // was 2% slower)
-template <bool kPow2>
+template <bool kPow2, bool kInt = false>
 __device__ __forceinline__ float div_c(float x, float d) { return x / d; }
 
 struct LevelD {
@@ -195,11 +239,11 @@ __device__ __forceinline__ int find_patch(const Decomp &D, int b, int g) {
 
 // op2d (ebKernels.m:13-25) at one cell from its face fluxes (kPow2: formed
 // with scale_faces' coefficients)
-template <bool kPow2>
+template <bool kPow2, bool kInt = false>
 __device__ __forceinline__ double op_flux(double feE, double feW, double fnN, double fnS, double cc, double q,
                                           const LevelD &L) {
-  if (kPow2) return (-(feE - feW) - (fnN - fnS)) + cc * q;
-  return (div_c<false>(-(feE - feW), L.dx) - div_c<false>(fnN - fnS, L.dy)) + cc * q;
+  if (kPow2) return (-(feE - feW) - (fnN - fnS)) + mul_on<kInt>(cc, q);
+  return (div_c<false, kInt>(-(feE - feW), L.dx) - div_c<false, kInt>(fnN - fnS, L.dy)) + mul_on<kInt>(cc, q);
 }
 
 // the same from its values and (unscaled) coefficients
@@ -927,7 +971,8 @@ __global__ void __launch_bounds__(kBlock) k_relax_n(LevelD L, const RelaxChunkD 
 // kT threads per block: kBlock, or fewer on a level whose kBlock grid would
 // leave SMs idle -- an SM issues about two FP64 operations per clock, so a
 // block's FP64 work is spread over more SMs.
-template <class T, bool kPow2, int kT = kBlock>
+// kInt: four of the five products on the integer pipe (mul_int_pipe)
+template <class T, bool kPow2, int kT = kBlock, bool kInt = false>
 __global__ void __launch_bounds__(kT, (sizeof(T) == 4 ? 8 : 5) * (kBlock / kT))
     k_relax(LevelD L, const RelaxChunkD *__restrict__ chunks, int nchunks, FieldsT<T> f, const T *__restrict__ pack,
             const Rule *__restrict__ perim, int m, T omega, int unit_omega, int fresh,
@@ -1036,15 +1081,15 @@ __global__ void __launch_bounds__(kT, (sizeof(T) == 4 ? 8 : 5) * (kBlock / kT))
     }
   }
   if (kPow2) {
-    v = v + qe * S.dE;
-    v = v + qw * S.dW;
-    v = v + qn * S.dN;
-    v = v + qs * S.dS;
+    v = v + mul_on<kInt>(qe, S.dE);
+    v = v + mul_on<kInt>(qw, S.dW);
+    v = v + mul_on<kInt>(qn, S.dN);
+    v = v + mul_on<kInt>(qs, S.dS);
   } else {
-    v = v + div_c<false>(qe * S.dE, H.dx);
-    v = v + div_c<false>(qw * S.dW, H.dx);
-    v = v + div_c<false>(qn * S.dN, H.dy);
-    v = v + div_c<false>(qs * S.dS, H.dy);
+    v = v + div_c<false, kInt>(mul_on<kInt>(qe, S.dE), H.dx);
+    v = v + div_c<false, kInt>(mul_on<kInt>(qw, S.dW), H.dx);
+    v = v + div_c<false, kInt>(mul_on<kInt>(qn, S.dN), H.dy);
+    v = v + div_c<false, kInt>(mul_on<kInt>(qs, S.dS), H.dy);
   }
   v = v * S.idg;
   if (unit_omega) f.Q[c] = v;
@@ -1546,7 +1591,7 @@ __device__ __forceinline__ void load_ring_item(const FieldsT<T> &f, const int *_
   if (on) f.QC[dst] = f.Q[src];
 }
 
-template <class T, bool kPow2, bool kChain>
+template <class T, bool kPow2, bool kInt, bool kChain>
 __device__ __forceinline__ void load_fp_item(const LevelD &L, const LevelD &Lc, const Decomp &D, const FieldsT<T> &f,
                                              int g) {
   if (g >= D.n) {
@@ -1618,15 +1663,15 @@ __device__ __forceinline__ void load_fp_item(const LevelD &L, const LevelD &Lc, 
   for (int j = 0; j < 2; ++j)
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-      fx[j][i] = dx[3 * j + i] * (v[j + 1][i + 1] - v[j + 1][i]);
-      fy[i][j] = dy[2 * i + j] * (v[i + 1][j + 1] - v[i][j + 1]);
+      fx[j][i] = mul_on<kInt>(dx[3 * j + i], v[j + 1][i + 1] - v[j + 1][i]);
+      fy[i][j] = mul_on<kInt>(dy[2 * i + j], v[i + 1][j + 1] - v[i][j + 1]);
     }
   const T *Fp = f.F + c_off + 2 * ci + 2 * cj * mx;
 #pragma unroll
   for (int t = 0; t < 4; ++t) {
     const int i = t & 1, j = t >> 1;
     rf[t] = dbl(Fp[i + j * mx]) -
-            op_flux<kPow2>(fx[j][i + 1], fx[j][i], fy[j + 1][i], fy[j][i], cf[t], v[j + 1][i + 1], L);
+            op_flux<kPow2, kInt>(fx[j][i + 1], fx[j][i], fy[j + 1][i], fy[j][i], cf[t], v[j + 1][i + 1], L);
   }
   const double rr = 0.25 * (((rf[0] + rf[1]) + rf[2]) + rf[3]);
   const T *QC = f.QC + qc_off;
@@ -1657,7 +1702,7 @@ __device__ __forceinline__ void load_corr_item(const LevelD &L, const LevelD &Lc
 // kT threads per block (kBlock, or 64 on a level whose kBlock grid leaves
 // SMs idle: a footprint cell is ~84 FP64 operations, and an SM issues about
 // two per clock); the decomposition's per-block patch table is kBlock-based
-template <class T, bool kPow2, int kT = kBlock>
+template <class T, bool kPow2, bool kInt, int kT = kBlock>
 __global__ void __launch_bounds__(kT) k_load(LevelD L, LevelD Lc, Decomp D, FieldsT<T> f, const int *__restrict__ ring,
                                              const int *__restrict__ ring_inst, int ring_off, int n_ring, CorrCSR C,
                                              int n_tgt) {
@@ -1670,7 +1715,7 @@ __global__ void __launch_bounds__(kT) k_load(LevelD L, LevelD Lc, Decomp D, Fiel
   }
   b -= nb_ring;
   if (b < nb_fp) {
-    load_fp_item<T, kPow2, true>(L, Lc, D, f, b * kT + threadIdx.x);
+    load_fp_item<T, kPow2, kInt, true>(L, Lc, D, f, b * kT + threadIdx.x);
     return;
   }
   b -= nb_fp;
@@ -1914,7 +1959,7 @@ constexpr int kResRows = 4;
 
 // kT threads per block (kBlock, or 64 where the kBlock grid would leave
 // SMs with unequal shares of the FP64 work)
-template <bool kL2, bool kPow2, int kT = kBlock>
+template <bool kL2, bool kPow2, bool kInt, int kT = kBlock>
 __global__ void __launch_bounds__(kT) k_residual(const LevelX *__restrict__ X, const PatchD *__restrict__ patches,
                                                  const ResTask *__restrict__ tasks, int ntask, Fields f, double *slots,
                                                  int nslots, unsigned long long *norms, int want_fn, int mass_corr,
@@ -1971,15 +2016,16 @@ __global__ void __launch_bounds__(kT) k_residual(const LevelX *__restrict__ X, c
     }
     chain_wait();
     const double *Q = f.Q + P.q_off + (lx + 1) + (lj0 + 1) * ldq;
-    double q = Q[0], fs = dN[0] * (q - Q[-ldq]);
+    double q = Q[0], fs = mul_on<kInt>(dN[0], q - Q[-ldq]);
 #pragma unroll
     for (int u = 0; u < kResRows; ++u) {
       if (u >= rows) break;
       const double *Qu = Q + u * ldq;
       const double qn = Qu[ldq];
-      const double feE = dE[u] * (Qu[1] - q), feW = dW[u] * (q - Qu[-1]), fnN = dN[u + 1] * (qn - q);
+      const double feE = mul_on<kInt>(dE[u], Qu[1] - q), feW = mul_on<kInt>(dW[u], q - Qu[-1]);
+      const double fnN = mul_on<kInt>(dN[u + 1], qn - q);
       if (!((fl[u] & 1) || (mass_corr && (fl[u] & 2)))) {
-        const double r = ft[u] - op_flux<kPow2>(feE, feW, fnN, fs, cf[u], q, Xk.L);
+        const double r = ft[u] - op_flux<kPow2, kInt>(feE, feW, fnN, fs, cf[u], q, Xk.L);
         take(r, ft[u]);
         if (rout) rout[cc + u * mx] = (float)r;
       }
