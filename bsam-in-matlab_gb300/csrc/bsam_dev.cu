@@ -636,20 +636,28 @@ void launch_tile_k(bsam_hier h, int grid, size_t smem, Args... args) {
 
 // Tiles of level k for precision p: every patch cut into equal rectangles of
 // at most tw x th cells.  The tables are counted on the device with the
-// widest windows, which are then cut to the needed cells' bounds, and written
-// there.
-int build_tiles(bsam_hier h, int k, int p, int tw, int th) {
+// widest windows (begin_tiles), which are then cut to the needed cells'
+// bounds, and written there (end_tiles, after a synchronisation that several
+// levels share).
+struct TileCount {
+  int k = 0;
+  std::vector<TileD> tiles;
+  std::vector<TileTab> tab;
+  DBuf<int> chunk0, bad;
+  int hbad = 0;
+  TileBuild B{};
+};
+
+int begin_tiles(bsam_hier h, int k, int p, int tw, int th, TileCount &C) {
   LevelPlan &L = h->lev[k];
   TilePlan &P = L.tile[p];
+  C.k = 0;
   P.release();
   P.state = -1;
-  P.tw = tw;
-  P.th = th;
   if (tw < 1 || th < 1 || tw > kTileMax || th > kTileMax || 2 * h->n_q > INT32_MAX ||
       (int64_t)L.rc_n * 2 * kPackRows * kChunk > INT32_MAX)
     return BSAM_OK;
   const int halo = L.qif ? kTileHalo : kTilePasses;
-  std::vector<TileD> tiles;
   std::vector<int> chunk0;
   int ch = 0, pa = L.p0, pb = L.p0;
   for (int g = L.p0; g < L.p1; ++g) {
@@ -677,37 +685,43 @@ int build_tiles(bsam_hier h, int k, int p, int tw, int th) {
         d.mx = d.my = halo;
         d.wx = d.w + 2 * halo;
         d.wy = d.h + 2 * halo;
-        tiles.push_back(d);
+        C.tiles.push_back(d);
       }
   }
-  const size_t nt = tiles.size();
+  const size_t nt = C.tiles.size();
   P.ntiles = (int)nt;
   cudaStream_t s = h->stream;
-  std::vector<TileTab> tab(nt);
-  DBuf<int> dch, bad;
-  int rc, hbad = 0;
-  if ((rc = P.tiles.upload(tiles.data(), nt, s)) || (rc = dch.upload(chunk0.data(), chunk0.size(), s)) ||
-      (rc = bad.upload(&hbad, 1, s)) || (rc = P.tab.alloc(nt)))
+  C.tab.resize(nt);
+  int rc;
+  if ((rc = P.tiles.upload(C.tiles.data(), nt, s)) || (rc = C.chunk0.upload(chunk0.data(), chunk0.size(), s)) ||
+      (rc = C.bad.upload(&C.hbad, 1, s)) || (rc = P.tab.alloc(nt)))
     return rc;
-  TileBuild B{};
-  B.patches = h->patches.p + L.p0;
-  B.perim = h->perim.p;
-  B.tiles = P.tiles.p;
-  B.chunk0 = dch.p;
-  B.tab = P.tab.p;
-  B.q_lo = (int)L.q_lo;
-  B.q_hi = (int)L.q_hi;
-  B.bad = bad.p;
-  k_tile_build<false><<<(unsigned)nt, kTileBuildT, 0, s>>>(B);
+  C.B.patches = h->patches.p + L.p0;
+  C.B.perim = h->perim.p;
+  C.B.tiles = P.tiles.p;
+  C.B.chunk0 = C.chunk0.p;
+  C.B.tab = P.tab.p;
+  C.B.q_lo = (int)L.q_lo;
+  C.B.q_hi = (int)L.q_hi;
+  C.B.bad = C.bad.p;
+  k_tile_build<false><<<(unsigned)nt, kTileBuildT, 0, s>>>(C.B);
   CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(tab.data(), P.tab.p, sizeof(TileTab) * nt, cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(&hbad, bad.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-  CK(cudaStreamSynchronize(s));
+  CK(cudaMemcpyAsync(C.tab.data(), P.tab.p, sizeof(TileTab) * nt, cudaMemcpyDeviceToHost, s));
+  CK(cudaMemcpyAsync(&C.hbad, C.bad.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+  C.k = k;
+  return BSAM_OK;
+}
+
+int end_tiles(bsam_hier h, int p, TileCount &C) {
+  if (!C.k) return BSAM_OK;
+  TilePlan &P = h->lev[C.k].tile[p];
+  const size_t nt = C.tiles.size();
+  cudaStream_t s = h->stream;
   int64_t ne = 0, nf = 0, wq = 0;
   P.win_cap = P.cap = P.nf_cap = 0;
-  for (size_t i = 0; i < nt && !hbad; ++i) {
-    TileTab &x = tab[i];
-    TileD &d = tiles[i];
+  for (size_t i = 0; i < nt && !C.hbad; ++i) {
+    TileTab &x = C.tab[i];
+    TileD &d = C.tiles[i];
     const int n = x.nA[kTileGroups - 1] + x.nB[kTileGroups - 1];
     x.ent = (int)ne;
     x.face = (int)nf;
@@ -728,22 +742,20 @@ int build_tiles(bsam_hier h, int k, int p, int tw, int th) {
   P.cap = (P.cap + 3) & ~3;
   P.win_cap = (P.win_cap + 3) & ~3;
   const size_t smem = p ? tile_smem<float>(P.win_cap, P.cap, P.nf_cap) : tile_smem<double>(P.win_cap, P.cap, P.nf_cap);
-  if (!hbad && ne < INT32_MAX && nf < INT32_MAX && wq < INT32_MAX && smem <= (size_t)kTileMaxBytes) {
+  if (!C.hbad && ne < INT32_MAX && nf < INT32_MAX && wq < INT32_MAX && smem <= (size_t)kTileMaxBytes) {
+    int rc;
     if ((rc = P.ent.alloc(std::max<size_t>((size_t)ne, 1))) || (rc = P.face.alloc(std::max<size_t>((size_t)nf, 1))) ||
         (rc = P.wq.alloc((size_t)wq)))
       return rc;
-    CK(cudaMemcpyAsync(P.tab.p, tab.data(), sizeof(TileTab) * nt, cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(P.tiles.p, tiles.data(), sizeof(TileD) * nt, cudaMemcpyHostToDevice, s));
-    B.ent = P.ent.p;
-    B.face = P.face.p;
-    B.wq = P.wq.p;
-    k_tile_build<true><<<(unsigned)nt, kTileBuildT, 0, s>>>(B);
+    CK(cudaMemcpyAsync(P.tab.p, C.tab.data(), sizeof(TileTab) * nt, cudaMemcpyHostToDevice, s));
+    CK(cudaMemcpyAsync(P.tiles.p, C.tiles.data(), sizeof(TileD) * nt, cudaMemcpyHostToDevice, s));
+    C.B.ent = P.ent.p;
+    C.B.face = P.face.p;
+    C.B.wq = P.wq.p;
+    k_tile_build<true><<<(unsigned)nt, kTileBuildT, 0, s>>>(C.B);
     CK(cudaGetLastError());
     P.state = 1;
   }
-  dch.release();
-  bad.release();
-  CK(cudaStreamSynchronize(s));
   return BSAM_OK;
 }
 
@@ -781,13 +793,30 @@ void tile_size(bsam_hier h, int k, int p, int *tw, int *th) {
   }
 }
 
-// level k's tiles, built on first use; usable or not in state
-int ensure_tiles(bsam_hier h, int k, int p) {
-  TilePlan &P = h->lev[k].tile[p];
-  if (P.state) return BSAM_OK;
-  int tw, th;
-  tile_size(h, k, p, &tw, &th);
-  return build_tiles(h, k, p, tw, th);
+// the levels' tiles, built on first use; usable or not in their state
+int ensure_tiles(bsam_hier h, const std::vector<int> &levels, int p) {
+  std::vector<TileCount> C(levels.size());
+  int rc = BSAM_OK;
+  bool any = false;
+  for (size_t i = 0; i < levels.size() && !rc; ++i) {
+    const int k = levels[i];
+    if (h->lev[k].tile[p].state) continue;
+    int tw, th;
+    tile_size(h, k, p, &tw, &th);
+    rc = begin_tiles(h, k, p, tw, th, C[i]);
+    any = true;
+  }
+  // the counts are on the host; later, the tables' host copies may go
+  if (any) {
+    if (cudaStreamSynchronize(h->stream) != cudaSuccess && !rc) rc = cuda_fail(cudaGetLastError(), "tile tables");
+    for (size_t i = 0; i < levels.size() && !rc; ++i) rc = end_tiles(h, p, C[i]);
+    if (cudaStreamSynchronize(h->stream) != cudaSuccess && !rc) rc = cuda_fail(cudaGetLastError(), "tile tables");
+  }
+  for (TileCount &c : C) {
+    c.chunk0.release();
+    c.bad.release();
+  }
+  return rc;
 }
 
 // does level k's V-cycle run its relaxations in the tile form: chosen for the
@@ -1452,7 +1481,6 @@ int tune_level(bsam_hier h, int k, int *best) {
   *best = 1;
   const int ns = std::max(h->opts.npre, 1);
   std::vector<int> cand{1};
-  if (int rc = ensure_tiles(h, k, p)) return rc;
   if (h->lev[k].tile[p].state == 1) cand.push_back(6);
   h->lev[k].dsm_shift[p] = dsm_shift_for<T>(h, k);
   if (h->lev[k].dsm_shift[p] >= 0) cand.push_back(5);
@@ -1472,7 +1500,6 @@ int tune_level(bsam_hier h, int k, int *best) {
   return BSAM_OK;
 }
 
-int autotune(bsam_hier h);
 
 uint64_t tune_key(int precision, bool pow2, int chunks) {
   int b = 0;
@@ -1510,7 +1537,20 @@ int ensure_f32(bsam_hier h) {
   return BSAM_OK;
 }
 
-int autotune(bsam_hier h) {
+// the tables of the levels whose form is the tiles; a level that cannot take
+// them runs one launch per colour pass
+int take_tiles(bsam_hier h, int p) {
+  std::vector<int> &rn = h->relax_n[p], levels;
+  for (int k = 2; k <= h->nlev; ++k)
+    if (rn[k] == 6) levels.push_back(k);
+  if (int rc = ensure_tiles(h, levels, p)) return rc;
+  for (int k : levels)
+    if (h->lev[k].tile[p].state != 1) rn[k] = 1;
+  return BSAM_OK;
+}
+
+// cached_only: only if nothing has to be timed
+int autotune(bsam_hier h, bool cached_only = false) {
   const int p = mixed(h) ? 1 : 0;
   if (h->tuned[p]) return BSAM_OK;
   h->tuned[p] = true;
@@ -1527,10 +1567,8 @@ int autotune(bsam_hier h) {
     if (kn == 0 && cluster_ctas() == 0) kn = 1;
     rn.assign(h->nlev + 1, (kn >= 0 && kn <= 6) ? kn : 1);
     rn[1] = 1;
-    for (int k = 2; k <= h->nlev && kn == 6; ++k) {
-      if (int rc = ensure_tiles(h, k, p)) return rc;
-      if (h->lev[k].tile[p].state != 1) rn[k] = 1;
-    }
+    if (kn == 6)
+      if (int rc = take_tiles(h, p)) return rc;
     for (int k = 2; k <= h->nlev; ++k)
       if (rn[k] == 5 && !dsm_ok(k)) rn[k] = 1;
     return BSAM_OK;
@@ -1548,12 +1586,14 @@ int autotune(bsam_hier h) {
       else rn[k] = it->second == 5 && !dsm_ok(k) ? 1 : it->second;
     }
   }
-  for (int k = 2; k <= h->nlev; ++k)
-    if (rn[k] == 6) {
-      if (int rc = ensure_tiles(h, k, p)) return rc;
-      if (h->lev[k].tile[p].state != 1) rn[k] = 1;
-    }
+  if (!todo.empty() && cached_only) {
+    h->tuned[p] = false;
+    rn.assign(h->nlev + 1, 1);
+    return BSAM_OK;
+  }
+  if (int rc = take_tiles(h, p)) return rc;
   if (todo.empty()) return BSAM_OK;
+  if (int rc = ensure_tiles(h, todo, p)) return rc;
   // the FP64 smoother runs on the solution itself: keep a copy to put back
   // (the FP32 correction is zeroed at the start of every correction cycle)
   DBuf<double> keep;
@@ -2798,6 +2838,14 @@ int bsam_set_opts(bsam_hier h, const bsam_solve_opts *opts) {
   if (rc) return rc;
   const bool replan = opts->ghost_interp != h->opts.ghost_interp;
   if (replan) return fail(BSAM_ERR_STATE, "GhostInterp is fixed at upload; upload the hierarchy again");
+  // a driver sets the options before every step: unchanged ones keep the
+  // graphs and the reduction plan
+  const bsam_solve_opts &o = h->opts;
+  bool same = opts->npre == o.npre && opts->npost == o.npost && opts->omega == o.omega &&
+              opts->mass_correction == o.mass_correction && opts->max_vcycles == o.max_vcycles &&
+              opts->rel_tol == o.rel_tol && opts->precision == o.precision;
+  for (const InstRes &r : h->hir) same = same && r.max_vcycles == o.max_vcycles && r.rel_tol == o.rel_tol;
+  if (same) return BSAM_OK;
   h->opts = *opts;
   drop_graph(h);
   rc = set_device(h);
@@ -3071,6 +3119,8 @@ int bsam_solve_cycles(bsam_hier h, double *res_hist, int hist_cap, int *vcycles,
   int nactive = 0;
   bool on_device = false;
   const Synced synced(h);
+  // forms known from other hierarchies of this context: straight to the graph
+  if (!h->tuned[mixed(h) ? 1 : 0] && !host_loop() && (rc = autotune(h, true))) return rc;
   if (h->tuned[mixed(h) ? 1 : 0] && !host_loop() && build_solve_graph(h)) {
     // the whole solve in one graph launch (once the smoother is tuned)
     CK(cudaGraphLaunch(h->sexec, h->stream));
