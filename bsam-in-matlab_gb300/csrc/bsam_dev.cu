@@ -179,7 +179,8 @@ struct bsam_hier_s {
   // device arrays
   DBuf<double> Q, F, FTrue, QC, CC, ID, DeW, DnS, bcg, cfd, pcoef, Ainv, bcRhs, slots, partials, hist;
   DBuf<uint8_t> flags;
-  DBuf<int> win, fp, ring, ints, ct_cell, ct_patch, ct_beg, ct_item, ct_j, active, iters, ones;
+  DBuf<int> win, fp, ring, ints, ct_cell, ct_patch, ct_beg, active, iters, ones;
+  DBuf<CorrRec> ct_rec;
   DBuf<int> g_inst, ring_inst;     // instance per ghost item / ring entry (batches only)
   DBuf<int> inst_nlev;             // per instance: its finest level
   // mixed form: FP32 correction, its right-hand side and coarse shadows,
@@ -1054,7 +1055,7 @@ void launch_restrict_fill(bsam_hier h, int k, int fill_k = FILL_NONE, int need =
 }
 
 CorrCSR corr_csr(bsam_hier h, const LevelPlan &L) {
-  return CorrCSR{h->ct_cell.p + L.ct_off, h->ct_patch.p + L.ct_off, h->ct_beg.p + L.ct_off, h->ct_item.p, h->ct_j.p};
+  return CorrCSR{h->ct_cell.p + L.ct_off, h->ct_patch.p + L.ct_off, h->ct_beg.p + L.ct_off, h->ct_rec.p};
 }
 
 // ebTransfer 'ring' + ebCoarseLoad (ebVcycle.m:28-29) in one launch
@@ -1359,7 +1360,7 @@ void launch_consistent(bsam_hier h, bool top_restricted = false) {
 // instead of at the start of each: within a solve F is written only by the
 // coarse loads, over the parent footprint (recomputed every V-cycle before
 // any read) and at the flux-correction targets, whose value the load forms
-// from FTrue itself (load_corr_item); every other cell keeps FTrue.  So the
+// from FTrue itself (corr_value); every other cell keeps FTrue.  So the
 // F each V-cycle reads is the one the reference's per-cycle reset gives.
 void reset_force(bsam_hier h) {
   if (h->ninst == 1) {
@@ -2221,6 +2222,43 @@ int validate(const bsam_hier_desc *d) {
   return BSAM_OK;
 }
 
+// the operands of the correction of coarse face j on face fc (0 W, 1 E, 2 S,
+// 3 N) of the patch r (ebFaceCorrections.m:18-61)
+CorrRec corr_rec(const int32_t *r, const int32_t *win, int fc, int j) {
+  const int mx = r[PD_MX], my = r[PD_MY], cmx = mx / 2, cmy = my / 2, ld = mx + 2, ldc = cmx + 2;
+  const int qo = r[PD_QOFF];
+  const int32_t *w = win + r[PD_WIN0];
+  CorrRec c{};
+  c.ldq = ld;
+  c.yface = fc >= 2;
+  if (fc < 2) {
+    const int ia = fc == 0 ? 1 : mx, ib = fc == 0 ? 0 : mx + 1, ic = fc == 0 ? 0 : cmx - 1, face = fc == 0 ? 0 : mx;
+    c.a1 = qo + ia + (2 * j + 1) * ld;
+    c.b1 = qo + ib + (2 * j + 1) * ld;
+    c.a2 = c.a1 + ld;
+    c.b2 = c.b1 + ld;
+    c.out = w[(fc == 0 ? 0 : cmx + 1) + (j + 1) * ldc];
+    c.qc = r[PD_QCOFF] + (ic + 1) + (j + 1) * ldc;
+    c.in = qo + (2 * ic + 1) + (2 * j + 1) * ld;
+    c.c1 = r[PD_DEWOFF] + face + 2 * j * (mx + 1);
+    c.c2 = c.c1 + mx + 1;
+    c.cf = r[PD_CFDOFF] + (fc == 0 ? 0 : cmy) + j;
+  } else {
+    const int ja = fc == 2 ? 1 : my, jb = fc == 2 ? 0 : my + 1, jc = fc == 2 ? 0 : cmy - 1, face = fc == 2 ? 0 : my;
+    c.a1 = qo + (2 * j + 1) + ja * ld;
+    c.b1 = qo + (2 * j + 1) + jb * ld;
+    c.a2 = c.a1 + 1;
+    c.b2 = c.b1 + 1;
+    c.out = w[(j + 1) + (fc == 2 ? 0 : cmy + 1) * ldc];
+    c.qc = r[PD_QCOFF] + (j + 1) + (jc + 1) * ldc;
+    c.in = qo + (2 * j + 1) + (2 * jc + 1) * ld;
+    c.c1 = r[PD_DNSOFF] + 2 * j + face * mx;
+    c.c2 = c.c1 + 1;
+    c.cf = r[PD_CFDOFF] + 2 * cmy + (fc == 2 ? 0 : cmx) + j;
+  }
+  return c;
+}
+
 int do_upload(bsam_hier h, const bsam_hier_desc *d) {
   int rc = validate(d);
   if (rc) return rc;
@@ -2278,7 +2316,8 @@ int do_upload(bsam_hier h, const bsam_hier_desc *d) {
   B.pinst = pinst;
   h->lev.assign(d->nlev + 1, LevelPlan());
   std::vector<uint8_t> flags(d->covered, d->covered + d->n_cells);
-  std::vector<int> ct_cell, ct_patch, ct_beg, ct_item, ct_j;
+  std::vector<int> ct_cell, ct_patch, ct_beg;
+  std::vector<CorrRec> ct_rec;
   for (int k = 1; k <= d->nlev; ++k) {
     LevelPlan &L = h->lev[k];
     const int32_t *lv = d->levels + (size_t)(k - 1) * LDN;
@@ -2331,11 +2370,8 @@ int do_upload(bsam_hier h, const bsam_hier_desc *d) {
         if (q < 0) return fail(BSAM_ERR_ARG, "correction target is not a cell of the parent level");
         ct_cell.push_back(cell);
         ct_patch.push_back(q);
-        ct_beg.push_back((int)ct_item.size());
-        for (size_t t = i; t < e; ++t) {
-          ct_item.push_back(items[t].item);
-          ct_j.push_back(items[t].j);
-        }
+        ct_beg.push_back((int)ct_rec.size());
+        for (size_t t = i; t < e; ++t) ct_rec.push_back(corr_rec(B.P(L.p0 + (items[t].item >> 2)), d->win, items[t].item & 3, items[t].j));
         flags[cell] |= 2;
         i = e;
       }
@@ -2343,7 +2379,7 @@ int do_upload(bsam_hier h, const bsam_hier_desc *d) {
       // sentinel row so that tbeg[t + 1] exists for the level's last target
       ct_cell.push_back(0);
       ct_patch.push_back(0);
-      ct_beg.push_back((int)ct_item.size());
+      ct_beg.push_back((int)ct_rec.size());
     }
   }
   for (int p = 0; p < d->npatch; ++p) pd[p].pe_off = B.pe_off[p];
@@ -2411,7 +2447,20 @@ int do_upload(bsam_hier h, const bsam_hier_desc *d) {
         const int32_t *r = B.P(p);
         const int n = r[PD_MX] * r[PD_MY], nc = r[PD_MX] * ((r[PD_MY] + kResRows - 1) / kResRows);
         for (int c = 0; c < n; ++c) h->inst_visible[i] += (d->covered[r[PD_COFF] + c] == 0);
-        for (int b0 = 0; b0 < nc; b0 += 32) cells.push_back(ResTask{0, k, p, b0, std::min(32, nc - b0), ns++, i, 0});
+        // items all of whose cells a finer level covers contribute nothing
+        const uint8_t *cov = d->covered + r[PD_COFF];
+        auto visible = [&](int e) {
+          const int x = e % r[PD_MX], y0 = e / r[PD_MX] * kResRows;
+          for (int y = y0; y < std::min(y0 + kResRows, (int)r[PD_MY]); ++y)
+            if (!cov[x + y * r[PD_MX]]) return true;
+          return false;
+        };
+        for (int b0 = 0; b0 < nc; b0 += 32) {
+          const int n1 = std::min(32, nc - b0);
+          bool any = false;
+          for (int e = b0; e < b0 + n1 && !any; ++e) any = visible(e);
+          if (any) cells.push_back(ResTask{0, k, p, b0, n1, ns++, i, 0});
+        }
       }
       if (k < d->nlev) {
         const LevelPlan &Lf = h->lev[k + 1];
@@ -2618,7 +2667,7 @@ int do_upload(bsam_hier h, const bsam_hier_desc *d) {
       (rc = h->g_e.upload(B.ge.data(), B.ge.size(), s)) || (rc = h->ct_cell.upload(ct_cell.data(), ct_cell.size(), s)) ||
       (rc = h->ct_patch.upload(ct_patch.data(), ct_patch.size(), s)) ||
       (rc = h->ct_beg.upload(ct_beg.data(), ct_beg.size(), s)) ||
-      (rc = h->ct_item.upload(ct_item.data(), ct_item.size(), s)) || (rc = h->ct_j.upload(ct_j.data(), ct_j.size(), s)) ||
+      (rc = h->ct_rec.upload(ct_rec.data(), ct_rec.size(), s)) ||
       (rc = h->rtasks.upload(tasks.data(), tasks.size(), s)) || (rc = h->sranges.upload(ranges.data(), ranges.size(), s)) ||
       (rc = h->instres.upload(ir.data(), ir.size(), s)) || (rc = h->coarsest.upload(cds.data(), cds.size(), s)) ||
       (rc = h->slots.alloc(3 * (size_t)h->nslots)) || (rc = h->acc.alloc(h->ninst)) ||
@@ -2668,14 +2717,15 @@ void release(bsam_hier h) {
   for (DBuf<float> *b : {&h->E, &h->F32, &h->QC32, &h->DeW32, &h->DnS32, &h->CC32, &h->ID32, &h->pcoef32, &h->cfd32,
                          &h->bcg32, &h->rpack32})
     b->release();
-  for (DBuf<int> *b : {&h->win, &h->fp, &h->ring, &h->ints, &h->ct_cell, &h->ct_patch, &h->ct_beg, &h->ct_item,
-                       &h->ct_j, &h->active, &h->iters, &h->ones, &h->g_inst, &h->ring_inst, &h->inst_nlev, &h->g_dst, &h->g_a, &h->g_b, &h->g_c, &h->g_d, &h->g_e,
+  for (DBuf<int> *b : {&h->win, &h->fp, &h->ring, &h->ints, &h->ct_cell, &h->ct_patch, &h->ct_beg,
+                       &h->active, &h->iters, &h->ones, &h->g_inst, &h->ring_inst, &h->inst_nlev, &h->g_dst, &h->g_a, &h->g_b, &h->g_c, &h->g_d, &h->g_e,
                        &h->ga_a, &h->ga_b, &h->ga_c, &h->win_alt})
     b->release();
   h->flags.release(); h->g_type.release(); h->patches.release(); h->acc.release(); h->perim.release();
   h->rchunks.release(); h->pchunks.release(); h->cact.release(); h->crange.release(); h->levelx.release(); h->rtasks.release(); h->instres.release(); h->sranges.release();
   h->coarsest.release();
   h->norms.release();
+  h->ct_rec.release();
   h->ga_rt.release();
   h->flux_faces.release();
   for (LevelPlan &L : h->lev)

@@ -37,6 +37,11 @@ __device__ __forceinline__ void chain_wait() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// the wait of a kernel that writes operands which its successors read before
+// their own wait (coefficients, sources): no early trigger, so that the next
+// kernel starts when this one's stores are visible
+__device__ __forceinline__ void chain_wait_static() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // a solution load; kCG: from L2 (ld.global.cg), for kernels whose blocks
 // read values other blocks of the same launch wrote after a cluster barrier
 // (another SM's L1 may hold an older copy of the line)
@@ -316,30 +321,13 @@ __device__ __forceinline__ T eval_rule(const GhostItems &G, int i, const T *Q, c
   }
 }
 
-// one ghost item: its final value (or the QC ring refresh)
-template <class T, bool kCG = false>
-__device__ __forceinline__ void ghost_item(const GhostItems &G, int i, int8_t ty, int dst, T *Q, T *QC, const T *bcg,
-                                           T hx, T hy) {
-  if (ty == G_RING) {
-    QC[dst] = ld_sol<kCG>(Q + G.a[i]);
-  } else if (ty == G_PHYS_CORNER) {
-    // (face ghost 1 + face ghost 2) - interior, the face ghosts evaluated by
-    // their own final rules (ebFillGhosts.m:84-89 reads them after stage 3)
-    const T v1 = eval_rule<T, kCG>(G, G.a[i], Q, bcg, hx, hy);
-    const T v2 = eval_rule<T, kCG>(G, G.b[i], Q, bcg, hx, hy);
-    Q[dst] = (v1 + v2) - ld_sol<kCG>(Q + G.c[i]);
-  } else {
-    Q[dst] = eval_rule<T, kCG>(G, i, Q, bcg, hx, hy);
-  }
-}
-
 // A ghost item in two stages, so that every load it needs is in flight at
-// once: ghost_prep reads the item's static indices (before a kernel's
-// programmatic-launch wait), ghost_apply requests all of its solution
+// once: ghost_prep reads the item's static indices and boundary value (before
+// a kernel's programmatic-launch wait), ghost_apply requests all of its solution
 // operands and its boundary value before it looks at the rule's kind, so
 // the lanes of a warp that fill different kinds of ghosts wait for one round
 // of loads together.  Operand slots a kind does not read repeat its first
-// operand.  A physical corner evaluates its two face rules as ghost_item does.
+// operand.
 //
 // GhostAlt: the operands of a level's ghost items for the fill that follows
 // the restriction of the level above into it, fused into one launch with
@@ -354,15 +342,17 @@ struct GhostAlt {
   int sh;                      // where the finer level lives (FieldsT::lsh)
 };
 
+template <class T>
 struct GhostPrep {
   int8_t ty;
-  int dst, a, b, c, d, e, g, nb;   // g: boundary-data index (-1: none); nb: Neumann side flag
+  int dst, a, b, c, d, e;
+  T g;                         // a physical rule's boundary part: 8/3 g or h g
 };
 
-template <bool kAlt = false>
-__device__ __forceinline__ GhostPrep ghost_prep(const GhostItems &G, int i, int8_t ty, int dst,
-                                                const GhostAlt *A = nullptr) {
-  GhostPrep P;
+template <class T, bool kAlt = false>
+__device__ __forceinline__ GhostPrep<T> ghost_prep(const GhostItems &G, int i, int8_t ty, int dst, const T *bcg, T hx,
+                                                   T hy, const GhostAlt *A = nullptr) {
+  GhostPrep<T> P;
   P.ty = ty;
   P.dst = dst;
   const int a = kAlt ? __ldg(A->a + i) : __ldg(G.a + i);
@@ -378,9 +368,35 @@ __device__ __forceinline__ GhostPrep ghost_prep(const GhostItems &G, int i, int8
   const int pa = kAlt ? __ldg(G.a + i) : a;
   P.d = ue ? __ldg(G.d + i) : pa;
   P.e = ue ? __ldg(G.e + i) : pa;
-  P.g = (ty == G_DIRICHLET || ty == G_NEUMANN) ? __ldg(G.e + i) : -1;
-  P.nb = ty == G_NEUMANN ? __ldg(G.b + i) : 0;
+  P.g = T(0);
+  if (ty == G_DIRICHLET) P.g = T(8.0 / 3.0) * __ldg(bcg + __ldg(G.e + i));
+  else if (ty == G_NEUMANN) P.g = (__ldg(G.b + i) ? hy : hx) * __ldg(bcg + __ldg(G.e + i));
   return P;
+}
+
+// an item as a fill kernel holds it across its programmatic-launch wait: a
+// physical corner also holds its two face rules (their item and boundary
+// loads cost a corner's fill 0.5 us after the wait)
+template <class T>
+struct GhostPre {
+  GhostPrep<T> P, P1, P2;
+  int pc;                      // corner: the interior operand
+};
+template <class T, bool kAlt = false>
+__device__ __forceinline__ GhostPre<T> ghost_pre(const GhostItems &G, int i, int8_t ty, int dst, const T *bcg, T hx,
+                                                 T hy, const GhostAlt *A = nullptr) {
+  GhostPre<T> X;
+  if (ty == G_PHYS_CORNER) {
+    const int r1 = __ldg(G.a + i), r2 = __ldg(G.b + i);
+    X.P.ty = ty;
+    X.P.dst = dst;
+    X.pc = kAlt ? __ldg(A->c + i) : __ldg(G.c + i);
+    X.P1 = ghost_prep<T, kAlt>(G, r1, __ldg(G.type + r1), 0, bcg, hx, hy, A);
+    X.P2 = ghost_prep<T, kAlt>(G, r2, __ldg(G.type + r2), 0, bcg, hx, hy, A);
+  } else {
+    X.P = ghost_prep<T, kAlt>(G, i, ty, dst, bcg, hx, hy, A);
+  }
+  return X;
 }
 
 // a solution operand: a cell of Q, or (code < 0, fused fills only) the
@@ -395,28 +411,26 @@ __device__ __forceinline__ T ghost_operand(const T *Q, int code, const GhostAlt 
   return ld_sol<kCG>(Q + code);
 }
 
-// a ghost's value from its operands and boundary datum (eval_rule's
+// a ghost's value from its operands and boundary part (eval_rule's
 // arithmetic, every kind but the ring refresh and the physical corner)
 template <class T>
-__device__ __forceinline__ T ghost_formula(int ty, T qa, T qb, T qc, T qd, T qe, T g, int nb, T hx, T hy) {
-  const T c23 = T(2.0 / 3.0), c13 = T(1.0 / 3.0), c83 = T(8.0 / 3.0);
+__device__ __forceinline__ T ghost_formula(int ty, T qa, T qb, T qc, T qd, T qe, T g) {
+  const T c23 = T(2.0 / 3.0), c13 = T(1.0 / 3.0);
   switch (ty) {
     case G_LIF_CORNER: return c23 * qc + c13 * qa;
-    case G_DIRICHLET: return (c83 * g - 2 * qa) + c13 * qb;
-    case G_NEUMANN: return qa + (nb ? hy : hx) * g;
+    case G_DIRICHLET: return (g - 2 * qa) + c13 * qb;
+    case G_NEUMANN: return qa + g;
     default: return rule_value<T>(ty, qa, qb, qc, qd, qe);   // COPY, QIF, QIF_END, LIF
   }
 }
 
 // the value of a prepared item that is not a ring refresh or a corner
 template <class T, bool kCG, bool kAlt>
-__device__ __forceinline__ T ghost_value(const GhostPrep &P, const T *Q, const T *bcg, T hx, T hy,
-                                         const GhostAlt *A) {
+__device__ __forceinline__ T ghost_value(const GhostPrep<T> &P, const T *Q, const GhostAlt *A) {
   const T qa = ghost_operand<T, kCG, kAlt>(Q, P.a, A), qb = ghost_operand<T, kCG, kAlt>(Q, P.b, A);
   const T qc = ghost_operand<T, kCG, kAlt>(Q, P.c, A);
   const T qd = ld_sol<kCG>(Q + P.d), qe = ld_sol<kCG>(Q + P.e);
-  const T g = P.g >= 0 ? bcg[P.g] : T(0);
-  return ghost_formula<T>(P.ty, qa, qb, qc, qd, qe, g, P.nb, hx, hy);
+  return ghost_formula<T>(P.ty, qa, qb, qc, qd, qe, P.g);
 }
 
 // A level's own fill where the level lives at Q + sh: operands inside the
@@ -426,52 +440,36 @@ struct GhostHome {
   int lo, n, sh;
 };
 template <class T, bool kZero>
-__device__ __forceinline__ void ghost_apply_home(const GhostItems &G, const GhostPrep &P, int i, T *Q, T *QC,
-                                                 const T *bcg, T hx, T hy, const GhostHome &M, bool zero) {
+__device__ __forceinline__ void ghost_apply_home(const GhostPre<T> &X, T *Q, T *QC, const GhostHome &M, bool zero) {
   auto op = [&](int j) -> T {
     if ((unsigned)(j - M.lo) < (unsigned)M.n) return Q[j + M.sh];
     return kZero && zero ? T(0) : Q[j];
   };
-  auto value = [&](const GhostPrep &R) -> T {
-    return ghost_formula<T>(R.ty, op(R.a), op(R.b), op(R.c), op(R.d), op(R.e), R.g >= 0 ? bcg[R.g] : T(0), R.nb, hx,
-                            hy);
+  auto value = [&](const GhostPrep<T> &R) -> T {
+    return ghost_formula<T>(R.ty, op(R.a), op(R.b), op(R.c), op(R.d), op(R.e), R.g);
   };
-  if (P.ty == G_RING) {
-    QC[P.dst] = Q[P.a];
+  if (X.P.ty == G_RING) {
+    QC[X.P.dst] = Q[X.P.a];
     return;
   }
-  T v;
-  if (P.ty == G_PHYS_CORNER) {
-    const int r1 = G.a[i], r2 = G.b[i];
-    const T v1 = value(ghost_prep(G, r1, G.type[r1], 0)), v2 = value(ghost_prep(G, r2, G.type[r2], 0));
-    v = (v1 + v2) - op(G.c[i]);
-  } else {
-    v = value(P);
-  }
-  Q[P.dst + M.sh] = v;
+  // a corner: (face ghost 1 + face ghost 2) - interior, the face ghosts
+  // evaluated by their own final rules (ebFillGhosts.m:84-89 reads them after
+  // stage 3)
+  Q[X.P.dst + M.sh] = X.P.ty == G_PHYS_CORNER ? (value(X.P1) + value(X.P2)) - op(X.pc) : value(X.P);
 }
 
 template <class T, bool kCG = false, bool kAlt = false>
-__device__ __forceinline__ void ghost_apply(const GhostItems &G, int i, const GhostPrep &P, T *Q, T *QC, const T *bcg,
-                                            T hx, T hy, const GhostAlt *A = nullptr) {
-  if (P.ty == G_PHYS_CORNER) {
-    if (!kAlt) {
-      ghost_item<T, kCG>(G, i, P.ty, P.dst, Q, QC, bcg, hx, hy);
-      return;
-    }
-    // (face ghost 1 + face ghost 2) - interior, each face ghost by its own
-    // rule with the fused fill's operands
-    const int r1 = G.a[i], r2 = G.b[i];
-    const T v1 = ghost_value<T, kCG, true>(ghost_prep<true>(G, r1, G.type[r1], 0, A), Q, bcg, hx, hy, A);
-    const T v2 = ghost_value<T, kCG, true>(ghost_prep<true>(G, r2, G.type[r2], 0, A), Q, bcg, hx, hy, A);
-    Q[P.dst] = (v1 + v2) - ghost_operand<T, kCG, true>(Q, __ldg(A->c + i), A);
+__device__ __forceinline__ void ghost_apply(const GhostPre<T> &X, T *Q, T *QC, const GhostAlt *A = nullptr) {
+  if (X.P.ty == G_RING) {
+    QC[X.P.dst] = ld_sol<kCG>(Q + X.P.a);
     return;
   }
-  if (P.ty == G_RING) {
-    QC[P.dst] = ld_sol<kCG>(Q + P.a);
+  if (X.P.ty == G_PHYS_CORNER) {
+    const T v1 = ghost_value<T, kCG, kAlt>(X.P1, Q, A), v2 = ghost_value<T, kCG, kAlt>(X.P2, Q, A);
+    Q[X.P.dst] = (v1 + v2) - ghost_operand<T, kCG, kAlt>(Q, X.pc, A);
     return;
   }
-  Q[P.dst] = ghost_value<T, kCG, kAlt>(P, Q, bcg, hx, hy, A);
+  Q[X.P.dst] = ghost_value<T, kCG, kAlt>(X.P, Q, A);
 }
 
 // kT threads per block: kBlock, or 64 on a level whose kBlock grid leaves
@@ -488,11 +486,11 @@ __global__ void __launch_bounds__(kT) k_ghost(GhostItems G, int off, int n, T *_
   // (their own V-cycle starts below it)
   const int inst = (t < n && G.inst) ? G.inst[i] : -1;
   const bool skip = t >= n || (inst >= 0 && (!active[inst] || inst_nlev[inst] < need));
-  GhostPrep P;
-  if (!skip) P = ghost_prep(G, i, G.type[i], G.dst[i]);
+  GhostPre<T> X;
+  if (!skip) X = ghost_pre<T>(G, i, G.type[i], G.dst[i], bcg, T(hx_), T(hy_));
   chain_wait();
   if (skip) return;
-  ghost_apply_home<T, false>(G, P, i, Q, QC, bcg, T(hx_), T(hy_), M, false);
+  ghost_apply_home<T, false>(X, Q, QC, M, false);
 }
 
 // Ghost fills of several levels in one launch: span s holds the items
@@ -528,11 +526,11 @@ __global__ void __launch_bounds__(kT) k_ghost_spans(GhostItems G, GhostSpans S, 
   const int i = off + (t - b);
   const int inst = (in && G.inst) ? G.inst[i] : -1;
   const bool skip = !in || (inst >= 0 && !active[inst]);
-  GhostPrep P;
-  if (!skip) P = ghost_prep(G, i, G.type[i], G.dst[i]);
+  GhostPre<T> X;
+  if (!skip) X = ghost_pre<T>(G, i, G.type[i], G.dst[i], bcg, T(hx), T(hy));
   chain_wait();
   if (skip) return;
-  ghost_apply<T>(G, i, P, Q, QC, bcg, T(hx), T(hy));
+  ghost_apply<T>(X, Q, QC);
 }
 
 // ---------------------------------------------------------------------------
@@ -1129,7 +1127,7 @@ __global__ void __launch_bounds__(kClusterBlock, 1)
     const int i = g_off + t;
     const int inst = G.inst ? G.inst[i] : -1;
     if (inst >= 0 && !f.active[inst]) continue;
-    ghost_apply<T, true>(G, i, ghost_prep(G, i, G.type[i], G.dst[i]), f.Q, f.QC, f.bcg, T(hx_), T(hy_));
+    ghost_apply<T, true>(ghost_pre<T>(G, i, G.type[i], G.dst[i], f.bcg, T(hx_), T(hy_)), f.Q, f.QC);
   }
 }
 
@@ -1146,7 +1144,7 @@ __global__ void __launch_bounds__(kClusterBlock, 1)
 // and its ghost rule with the rule's parent-cell operands (cells outside the
 // range do not change during the relaxation), so a pass waits only for the
 // shared-memory loads of the solution.  The arithmetic of every update and
-// ghost is relax_cell's and ghost_item's, so the results are the chained
+// ghost is relax_cell's and ghost_apply's, so the results are the chained
 // passes' bit for bit.  The host uses it on levels with at most one colour
 // cell per thread and colour; the dynamic shared memory is the slice and
 // ten values per thread (the rules' parent-cell operands).
@@ -1322,11 +1320,10 @@ __device__ __forceinline__ void dsm_cell_update(const LevelD &L, const FieldsT<T
 template <class T>
 __device__ __forceinline__ T ghost_eval_dsm(const GhostItems &G, int i, const FieldsT<T> &f, T hx, T hy,
                                             const DsmRange<T> &D) {
-  const GhostPrep P = ghost_prep(G, i, G.type[i], 0);
+  const GhostPrep<T> P = ghost_prep<T>(G, i, G.type[i], 0, f.bcg, hx, hy);
   const T qa = dsm_sol(D, f.Q, P.a), qb = dsm_sol(D, f.Q, P.b), qc = dsm_sol(D, f.Q, P.c);
   const T qd = dsm_sol(D, f.Q, P.d), qe = dsm_sol(D, f.Q, P.e);
-  const T g = P.g >= 0 ? f.bcg[P.g] : T(0);
-  return ghost_formula<T>(P.ty, qa, qb, qc, qd, qe, g, P.nb, hx, hy);
+  return ghost_formula<T>(P.ty, qa, qb, qc, qd, qe, P.g);
 }
 
 template <class T, bool kPow2>
@@ -1473,96 +1470,102 @@ __global__ void __launch_bounds__(kT) k_restrict_fill(LevelD L, Decomp D, Fields
     const int inst = (t < f_n && G.inst) ? G.inst[i] : -1;
     const int8_t ty = t < f_n ? G.type[i] : G_COPY;
     const bool skip = t >= f_n || (inst >= 0 && !active[inst]) || (ty == G_RING && !f_ring);
-    GhostPrep P;
-    if (!skip) P = ghost_prep(G, i, ty, G.dst[i]);
+    GhostPre<T> X;
+    if (!skip) X = ghost_pre<T>(G, i, ty, G.dst[i], f.bcg, T(fhx), T(fhy));
     chain_wait();
     if (skip) return;
-    ghost_apply_home<T, true>(G, P, i, f.Q, f.QC, f.bcg, T(fhx), T(fhy), M, f_zero != 0);
+    ghost_apply_home<T, true>(X, f.Q, f.QC, M, f_zero != 0);
     return;
   }
   const int t = ((int)blockIdx.x - nb_r - nb_f) * kT + threadIdx.x;
   const int i = g_off + t;
   const int inst = (t < g_n && G.inst) ? G.inst[i] : -1;
   const bool skip = t >= g_n || (inst >= 0 && (!active[inst] || inst_nlev[inst] < need));
-  GhostPrep P;
-  if (!skip) P = ghost_prep<true>(G, i, G.type[i], G.dst[i], &A);
+  GhostPre<T> X;
+  if (!skip) X = ghost_pre<T, true>(G, i, G.type[i], G.dst[i], f.bcg, T(hx_), T(hy_), &A);
   chain_wait();
   if (skip) return;
-  ghost_apply<T, false, true>(G, i, P, f.Q, f.QC, f.bcg, T(hx_), T(hy_), &A);
+  ghost_apply<T, false, true>(X, f.Q, f.QC, &A);
 }
 // ---------------------------------------------------------------------------
-// ebFaceCorrections (ebFaceCorrections.m:18-61): correction of coarse face j
-// on face fc (0 W, 1 E, 2 S, 3 N) of patch P.  The coarse values are read
-// where the reference's QC holds them: the outer (ring) cell from the
-// parent's Q through the window table, the inner cell from QC's interior
-// (`qc_inner` false) or recomputed as the restriction of its four fine cells
-// (`qc_inner` true: the residual's refresh, ebCompResidual.m:32-38).
-// The arithmetic is FP64 for either value type (the reflux of the mixed
-// form stays FP64).
+// ebFaceCorrections (ebFaceCorrections.m:18-61): the correction of one coarse
+// face.  Its operands' indices are resolved at upload: the fine cells either
+// side of the two fine faces (a - b), the coarse values where the reference's
+// QC holds them -- the outer (ring) cell in the parent's Q, the inner cell in
+// QC's interior (`qc_inner` false) or recomputed as the restriction of its
+// four fine cells (`qc_inner` true: the residual's refresh,
+// ebCompResidual.m:32-38) -- and the three diffusivities.  The arithmetic is
+// FP64 for either value type (the reflux of the mixed form stays FP64).
+struct __align__(16) CorrRec {
+  int a1, b1, a2, b2;          // fine cells (Q)
+  int out, qc, in, ldq;        // parent's cell (Q), QC cell, first inner fine cell (Q) and its row stride
+  int c1, c2, cf, yface;       // DeW or DnS twice, interface D; 1: a y face
+};
+
+// a record and its diffusivities, held across a programmatic-launch wait
+struct CorrPre {
+  CorrRec r;
+  double d1, d2, cf;
+};
+template <class T>
+__device__ __forceinline__ CorrPre corr_pre(const CorrRec *__restrict__ rec, const FieldsT<T> &f) {
+  CorrPre X;
+  const int4 *p = reinterpret_cast<const int4 *>(rec);
+  const int4 u = __ldg(p), v = __ldg(p + 1), w = __ldg(p + 2);
+  X.r = CorrRec{u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w, w.x, w.y, w.z, w.w};
+  const T *D = X.r.yface ? f.DnS : f.DeW;
+  X.d1 = dbl(__ldg(D + X.r.c1));
+  X.d2 = dbl(__ldg(D + X.r.c2));
+  X.cf = dbl(__ldg(f.cfd + X.r.cf));
+  return X;
+}
 template <bool kPow2, class T>
-__device__ __forceinline__ double face_corr(const PatchD &P, const FieldsT<T> &f, int fc, int j,
-                                            const DivC &hc2, bool qc_inner) {
-  const int mx = P.mx, my = P.my, cmx = mx >> 1, cmy = my >> 1;
-  const int ldq = mx + 2, ldc = cmx + 2;
-  const T *Q = f.Q + P.q_off + f.lsh, *QC = f.QC + P.qc_off;
-  const int *win = f.win + P.win_off;
-  const T *DeW = f.DeW + P.dew_off, *DnS = f.DnS + P.dns_off, *cfd = f.cfd + P.cfd_off;
-  auto q = [&](int i) { return dbl(Q[i]); };
-  double v;
-  switch (fc) {
-    case 0: {
-      const int r1 = 2 * j + 1, r2 = 2 * j + 2;
-      const double out = dbl(f.Q[win[(j + 1) * ldc]]);
-      const double in = dbl(qc_inner ? restrict_cell<T>(Q, ldq, 0, j) : QC[1 + (j + 1) * ldc]);
-      v = (dbl(DeW[(2 * j) * (mx + 1)]) * (q(1 + r1 * ldq) - q(r1 * ldq)) +
-           dbl(DeW[(2 * j + 1) * (mx + 1)]) * (q(1 + r2 * ldq) - q(r2 * ldq))) +
-          dbl(cfd[j]) * (out - in);
-      break;
-    }
-    case 1: {
-      const int r1 = 2 * j + 1, r2 = 2 * j + 2;
-      const double out = dbl(f.Q[win[cmx + 1 + (j + 1) * ldc]]);
-      const double in = dbl(qc_inner ? restrict_cell<T>(Q, ldq, cmx - 1, j) : QC[cmx + (j + 1) * ldc]);
-      v = (dbl(DeW[mx + (2 * j) * (mx + 1)]) * (q(mx + r1 * ldq) - q(mx + 1 + r1 * ldq)) +
-           dbl(DeW[mx + (2 * j + 1) * (mx + 1)]) * (q(mx + r2 * ldq) - q(mx + 1 + r2 * ldq))) +
-          dbl(cfd[cmy + j]) * (out - in);
-      break;
-    }
-    case 2: {
-      const int c1 = 2 * j + 1, c2 = 2 * j + 2;
-      const double out = dbl(f.Q[win[j + 1]]);
-      const double in = dbl(qc_inner ? restrict_cell<T>(Q, ldq, j, 0) : QC[j + 1 + ldc]);
-      v = (dbl(DnS[2 * j]) * (q(c1 + ldq) - q(c1)) + dbl(DnS[2 * j + 1]) * (q(c2 + ldq) - q(c2))) +
-          dbl(cfd[2 * cmy + j]) * (out - in);
-      break;
-    }
-    default: {
-      const int c1 = 2 * j + 1, c2 = 2 * j + 2;
-      const double out = dbl(f.Q[win[j + 1 + (cmy + 1) * ldc]]);
-      const double in = dbl(qc_inner ? restrict_cell<T>(Q, ldq, j, cmy - 1) : QC[j + 1 + cmy * ldc]);
-      v = (dbl(DnS[2 * j + my * mx]) * (q(c1 + my * ldq) - q(c1 + (my + 1) * ldq)) +
-           dbl(DnS[2 * j + 1 + my * mx]) * (q(c2 + my * ldq) - q(c2 + (my + 1) * ldq))) +
-          dbl(cfd[2 * cmy + cmx + j]) * (out - in);
-      break;
-    }
+__device__ __forceinline__ double corr_value(const CorrPre &X, const FieldsT<T> &f, const LevelD &Lc, bool qc_inner) {
+  const CorrRec &r = X.r;
+  const T *Q = f.Q + f.lsh;
+  const double out = dbl(f.Q[r.out]);
+  double in;
+  if (qc_inner) {
+    const T *q = Q + r.in;
+    in = dbl(T(0.25) * (((q[0] + q[1]) + q[r.ldq]) + q[r.ldq + 1]));
+  } else {
+    in = dbl(f.QC[r.qc]);
   }
-  return div_c<kPow2>(v, hc2);
+  const double v = (X.d1 * (dbl(Q[r.a1]) - dbl(Q[r.b1])) + X.d2 * (dbl(Q[r.a2]) - dbl(Q[r.b2]))) + X.cf * (out - in);
+  return div_c<kPow2>(v, r.yface ? Lc.dy : Lc.dx);
 }
 
 // gather-form corrections of one target coarse cell: contributions in the
 // reference's order (fine patch ascending, faces W, E, S, N)
 struct CorrCSR {
-  const int *cell, *patch, *beg, *item, *jj;   // item = (level-local fine patch << 2) | face
+  const int *cell, *patch, *beg;
+  const CorrRec *rec;
 };
 
+// a target's contributions, the first two (nearly all targets have no more)
+// read before the programmatic-launch wait: with item, patch and index
+// arithmetic after it the coarse loads of a 4-level hierarchy of 64^2 patches
+// took 4.5-5 us each, now 3.4-4
+struct CorrTarget {
+  int beg, end;
+  CorrPre x0, x1;
+};
+template <class T>
+__device__ __forceinline__ CorrTarget corr_target(const CorrCSR &C, int t, const FieldsT<T> &f) {
+  CorrTarget X;
+  X.beg = __ldg(C.beg + t);
+  X.end = __ldg(C.beg + t + 1);
+  if (X.beg < X.end) X.x0 = corr_pre<T>(C.rec + X.beg, f);
+  if (X.beg + 1 < X.end) X.x1 = corr_pre<T>(C.rec + X.beg + 1, f);
+  return X;
+}
 template <bool kPow2, class T>
-__device__ __forceinline__ double add_corrections(double v, const CorrCSR &C, int t, const LevelD &Lf, const LevelD &Lc,
+__device__ __forceinline__ double add_corrections(double v, const CorrTarget &X, const CorrCSR &C, const LevelD &Lc,
                                                   const FieldsT<T> &f, bool qc_inner) {
-  for (int i = C.beg[t]; i < C.beg[t + 1]; ++i) {
-    const int it = C.item[i];
-    const int fc = it & 3;
-    v = v + face_corr<kPow2>(Lf.patches[it >> 2], f, fc, C.jj[i], fc < 2 ? Lc.dx : Lc.dy, qc_inner);
-  }
+  if (X.beg >= X.end) return v;
+  v = v + corr_value<kPow2>(X.x0, f, Lc, qc_inner);
+  if (X.beg + 1 < X.end) v = v + corr_value<kPow2>(X.x1, f, Lc, qc_inner);
+  for (int i = X.beg + 2; i < X.end; ++i) v = v + corr_value<kPow2>(corr_pre<T>(C.rec + i, f), f, Lc, qc_inner);
   return v;
 }
 
@@ -1689,14 +1692,20 @@ __device__ __forceinline__ void load_corr_item(const LevelD &L, const LevelD &Lc
                                                int n_tgt, int t) {
   const bool on = t < n_tgt && f.active[Lc.patches[C.patch[t]].inst];
   const int cell = on ? C.cell[t] : 0;
+  CorrTarget X;
+  double base = 0.0;
+  if (on) {
+    X = corr_target<T>(C, t, f);
+    if (sizeof(T) == sizeof(double)) base = f.FTrue[cell];
+  }
   if (kChain) chain_wait();
   if (!on) return;
   // FP64: the target's F before its corrections is FTrue (the value the
   // reference's per-cycle reset F = FTrue leaves there), so the V-cycle does
   // not depend on a reset of F before it; the correction cycle of the mixed
   // form adds to its own right-hand side
-  const double base = sizeof(T) == sizeof(double) ? f.FTrue[cell] : dbl(f.F[cell]);
-  f.F[cell] = T(add_corrections<kPow2, T>(base, C, t, L, Lc, f, false));
+  if (sizeof(T) != sizeof(double)) base = dbl(f.F[cell]);
+  f.F[cell] = T(add_corrections<kPow2, T>(base, X, C, Lc, f, false));
 }
 
 // kT threads per block (kBlock, or 64 on a level whose kBlock grid leaves
@@ -1832,11 +1841,11 @@ __global__ void __launch_bounds__(kT) k_fill_prolong(GhostItems G, int g_off, in
     const int i = g_off + t;
     const int inst = (t < g_n && G.inst) ? G.inst[i] : -1;
     const bool skip = t >= g_n || (inst >= 0 && !active[inst]);
-    GhostPrep P;
-    if (!skip) P = ghost_prep(G, i, G.type[i], G.dst[i]);
+    GhostPre<T> X;
+    if (!skip) X = ghost_pre<T>(G, i, G.type[i], G.dst[i], f.bcg, W.hx, W.hy);
     chain_wait();
     if (skip) return;
-    ghost_apply<T>(G, i, P, f.Q, f.QC, f.bcg, W.hx, W.hy);
+    ghost_apply<T>(X, f.Q, f.QC);
     return;
   }
   prolong_item<T, true>(L, D, f, correct, ((int)blockIdx.x - nb_g) * kT + threadIdx.x, &W);
@@ -2033,21 +2042,38 @@ __global__ void __launch_bounds__(kT) k_residual(const LevelX *__restrict__ X, c
       fs = fnN;
     }
   } else {   // targets of this level, corrections from the level above
+    const LevelX &Xf = X[T.level + 1];
+    const bool on = mass_corr && lane < T.n;
+    CorrTarget Y;
+    int cell = 0, c = 0, ldq = 0;
+    double dE = 0, dW = 0, dN = 0, dS = 0, cf = 0, ft = 0;
+    bool vis = false;
+    if (on) {
+      const int g = T.b + lane;
+      cell = __ldg(Xf.C.cell + g);
+      const PatchD &Pc = Xk.L.patches[__ldg(Xf.C.patch + g)];
+      const int s = cell - Pc.c_off, mx = Pc.mx;
+      const int lj = s / mx, lx = s - lj * mx;
+      ldq = mx + 2;
+      c = Pc.q_off + (lx + 1) + (lj + 1) * ldq;
+      const double *DeW = f.DeW + Pc.dew_off + lx + lj * (mx + 1), *DnS = f.DnS + Pc.dns_off + lx + lj * mx;
+      dE = __ldg(DeW + 1);
+      dW = __ldg(DeW);
+      dN = __ldg(DnS + mx);
+      dS = __ldg(DnS);
+      cf = __ldg(f.CC + cell);
+      ft = __ldg(f.FTrue + cell);
+      vis = !(__ldg(f.flags + cell) & 1);
+      Y = corr_target<double>(Xf.C, g, f);
+    }
     chain_wait();
     if (!mass_corr) return;
-    const LevelX &Xf = X[T.level + 1];
-    if (lane < T.n) {
-      const int g = T.b + lane;
-      const int cell = Xf.C.cell[g];
-      const PatchD &Pc = Xk.L.patches[Xf.C.patch[g]];
-      const int s = cell - Pc.c_off;
-      const int lj = s / Pc.mx, lx = s - lj * Pc.mx;
-      const double ft = f.FTrue[cell];
-      double r = ft - op_cell_r<kPow2>(f.Q + Pc.q_off, Pc.mx + 2, f.DeW + Pc.dew_off, f.DnS + Pc.dns_off, f.CC[cell], Pc.mx,
-                                lx, lj, Xk.L);
-      r = add_corrections<kPow2>(r, Xf.C, g, Xf.L, Xk.L, f, true);
+    if (on) {
+      const double *Q = f.Q + c;
+      double r = ft - op_pre<kPow2>(Q[0], Q[1], Q[-1], Q[ldq], Q[-ldq], dE, dW, dN, dS, cf, Xk.L);
+      r = add_corrections<kPow2>(r, Y, Xf.C, Xk.L, f, true);
       if (rout) rout[cell] = (float)r;
-      if (!(f.flags[cell] & 1)) take(r, ft);
+      if (vis) take(r, ft);
     }
   }
   if (!kL2 && !norms) return;
@@ -2393,7 +2419,7 @@ __global__ void __launch_bounds__(kBlock) k_uoo_transfer(LevelD L, Decomp D, con
 __global__ void __launch_bounds__(kBlock) k_prhs(Decomp D, const PatchD *__restrict__ patches, double *FTrue,
                                                  const double *__restrict__ fsrc, const double *__restrict__ Uo,
                                                  const double *__restrict__ Uoo, double dt, int bdf2) {
-  chain_wait();
+  chain_wait_static();
   const int g = blockIdx.x * kBlock + threadIdx.x;
   if (g >= D.n) return;
   const int p = find_patch(D, blockIdx.x, g);
@@ -2502,7 +2528,7 @@ __global__ void __launch_bounds__(kBlock) k_tag_buffer(const uint8_t *__restrict
 
 // FP32 copy of an FP64 array (coefficient copies of the mixed form)
 __global__ void __launch_bounds__(kBlock) k_to_f32(const double *__restrict__ a, float *__restrict__ b, long long n) {
-  chain_wait();
+  chain_wait_static();
   for (long long i = blockIdx.x * (long long)kBlock + threadIdx.x; i < n; i += (long long)gridDim.x * kBlock)
     b[i] = (float)a[i];
 }
