@@ -1066,7 +1066,10 @@ void launch_coarse_load(bsam_hier h, int k, int home = 0) {
   const int ntgt = h->opts.mass_correction ? L.ct_n : 0;
   Launch l(h, K_LOAD, 50.0 * tscale<T>() * (double)L.ncells, k);
   const int *ri = (const int *)(h->ninst > 1 ? h->ring_inst.p : nullptr);
-  const bool spread = D.nblocks < spread_limit(h);   // the footprint's FP64 work over more SMs
+  // the footprint's FP64 work over more SMs, in a batch too: with few
+  // instances left a 256-thread block of 40 operations a thread is 3 us of its
+  // SM's FP64 pipe (14 of 64 instances, 473 blocks: 9.9 us, 1,887: 4.5)
+  const bool spread = D.nblocks < 8 * sm_count();
   const int kt = spread ? 64 : kBlock;
   auto nb = [&](int n) { return (n + kt - 1) / kt; };
   auto go = [&](auto kern) {
@@ -1093,10 +1096,17 @@ void launch_prolong(bsam_hier h, int k, int correct, int home = 0) {
   const LevelPlan &L = h->lev[k];
   Decomp D = decomp(h, L.coarse);
   Launch l(h, K_PROLONG, 20.0 * tscale<T>() * (double)L.ncells, k);
-  if (D.nblocks < spread_limit(h))
-    launch_k(h, k_prolong<T, 64>, (D.n + 63) / 64, 64, leveld(h, k), D, fields_at<T>(h, home), correct);
-  else
-    launch_k(h, k_prolong<T>, D.nblocks, kBlock, leveld(h, k), D, fields_at<T>(h, home), correct);
+  auto go = [&](auto kern, int kt) {
+    launch_k(h, kern, (D.n + kt - 1) / kt, kt, leveld(h, k), D, fields_at<T>(h, home), correct);
+  };
+  const bool small = D.nblocks < spread_limit(h);
+  if (sizeof(T) == sizeof(double) && L.ncells >= kIntMinCells) {
+    if (small) go(k_prolong<T, true, 64>, 64);
+    else go(k_prolong<T, true>, kBlock);
+  } else {
+    if (small) go(k_prolong<T, false, 64>, 64);
+    else go(k_prolong<T, false>, kBlock);
+  }
 }
 
 // the closing fill of level k-1 and the prolongation-correction of level k
@@ -1143,9 +1153,10 @@ void launch_coarsest(bsam_hier h, bool defer_fill = false) {
   {
     Launch l(h, K_COARSEST, 8.0 * (double)h->Ainv.n, 1);
     cudaLaunchConfig_t cfg = {};
-    const int rows = h->ninst > 1 ? 8 : 1;
+    const bool batch = h->ninst > 1;
+    const int rows = batch ? kBRows : 1;
     cfg.gridDim = dim3((unsigned)((h->coarse_max_rows + rows - 1) / rows), (unsigned)h->ncoarse_patches);
-    cfg.blockDim = dim3(32 * rows);
+    cfg.blockDim = dim3(batch ? 32 * kBWarps : 32);
     cfg.stream = h->stream;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1153,11 +1164,11 @@ void launch_coarsest(bsam_hier h, bool defer_fill = false) {
     cfg.attrs = at;
     cfg.numAttrs = 1;
     const double *rhs = sizeof(T) == sizeof(double) ? (const double *)h->bcRhs.p : nullptr;
-    if (rows == 1)
-      cudaLaunchKernelEx(&cfg, k_coarsest<T, 1>, (const double *)h->Ainv.p, rhs, (const CoarsestD *)h->coarsest.p,
-                         fields_t<T>(h));
+    if (batch)
+      cudaLaunchKernelEx(&cfg, k_coarsest_batch<T>, (const double *)h->Ainv.p, rhs,
+                         (const CoarsestD *)h->coarsest.p, fields_t<T>(h));
     else
-      cudaLaunchKernelEx(&cfg, k_coarsest<T, 8>, (const double *)h->Ainv.p, rhs, (const CoarsestD *)h->coarsest.p,
+      cudaLaunchKernelEx(&cfg, k_coarsest<T>, (const double *)h->Ainv.p, rhs, (const CoarsestD *)h->coarsest.p,
                          fields_t<T>(h));
   }
   if (!defer_fill) launch_fill<T>(h, 1);

@@ -95,6 +95,42 @@ __device__ __forceinline__ float mul_on(float a, float b) {
   return a * b;
 }
 
+// 3 x and 9 x on the integer pipe, correctly rounded: the significand times K
+// has one or two bits (K = 9: three or four) too many, which are rounded to
+// nearest even; zeros, denormals, infinities, NaN and results beyond the
+// range take the multiply instruction
+template <int K>
+__device__ __forceinline__ double times_int_pipe(double x) {
+  static_assert(K == 3 || K == 9, "");
+  constexpr int kLog = K == 3 ? 1 : 3;
+  const unsigned h = (unsigned)__double2hiint(x), l = (unsigned)__double2loint(x);
+  const uint64_t m = ((uint64_t)((h & 0xfffffu) | 0x100000u) << 32) | l;
+  const uint64_t w = m + (m << kLog);
+  const unsigned n = kLog + ((unsigned)(w >> (53 + kLog)) & 1u);       // bits to drop
+  const uint64_t r = (w + ((1u << (n - 1)) - 1u) + ((unsigned)(w >> n) & 1u)) >> n;
+  const unsigned e = h & 0x7ff00000u;
+  // the significand's leading bit adds the one that the exponent field lacks
+  const double q = __hiloint2double((int)((unsigned)(r >> 32) + ((h & 0xfff00000u) + ((n - 1) << 20))), (int)(unsigned)r);
+  const bool in = e - 0x00100000u < 0x7f800000u;                       // 1 <= exponent field <= 2040
+  return in ? q : mul_fp64_pipe(x, (double)K);
+}
+// x / 16: the exponent field less four
+__device__ __forceinline__ double sixteenth_int_pipe(double x) {
+  const unsigned h = (unsigned)__double2hiint(x);
+  const bool in = (h & 0x7ff00000u) - 0x00500000u < 0x7fa00000u;       // 5 <= exponent field <= 2046
+  return in ? __hiloint2double((int)(h - 0x00400000u), __double2loint(x)) : mul_fp64_pipe(x, 0.0625);
+}
+template <int K, bool kInt, class T>
+__device__ __forceinline__ T times(T x) {
+  if constexpr (kInt && sizeof(T) == 8) return times_int_pipe<K>(x);
+  else return T(K) * x;
+}
+template <bool kInt, class T>
+__device__ __forceinline__ T sixteenth(T x) {
+  if constexpr (kInt && sizeof(T) == 8) return sixteenth_int_pipe(x);
+  else return x / 16;
+}
+
 // per-patch metadata on the device
 struct PatchD {
   int mx, my, par0, level;
@@ -1736,8 +1772,13 @@ __global__ void __launch_bounds__(kT) k_load(LevelD L, LevelD Lc, Decomp D, Fiel
 // (ebTransfer.m:57-71) adds P(W - QC) to the interior; mode 0 writes P(W)
 // (new-level initial guess, ebAddLevel.m:26-31).  One thread per coarse cell
 // writes its four fine cells.
-// kT threads per block: kBlock, or 64 on a level whose kBlock grid leaves
-// SMs idle (about 37 FP64 operations per coarse cell, two per clock per SM)
+//
+// The FP64 form is bound by the FP64 pipe: 32 operations a coarse cell.
+// Levels large enough to keep the pipe busy (kInt) form the five products and
+// the four sixteenths on the integer pipe: 1,048,576 fine cells 18.2 us ->
+// 15.3, 379,536 in patches 8.5 -> 7.5.  (Threads of two or four coarse cells
+// that share their differences took 13.2 us on the former, but 4.7 to 8
+// instead of 3.3 on small levels.)
 // A parent-window operand of the prolongation fused with the parent level's
 // closing fill (k_fill_prolong): a code >= 0 is a cell of Q; a code < 0 is
 // the ghost cell that ghost item -1 - code fills in the same launch, whose
@@ -1766,7 +1807,7 @@ __device__ __forceinline__ T window_value(const T *Q, int code, const WindowGhos
   return eval_rule<T>(G, i, Q, W->bcg, W->hx, W->hy);
 }
 
-template <class T, bool kChain>
+template <class T, bool kChain, bool kInt>
 __device__ __forceinline__ void prolong_item(const LevelD &L, const Decomp &D, const FieldsT<T> &f, int correct,
                                              int g, const WindowGhosts<T> *W = nullptr) {
   if (g >= D.n) {
@@ -1801,11 +1842,13 @@ __device__ __forceinline__ void prolong_item(const LevelD &L, const Decomp &D, c
       const T wv = window_value<T>(f.Q, src[dj][di], W);
       E[dj][di] = correct ? wv - QC[w] : wv;
     }
-  const T C = E[1][1], Wm = E[1][0], Wp = E[1][2], Sm = E[0][1], Sp = E[2][1];
-  const T f11 = (((9 * C + 3 * Wm) + 3 * Sm) + E[0][0]) / 16;
-  const T f21 = (((9 * C + 3 * Wp) + 3 * Sm) + E[0][2]) / 16;
-  const T f12 = (((9 * C + 3 * Wm) + 3 * Sp) + E[2][0]) / 16;
-  const T f22 = (((9 * C + 3 * Wp) + 3 * Sp) + E[2][2]) / 16;
+  const T c9 = times<9, kInt>(E[1][1]);
+  const T w = c9 + times<3, kInt>(E[1][0]), e = c9 + times<3, kInt>(E[1][2]);
+  const T s3 = times<3, kInt>(E[0][1]), n3 = times<3, kInt>(E[2][1]);
+  const T f11 = sixteenth<kInt>((w + s3) + E[0][0]);
+  const T f21 = sixteenth<kInt>((e + s3) + E[0][2]);
+  const T f12 = sixteenth<kInt>((w + n3) + E[2][0]);
+  const T f22 = sixteenth<kInt>((e + n3) + E[2][2]);
   T *Q = f.Q + q_off + f.lsh;
   const int c = (2 * a + 1) + (2 * b + 1) * ldq;
   if (correct) {
@@ -1821,9 +1864,11 @@ __device__ __forceinline__ void prolong_item(const LevelD &L, const Decomp &D, c
   }
 }
 
-template <class T, int kT = kBlock>
+// kT threads per block: kBlock, or 64 on a level whose kBlock grid leaves
+// SMs idle
+template <class T, bool kInt, int kT = kBlock>
 __global__ void __launch_bounds__(kT) k_prolong(LevelD L, Decomp D, FieldsT<T> f, int correct) {
-  prolong_item<T, true>(L, D, f, correct, blockIdx.x * kT + threadIdx.x);
+  prolong_item<T, true, kInt>(L, D, f, correct, blockIdx.x * kT + threadIdx.x);
 }
 
 // The closing ghost fill of level k-1 (the end of its V-cycle) and the
@@ -1848,7 +1893,7 @@ __global__ void __launch_bounds__(kT) k_fill_prolong(GhostItems G, int g_off, in
     ghost_apply<T>(X, f.Q, f.QC);
     return;
   }
-  prolong_item<T, true>(L, D, f, correct, ((int)blockIdx.x - nb_g) * kT + threadIdx.x, &W);
+  prolong_item<T, true, false>(L, D, f, correct, ((int)blockIdx.x - nb_g) * kT + threadIdx.x, &W);
 }
 
 // ---------------------------------------------------------------------------
@@ -1861,17 +1906,16 @@ struct CoarsestD {
 
 // bcRhs null: a homogeneous problem (the correction cycle of the mixed
 // form), whose F is FP32 while the solve itself stays FP64.
-// one warp per row, kRows rows per block: one row per block spreads a single
-// hierarchy's rows' FP64 work over as many SMs as there are rows; a batch
-// keeps eight, since most of its instances' blocks exit at once in its last
-// V-cycles
-// one row of the coarsest solve, computed by one warp (lane = lane index)
-template <class T, bool kChain>
-__device__ __forceinline__ void coarsest_row(const double *__restrict__ Ainv, const double *__restrict__ bcRhs,
-                                             const CoarsestD &D, const FieldsT<T> &f, int row, int lane) {
-  const int N = D.N;
+//
+// One hierarchy: one row per block, which spreads the rows' FP64 work over
+// as many SMs as there are rows.
+template <class T>
+__global__ void __launch_bounds__(32) k_coarsest(const double *__restrict__ Ainv, const double *__restrict__ bcRhs,
+                                                 const CoarsestD *__restrict__ cd, FieldsT<T> f) {
+  const CoarsestD D = cd[0];
+  const int row = blockIdx.x, lane = threadIdx.x, N = D.N;
   if (row >= N || !f.active[D.inst]) {
-    if (kChain) chain_wait();
+    chain_wait();
     return;
   }
   const double *a = Ainv + D.ainv_off + (size_t)row * N;
@@ -1884,7 +1928,7 @@ __device__ __forceinline__ void coarsest_row(const double *__restrict__ Ainv, co
     av[i] = c < N ? __ldg(a + c) : 0.0;
     bv[i] = (c < N && rhs) ? __ldg(rhs + c) : 0.0;
   }
-  if (kChain) chain_wait();
+  chain_wait();
   const T *F = f.F + D.c_off;
   double s = 0.0;
 #pragma unroll
@@ -1904,12 +1948,74 @@ __device__ __forceinline__ void coarsest_row(const double *__restrict__ Ainv, co
   }
 }
 
-template <class T, int kRows = 1>
-__global__ void __launch_bounds__(32 * kRows) k_coarsest(const double *__restrict__ Ainv,
-                                                         const double *__restrict__ bcRhs,
-                                                         const CoarsestD *__restrict__ cd, FieldsT<T> f) {
+// A batch (blockIdx.y: instance): bound by the FP64 pipe, where a warp per
+// row costs 29 operations (8 of F + bcRhs, 8 products, 8 sums, 5 of the
+// tree).  A block of kBRows rows forms F + bcRhs once in shared memory, the
+// products go to the integer pipe (the same bits, mul_int_pipe), and a warp
+// holds four rows, whose trees share the halves that a tree leaves idle: 10
+// operations a row, each sum in the order above.  64 instances of 256 rows
+// 32 us -> 17.
+constexpr int kBWarps = 4, kBRows = 4 * kBWarps, kBCols = 256;
+template <class T>
+__global__ void __launch_bounds__(32 * kBWarps, 7) k_coarsest_batch(const double *__restrict__ Ainv,
+                                                                 const double *__restrict__ bcRhs,
+                                                                 const CoarsestD *__restrict__ cd, FieldsT<T> f) {
+  __shared__ double v[kBCols];
   const CoarsestD D = cd[blockIdx.y];
-  coarsest_row<T, true>(Ainv, bcRhs, D, f, blockIdx.x * kRows + (int)(threadIdx.x >> 5), threadIdx.x & 31);
+  const int lane = threadIdx.x & 31, N = D.N;
+  const int b0 = blockIdx.x * kBRows, row0 = b0 + (int)(threadIdx.x >> 5) * 4;
+  if (b0 >= N || !f.active[D.inst]) {
+    chain_wait();
+    return;
+  }
+  const double *rhs = bcRhs ? bcRhs + D.rhs_off : nullptr;
+  const double *a = Ainv + D.ainv_off;
+  // a ring of four columns per lane and row (more would leave the grid two
+  // waves of blocks)
+  constexpr int kRing = 4;
+  double av[4][kRing];
+  auto load = [&](int slot, int c) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) av[q][slot] = c < N ? __ldg(a + (size_t)min(row0 + q, N - 1) * N + c) : 0.0;
+  };
+#pragma unroll
+  for (int i = 0; i < kRing; ++i) load(i, lane + 32 * i);
+  chain_wait();
+  const T *F = f.F + D.c_off;
+  double s[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int c0 = 0; c0 < N; c0 += kBCols) {
+    if (c0) __syncthreads();                 // the last columns' readers
+    for (int c = threadIdx.x; c < kBCols && c0 + c < N; c += 32 * kBWarps)
+      v[c] = dbl(F[c0 + c]) + (rhs ? __ldg(rhs + c0 + c) : 0.0);
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kBCols / 32; ++i) {
+      const int c = lane + 32 * i;
+      if (c0 + c < N) {
+        const double x = v[c];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) s[q] = s[q] + mul_int_pipe(av[q][i % kRing], x);
+        load(i % kRing, c0 + c + 32 * kRing);
+      }
+    }
+  }
+  // halving trees: lanes l < off add lane l + off; the second of a pair of
+  // trees runs in the lanes that the first has given up
+  auto pair = [&](double x, double y, int off) -> double {
+    const bool up = lane & off;
+    const double mine = up ? y : x, sent = up ? x : y;
+    return mine + __shfl_xor_sync(0xffffffffu, sent, off);
+  };
+  const double t0 = pair(s[0], s[1], 16), t1 = pair(s[2], s[3], 16);
+  double t = pair(t0, t1, 8);
+#pragma unroll
+  for (int off = 4; off >= 1; off >>= 1) t = t + __shfl_xor_sync(0xffffffffu, t, off);
+  // rows 0, 1 of the pair in lanes 0, 16; rows 2, 3 in lanes 8, 24
+  const int q = (lane >> 4) + ((lane >> 3) & 1) * 2, row = row0 + q;
+  if ((lane & 7) == 0 && row < N) {
+    const int i = row % D.n1, j = row / D.n1;
+    f.Q[D.q_off + (i + 1) + (j + 1) * (D.n1 + 2)] = T(t);
+  }
 }
 
 // ---------------------------------------------------------------------------
