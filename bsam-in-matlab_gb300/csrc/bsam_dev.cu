@@ -208,9 +208,6 @@ struct bsam_hier_s {
   // footprint coded -1 - (entry of ga_rt)
   DBuf<int> ga_a, ga_b, ga_c;
   DBuf<int2> ga_rt;
-  // window tables for the prolongation fused with the parent's closing fill
-  // (k_fill_prolong): a parent ghost cell coded -1 - (its ghost item)
-  DBuf<int> win_alt;
   DBuf<PatchD> patches;
   DBuf<ResAcc> acc;
   DBuf<Rule> perim;                // per-patch perimeter ghost rules (inline)
@@ -282,20 +279,23 @@ Fields fields(bsam_hier h) {
 // how to divide by the constant d (DivC).  elo and espan: x, its quotient
 // and the remainder of the correction step (53 binary digits below x) all
 // stay normal, with a margin of two.
-DivC div_const(double d) {
-  DivC c;
+template <class T>
+DivK<T> div_const(T d) {
+  constexpr int kDig = sizeof(T) == 8 ? 53 : 24, kTop = sizeof(T) == 8 ? 2044 : 252;
+  DivK<T> c;
   c.d = d;
-  c.r = 1.0 / d;
+  c.r = T(1) / d;
   int e;
-  const double m = std::frexp(d, &e);
-  const double rel = std::fabs(std::fma(c.r, d, -1.0));   // exact: |r d - 1| is below an ulp
+  const T m = std::frexp(d, &e);
+  const T rel = std::fabs(std::fma(c.r, d, T(-1)));   // exact: |r d - 1| is below an ulp
   c.kexp = (1 - e) * (1 << 20);
-  c.ops = m == 0.5 ? 1 : rel < std::ldexp(1.0, -54) ? 3 : 5;
+  c.ops = m == T(0.5) ? 1 : rel < std::ldexp(T(1), -kDig - 1) ? 3 : 5;
   // biased exponents; the quotient's is x's minus (e - 1), give or take one
-  const int lo = std::max(57, 3 + (e - 1)), hi = std::min(2044, 2044 + (e - 1));
+  const int lo = std::max(kDig + 4, 3 + (e - 1)), hi = std::min(kTop, kTop + (e - 1));
   c.elo = (unsigned)lo;
   c.espan = (unsigned)std::max(hi - lo, 0);
-  if (e - 1 > 1000 || e - 1 < -1000) c.elo = 2048, c.espan = 0;   // always divide
+  // far out (or a constant that FP32 cannot hold): always divide
+  if (!std::isnormal(d) || e - 1 > kTop / 2 - 22 || e - 1 < 22 - kTop / 2) c.elo = 2048, c.espan = 0;
   return c;
 }
 
@@ -307,7 +307,7 @@ LevelD leveld(bsam_hier h, int k) {
   d.pow2 = L.pow2 ? 1 : 0;
   d.dx = div_const(L.hx * L.hx); d.dy = div_const(L.hy * L.hy);
   d.fhx = (float)d.hx; d.fhy = (float)d.hy;
-  d.fhx2 = (float)(L.hx * L.hx); d.fhy2 = (float)(L.hy * L.hy);
+  d.fdx = div_const((float)(L.hx * L.hx)); d.fdy = div_const((float)(L.hy * L.hy));
   return d;
 }
 
@@ -1109,47 +1109,9 @@ void launch_prolong(bsam_hier h, int k, int correct, int home = 0) {
   }
 }
 
-// the closing fill of level k-1 and the prolongation-correction of level k
-// (launch_fill(k - 1) + launch_prolong(k, 1)) in one launch
-template <class T = double>
-void launch_fill_prolong(bsam_hier h, int k, int home = 0) {
-  const LevelPlan &L = h->lev[k], &Lc = h->lev[k - 1];
-  if (!Lc.g1_n) {
-    launch_prolong<T>(h, k, 1, home);
-    return;
-  }
-  Decomp D = decomp(h, L.coarse);
-  FieldsT<T> f = fields_at<T>(h, home);
-  Launch l(h, K_PROLONG, 20.0 * tscale<T>() * (double)L.ncells, k);
-  const WindowGhosts<T> W{h->win_alt.p, ghost_items(h), f.bcg, (T)Lc.hx, (T)Lc.hy};
-  if (nblk(Lc.g1_n) + D.nblocks < spread_limit(h)) {
-    const int nb = (Lc.g1_n + 63) / 64;
-    launch_k(h, k_fill_prolong<T, 64>, nb + (D.n + 63) / 64, 64, ghost_items(h), Lc.g1_off, Lc.g1_n, nb,
-             leveld(h, k), D, f, 1, W, (const int *)h->active.p, (const int *)h->inst_nlev.p);
-  } else {
-    const int nb = nblk(Lc.g1_n);
-    launch_k(h, k_fill_prolong<T>, nb + D.nblocks, kBlock, ghost_items(h), Lc.g1_off, Lc.g1_n, nb, leveld(h, k), D,
-             f, 1, W, (const int *)h->active.p, (const int *)h->inst_nlev.p);
-  }
-}
-
-// can level k's V-cycle leave its closing fill to the prolongation of level
-// k + 1 (launch_fill_prolong): in the FP32 correction cycle, unless the
-// post-smoothing runs as one cluster launch, which fills the level itself.
-// The FP64 cycle keeps separate launches: there the fused launch's
-// prolongation items wait for the parent ghosts' rules on top of their FP64
-// work, and the starfish iteration measured no faster fused (the FP32 cycle
-// 1% faster); both forms give the same bits.
-template <class T>
-bool fill_deferrable(bsam_hier h, int k) {
-  if (sizeof(T) == sizeof(double)) return false;
-  if (k == 1 || h->opts.npost <= 0) return true;
-  return relax_form<T>(h, k) != 0;
-}
-
 // the FP32 correction cycle solves a homogeneous problem: no boundary rhs
 template <class T = double>
-void launch_coarsest(bsam_hier h, bool defer_fill = false) {
+void launch_coarsest(bsam_hier h) {
   {
     Launch l(h, K_COARSEST, 8.0 * (double)h->Ainv.n, 1);
     cudaLaunchConfig_t cfg = {};
@@ -1171,15 +1133,15 @@ void launch_coarsest(bsam_hier h, bool defer_fill = false) {
       cudaLaunchKernelEx(&cfg, k_coarsest<T>, (const double *)h->Ainv.p, rhs, (const CoarsestD *)h->coarsest.p,
                          fields_t<T>(h));
   }
-  if (!defer_fill) launch_fill<T>(h, 1);
+  launch_fill<T>(h, 1);
 }
 
 // ebVcycle (ebVcycle.m:16-35) from level k down.  defer_fill: the caller
-// fuses this level's closing fill with its own prolongation
+// fuses this level's closing fill with its fill-down
 template <class T = double>
 void launch_vcycle(bsam_hier h, int k, bool defer_fill = false) {
   if (k == 1) {
-    launch_coarsest<T>(h, defer_fill);
+    launch_coarsest<T>(h);
     return;
   }
   // the pre-smoothing's closing fill joins the restriction's launch where
@@ -1192,10 +1154,8 @@ void launch_vcycle(bsam_hier h, int k, bool defer_fill = false) {
   const int home = level_home<T>(h, k);
   launch_restrict_fill<T>(h, k, !pre_fused ? FILL_NONE : zero ? FILL_ZERO : FILL_PRE, -1, home);
   launch_coarse_load<T>(h, k, home);
-  const bool fused = fill_deferrable<T>(h, k - 1);
-  launch_vcycle<T>(h, k - 1, fused);
-  if (fused) launch_fill_prolong<T>(h, k, home);
-  else launch_prolong<T>(h, k, 1, home);
+  launch_vcycle<T>(h, k - 1);
+  launch_prolong<T>(h, k, 1, home);
   // the fill after the correction (ebVcycle.m:32) only feeds the first
   // post-smoothing pass, whose ghost reads then evaluate the same rules on
   // the same cells; the fill after the smoothing leaves the frame as the
@@ -1493,9 +1453,14 @@ int tune_level(bsam_hier h, int k, int *best) {
   *best = 1;
   const int ns = std::max(h->opts.npre, 1);
   std::vector<int> cand{1};
-  if (h->lev[k].tile[p].state == 1) cand.push_back(6);
   h->lev[k].dsm_shift[p] = dsm_shift_for<T>(h, k);
-  if (h->lev[k].dsm_shift[p] >= 0) cand.push_back(5);
+  // the one-cluster form only where the tables of the tiles cannot be had:
+  // with its fill it measured ahead of them on some FP32 levels of 700 to
+  // 2,000 cells by the tuner's margin, but not in the cycle, where the first
+  // relaxation's fill rides with the restriction (8.1 against 6.5 us there,
+  // 10.8 against 8.0 after the correction)
+  if (h->lev[k].tile[p].state == 1) cand.push_back(6);
+  else if (h->lev[k].dsm_shift[p] >= 0) cand.push_back(5);
   if (cand.size() > 1) {
     time_form<T>(h, k, 1, ns);           // warm-up: the first form timed is not the one that pays for it
     float bt = 1e30f;
@@ -2645,24 +2610,6 @@ int do_upload(bsam_hier h, const bsam_hier_desc *d) {
       h->lev[k].fuse_pre = ok;
       h->lev[k].fuse_top = ok && ring_ok;
     }
-    // windows: parent ghost cells -> the parent level's item filling them
-    std::vector<int> walt(d->win, d->win + d->n_win);
-    for (int k = 2; k <= d->nlev; ++k) {
-      const LevelPlan &L = h->lev[k], &Lc = h->lev[k - 1];
-      std::unordered_map<int, int> gh;     // parent Q ghost cell -> ghost item
-      for (int i = Lc.g1_off; i < Lc.g1_off + Lc.g1_n; ++i)
-        if (B.gt[i] != G_RING) gh[B.gdst[i]] = i;
-      for (int p = L.p0; p < L.p1; ++p) {
-        const int32_t *r = B.P(p);
-        const int nw = (r[PD_MX] / 2 + 2) * (r[PD_MY] / 2 + 2);
-        for (int w = r[PD_WIN0]; w < r[PD_WIN0] + nw; ++w) {
-          auto it = gh.find(d->win[w]);
-          if (it != gh.end()) walt[w] = -1 - it->second;
-        }
-      }
-    }
-    if (walt.empty()) walt.push_back(0);
-    if ((rc = h->win_alt.upload(walt.data(), walt.size(), s))) return rc;
     if (rt.empty()) rt.push_back(make_int2(0, 0));
     if ((rc = h->ga_a.upload(aa.data(), aa.size(), s)) || (rc = h->ga_b.upload(ab.data(), ab.size(), s)) ||
         (rc = h->ga_c.upload(ac.data(), ac.size(), s)) || (rc = h->ga_rt.upload(rt.data(), rt.size(), s)))
@@ -2730,7 +2677,7 @@ void release(bsam_hier h) {
     b->release();
   for (DBuf<int> *b : {&h->win, &h->fp, &h->ring, &h->ints, &h->ct_cell, &h->ct_patch, &h->ct_beg,
                        &h->active, &h->iters, &h->ones, &h->g_inst, &h->ring_inst, &h->inst_nlev, &h->g_dst, &h->g_a, &h->g_b, &h->g_c, &h->g_d, &h->g_e,
-                       &h->ga_a, &h->ga_b, &h->ga_c, &h->win_alt})
+                       &h->ga_a, &h->ga_b, &h->ga_c})
     b->release();
   h->flags.release(); h->g_type.release(); h->patches.release(); h->acc.release(); h->perim.release();
   h->rchunks.release(); h->pchunks.release(); h->cact.release(); h->crange.release(); h->levelx.release(); h->rtasks.release(); h->instres.release(); h->sranges.release();

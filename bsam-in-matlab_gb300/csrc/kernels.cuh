@@ -203,18 +203,25 @@ struct Decomp {
 // true division there, and the signed zero of the first product for x = 0.
 // A colour pass of a 15 x 11-based ragged level (660 cells): 4.1 us with
 // divisions, 3.6 with this; the three-level ragged solve 4.23 -> 3.95 ms.
-struct DivC {
-  double d, r;
+template <class T>
+struct DivK {
+  T d, r;
   int ops, kexp;               // kexp: what x / d adds to x's high word (ops 1)
   unsigned elo, espan;
 };
+using DivC = DivK<double>;
 
 __device__ __forceinline__ unsigned exp_bits(double x) { return ((unsigned)__double2hiint(x) >> 20) & 0x7ffu; }
 __device__ __forceinline__ bool is_zero(double x) {
   return (((unsigned)__double2hiint(x) << 1) | (unsigned)__double2loint(x)) == 0u;
 }
+__device__ __forceinline__ unsigned exp_bits(float x) { return (__float_as_uint(x) >> 23) & 0xffu; }
+__device__ __forceinline__ bool is_zero(float x) { return (__float_as_uint(x) << 1) == 0u; }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 
 __device__ __noinline__ double div_out_of_line(double x, double d) { return x / d; }
+__device__ __noinline__ float div_out_of_line(float x, float d) { return x / d; }
 
 // kPow2: the kernel's variant for levels where every constant is a power of
 // two (ops 1), which carries none of the other code
@@ -248,27 +255,64 @@ __device__ __forceinline__ void scale_faces(double (&c)[kN], const DivC &D, bool
     c[i] = in ? __hiloint2double(__double2hiint(c[i]) + D.kexp, __double2loint(c[i])) : c[i] * D.r;
 }
 
-// FP32: a divide is short there (with the steps above the ragged mixed solve
-// was 2% slower)
+// The quotients of several values at once, the first kX by dx and the rest by
+// dy: the steps of all of them overlap (an update's four were a chain of
+// about 1,000 cycles, one after the other because each has its out-of-range
+// branch), the range is looked at once, and the second step is taken if
+// either constant wants it (it leaves a correct quotient as it is).
+// Six passes of a tile: FP64 12 x 256 threads 10.3 us -> 8.5, FP32 9.2 -> 6.7
+// (three steps and a range test for FP32, where a divide alone is as short);
+// ragged three-level solve 2.86 -> 2.66 ms, ragged mixed solve 1.89 -> 1.78.
+template <int kX, int kN, bool kInt, class T>
+__device__ __forceinline__ void div_group(T (&x)[kN], const DivK<T> &dx, const DivK<T> &dy) {
+  T q[kN];
+  bool out = false;
+#pragma unroll
+  for (int i = 0; i < kN; ++i) {
+    const DivK<T> &D = i < kX ? dx : dy;
+    const T q0 = mul_on<kInt>(x[i], D.r);
+    q[i] = fma_rn(fma_rn(-q0, D.d, x[i]), D.r, q0);
+    out = out || exp_bits(x[i]) - D.elo > D.espan;
+  }
+  if (dx.ops == 5 || dy.ops == 5) {
+#pragma unroll
+    for (int i = 0; i < kN; ++i) {
+      const DivK<T> &D = i < kX ? dx : dy;
+      q[i] = fma_rn(fma_rn(-q[i], D.d, x[i]), D.r, q[i]);
+    }
+  }
+  if (out) {
+#pragma unroll
+    for (int i = 0; i < kN; ++i) {
+      const DivK<T> &D = i < kX ? dx : dy;
+      if (exp_bits(x[i]) - D.elo > D.espan) q[i] = is_zero(x[i]) ? x[i] * D.r : div_out_of_line(x[i], D.d);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < kN; ++i) x[i] = q[i];
+}
+
+// one FP32 quotient
 template <bool kPow2, bool kInt = false>
-__device__ __forceinline__ float div_c(float x, float d) { return x / d; }
+__device__ __forceinline__ float div_c(float x, const DivK<float> &D) { return x / D.d; }
 
 struct LevelD {
   const PatchD *patches;       // this level's patches
   double hx, hy;
   DivC dx, dy;                 // division by hx^2, hy^2
   int pow2;                    // hx2 and hy2 are powers of two
-  float fhx, fhy, fhx2, fhy2;  // FP32 copies for the correction cycle
+  float fhx, fhy;              // FP32 copies for the correction cycle
+  DivK<float> fdx, fdy;
 };
 
 // the level's cell sizes in the cycle's value type
 template <class T, class D2> struct LevelH {
   T hx, hy;
-  D2 dx, dy;                   // what div_c divides by
+  D2 dx, dy;                   // what div_c and div_group divide by
 };
 __device__ __forceinline__ LevelH<double, DivC> level_h(const LevelD &L, double) { return {L.hx, L.hy, L.dx, L.dy}; }
-__device__ __forceinline__ LevelH<float, float> level_h(const LevelD &L, float) {
-  return {L.fhx, L.fhy, L.fhx2, L.fhy2};
+__device__ __forceinline__ LevelH<float, DivK<float>> level_h(const LevelD &L, float) {
+  return {L.fhx, L.fhy, L.fdx, L.fdy};
 }
 
 // `b` is the block index within the decomposition
@@ -284,7 +328,9 @@ template <bool kPow2, bool kInt = false>
 __device__ __forceinline__ double op_flux(double feE, double feW, double fnN, double fnS, double cc, double q,
                                           const LevelD &L) {
   if (kPow2) return (-(feE - feW) - (fnN - fnS)) + mul_on<kInt>(cc, q);
-  return (div_c<false, kInt>(-(feE - feW), L.dx) - div_c<false, kInt>(fnN - fnS, L.dy)) + mul_on<kInt>(cc, q);
+  double d[2] = {-(feE - feW), fnN - fnS};
+  div_group<1, 2, kInt>(d, L.dx, L.dy);
+  return (d[0] - d[1]) + mul_on<kInt>(cc, q);
 }
 
 // the same from its values and (unscaled) coefficients
@@ -292,7 +338,10 @@ template <bool kPow2>
 __device__ __forceinline__ double op_pre(double q, double qe, double qw, double qn, double qs, double dE, double dW,
                                          double dN, double dS, double cc, const LevelD &L) {
   const double feE = dE * (qe - q), feW = dW * (q - qw), fnN = dN * (qn - q), fnS = dS * (q - qs);
-  return (div_c<kPow2>(-(feE - feW), L.dx) - div_c<kPow2>(fnN - fnS, L.dy)) + cc * q;
+  if (kPow2) return (div_c<true>(-(feE - feW), L.dx) - div_c<true>(fnN - fnS, L.dy)) + cc * q;
+  double d[2] = {-(feE - feW), fnN - fnS};
+  div_group<1, 2, false>(d, L.dx, L.dy);
+  return (d[0] - d[1]) + cc * q;
 }
 
 // the same at interior cell (li, lj) of a padded array
@@ -335,25 +384,6 @@ __device__ __forceinline__ T rule_value(int type, T qa, T qb, T qc, T qd, T qe) 
     case G_QIF: return (A1 * qa + A2 * qb) + A3 * qc;
     case G_QIF_END: return (A1 * qa + A2 * qb) + A3 * ((B1 * qc + B2 * qd) + B3 * qe);
     default: return (c23 * qc + c23 * qa) - c13 * qb;   // G_LIF
-  }
-}
-
-template <class T, bool kCG = false>
-__device__ __forceinline__ T eval_rule(const GhostItems &G, int i, const T *Q, const T *bcg, T hx, T hy) {
-  const T A1 = T(-1.0 / 5.0), A2 = T(2.0 / 3.0), A3 = T(8.0 / 15.0);
-  const T B1 = T(5.0 / 32.0), B2 = T(15.0 / 16.0), B3 = T(-3.0 / 32.0);
-  const T c23 = T(2.0 / 3.0), c13 = T(1.0 / 3.0), c83 = T(8.0 / 3.0);
-  const int a = G.a[i];
-  auto q = [&](int j) { return ld_sol<kCG>(Q + j); };
-  switch (G.type[i]) {
-    case G_COPY: return q(a);
-    case G_QIF: return (A1 * q(a) + A2 * q(G.b[i])) + A3 * q(G.c[i]);
-    case G_QIF_END:
-      return (A1 * q(a) + A2 * q(G.b[i])) + A3 * ((B1 * q(G.c[i]) + B2 * q(G.d[i])) + B3 * q(G.e[i]));
-    case G_LIF: return (c23 * q(G.c[i]) + c23 * q(a)) - c13 * q(G.b[i]);
-    case G_LIF_CORNER: return c23 * q(G.c[i]) + c13 * q(a);
-    case G_DIRICHLET: return (c83 * bcg[G.e[i]] - 2 * q(a)) + c13 * q(G.b[i]);
-    default: return q(a) + (G.b[i] ? hy : hx) * bcg[G.e[i]];   // G_NEUMANN
   }
 }
 
@@ -447,8 +477,8 @@ __device__ __forceinline__ T ghost_operand(const T *Q, int code, const GhostAlt 
   return ld_sol<kCG>(Q + code);
 }
 
-// a ghost's value from its operands and boundary part (eval_rule's
-// arithmetic, every kind but the ring refresh and the physical corner)
+// a ghost's value from its operands and boundary part (every kind but the
+// ring refresh and the physical corner)
 template <class T>
 __device__ __forceinline__ T ghost_formula(int ty, T qa, T qb, T qc, T qd, T qe, T g) {
   const T c23 = T(2.0 / 3.0), c13 = T(1.0 / 3.0);
@@ -810,10 +840,9 @@ __device__ __forceinline__ void cell_update(const LevelD &L, const FieldsT<T> &f
     t = t + qn * S.dN;
     t = t + qs * S.dS;
   } else {
-    t = t + div_c<false>(qe * S.dE, H.dx);
-    t = t + div_c<false>(qw * S.dW, H.dx);
-    t = t + div_c<false>(qn * S.dN, H.dy);
-    t = t + div_c<false>(qs * S.dS, H.dy);
+    T d[4] = {qe * S.dE, qw * S.dW, qn * S.dN, qs * S.dS};
+    div_group<2, 4, false>(d, H.dx, H.dy);
+    t = (((t + d[0]) + d[1]) + d[2]) + d[3];
   }
   t = t * S.idg;
   if (unit_omega) Q[c] = t;
@@ -1120,10 +1149,9 @@ __global__ void __launch_bounds__(kT, (sizeof(T) == 4 ? 8 : 5) * (kBlock / kT))
     v = v + mul_on<kInt>(qn, S.dN);
     v = v + mul_on<kInt>(qs, S.dS);
   } else {
-    v = v + div_c<false, kInt>(mul_on<kInt>(qe, S.dE), H.dx);
-    v = v + div_c<false, kInt>(mul_on<kInt>(qw, S.dW), H.dx);
-    v = v + div_c<false, kInt>(mul_on<kInt>(qn, S.dN), H.dy);
-    v = v + div_c<false, kInt>(mul_on<kInt>(qs, S.dS), H.dy);
+    T d[4] = {mul_on<kInt>(qe, S.dE), mul_on<kInt>(qw, S.dW), mul_on<kInt>(qn, S.dN), mul_on<kInt>(qs, S.dS)};
+    div_group<2, 4, kInt>(d, H.dx, H.dy);
+    v = (((v + d[0]) + d[1]) + d[2]) + d[3];
   }
   v = v * S.idg;
   if (unit_omega) f.Q[c] = v;
@@ -1352,7 +1380,7 @@ __device__ __forceinline__ void dsm_cell_update(const LevelD &L, const FieldsT<T
   else dsm_st(ac, omega * t + (1 - omega) * dsm_ld(ac, T(0)));
 }
 
-// one ghost rule's value (eval_rule's arithmetic) from the cluster's copy
+// one ghost rule's value from the cluster's copy
 template <class T>
 __device__ __forceinline__ T ghost_eval_dsm(const GhostItems &G, int i, const FieldsT<T> &f, T hx, T hy,
                                             const DsmRange<T> &D) {
@@ -1706,11 +1734,18 @@ __device__ __forceinline__ void load_fp_item(const LevelD &L, const LevelD &Lc, 
       fy[i][j] = mul_on<kInt>(dy[2 * i + j], v[i + 1][j + 1] - v[i][j + 1]);
     }
   const T *Fp = f.F + c_off + 2 * ci + 2 * cj * mx;
+  double dd[8];                // the four cells' flux differences
 #pragma unroll
   for (int t = 0; t < 4; ++t) {
     const int i = t & 1, j = t >> 1;
-    rf[t] = dbl(Fp[i + j * mx]) -
-            op_flux<kPow2, kInt>(fx[j][i + 1], fx[j][i], fy[j + 1][i], fy[j][i], cf[t], v[j + 1][i + 1], L);
+    dd[t] = -(fx[j][i + 1] - fx[j][i]);
+    dd[4 + t] = fy[j + 1][i] - fy[j][i];
+  }
+  if (!kPow2) div_group<4, 8, kInt>(dd, L.dx, L.dy);
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    const int i = t & 1, j = t >> 1;
+    rf[t] = dbl(Fp[i + j * mx]) - ((dd[t] - dd[4 + t]) + mul_on<kInt>(cf[t], v[j + 1][i + 1]));
   }
   const double rr = 0.25 * (((rf[0] + rf[1]) + rf[2]) + rf[3]);
   const T *QC = f.QC + qc_off;
@@ -1779,37 +1814,9 @@ __global__ void __launch_bounds__(kT) k_load(LevelD L, LevelD Lc, Decomp D, Fiel
 // 15.3, 379,536 in patches 8.5 -> 7.5.  (Threads of two or four coarse cells
 // that share their differences took 13.2 us on the former, but 4.7 to 8
 // instead of 3.3 on small levels.)
-// A parent-window operand of the prolongation fused with the parent level's
-// closing fill (k_fill_prolong): a code >= 0 is a cell of Q; a code < 0 is
-// the ghost cell that ghost item -1 - code fills in the same launch, whose
-// value the prolongation forms itself from the item's rule (the rule reads
-// interior cells and the level below, which the launch does not write) --
-// the value the fill stores, bit for bit.
-template <class T>
-struct WindowGhosts {
-  const int *win;              // window tables, ghost cells coded
-  GhostItems G;
-  const T *bcg;
-  T hx, hy;                    // cell size of the parent level (the ghosts' level)
-};
-
-template <class T>
-__device__ __forceinline__ T window_value(const T *Q, int code, const WindowGhosts<T> *W) {
-  if (W == nullptr || code >= 0) return Q[code];
-  const int i = -1 - code;
-  const GhostItems &G = W->G;
-  const int8_t ty = G.type[i];
-  if (ty == G_PHYS_CORNER) {
-    const T v1 = eval_rule<T>(G, G.a[i], Q, W->bcg, W->hx, W->hy);
-    const T v2 = eval_rule<T>(G, G.b[i], Q, W->bcg, W->hx, W->hy);
-    return (v1 + v2) - Q[G.c[i]];
-  }
-  return eval_rule<T>(G, i, Q, W->bcg, W->hx, W->hy);
-}
-
 template <class T, bool kChain, bool kInt>
 __device__ __forceinline__ void prolong_item(const LevelD &L, const Decomp &D, const FieldsT<T> &f, int correct,
-                                             int g, const WindowGhosts<T> *W = nullptr) {
+                                             int g) {
   if (g >= D.n) {
     if (kChain) chain_wait();
     return;
@@ -1824,7 +1831,7 @@ __device__ __forceinline__ void prolong_item(const LevelD &L, const Decomp &D, c
   const int s = g - __ldg(D.beg + p);
   const int b = s / cm, a = s - b * cm;
   const int ldw = cm + 2;
-  const int *win = (W ? W->win : f.win) + P.win_off;
+  const int *win = f.win + P.win_off;
   int src[3][3];
 #pragma unroll
   for (int dj = 0; dj < 3; ++dj)
@@ -1839,7 +1846,7 @@ __device__ __forceinline__ void prolong_item(const LevelD &L, const Decomp &D, c
 #pragma unroll
     for (int di = 0; di < 3; ++di) {
       const int w = (a + di) + (b + dj) * ldw;
-      const T wv = window_value<T>(f.Q, src[dj][di], W);
+      const T wv = f.Q[src[dj][di]];
       E[dj][di] = correct ? wv - QC[w] : wv;
     }
   const T c9 = times<9, kInt>(E[1][1]);
@@ -1869,31 +1876,6 @@ __device__ __forceinline__ void prolong_item(const LevelD &L, const Decomp &D, c
 template <class T, bool kInt, int kT = kBlock>
 __global__ void __launch_bounds__(kT) k_prolong(LevelD L, Decomp D, FieldsT<T> f, int correct) {
   prolong_item<T, true, kInt>(L, D, f, correct, blockIdx.x * kT + threadIdx.x);
-}
-
-// The closing ghost fill of level k-1 (the end of its V-cycle) and the
-// prolongation-correction of level k that follows it (ebVcycle.m:31-32) in
-// one launch: blocks [0, nb_g) fill level k-1, the rest prolong into level
-// k, forming any parent-window ghost from its rule (WindowGhosts), so no
-// item reads what another item of the launch writes.
-template <class T, int kT = kBlock>
-__global__ void __launch_bounds__(kT) k_fill_prolong(GhostItems G, int g_off, int g_n, int nb_g, LevelD L, Decomp D,
-                                                    FieldsT<T> f, int correct, WindowGhosts<T> W,
-                                                    const int *__restrict__ active,
-                                                    const int *__restrict__ inst_nlev) {
-  if ((int)blockIdx.x < nb_g) {
-    const int t = blockIdx.x * kT + threadIdx.x;
-    const int i = g_off + t;
-    const int inst = (t < g_n && G.inst) ? G.inst[i] : -1;
-    const bool skip = t >= g_n || (inst >= 0 && !active[inst]);
-    GhostPre<T> X;
-    if (!skip) X = ghost_pre<T>(G, i, G.type[i], G.dst[i], f.bcg, W.hx, W.hy);
-    chain_wait();
-    if (skip) return;
-    ghost_apply<T>(X, f.Q, f.QC);
-    return;
-  }
-  prolong_item<T, true, false>(L, D, f, correct, ((int)blockIdx.x - nb_g) * kT + threadIdx.x, &W);
 }
 
 // ---------------------------------------------------------------------------

@@ -352,8 +352,12 @@ __host__ __device__ inline size_t tile_smem(int win, int cap, int nf) {
 // second colour) from src to dst, two copies of the level's cells; nothing
 // else of either array is read or written, but with `stored` the first pass
 // reads the coarse-fine ghosts stored in src, as the last fill left them.
+// Five blocks per SM for FP32: left alone the compiler holds it to 32
+// registers, with its loads one after the other (114,756 cells 1.71 us a pass,
+// with 40 registers 1.70, with 48 1.54); FP64 keeps the 40 to 56 it takes by
+// itself (64: no faster).
 template <class T, bool kPow2>
-__global__ void __launch_bounds__(kTileT)
+__global__ void __launch_bounds__(kTileT, sizeof(T) == 4 ? 5 : 1)
     k_relax_tile(LevelD L, const TileD *__restrict__ tiles, const TileTab *__restrict__ tab,
                  const int *__restrict__ wq, const TileEnt *__restrict__ ent, const TileFace *__restrict__ face,
                  FieldsT<T> f, const T *src, T *dst, const T *__restrict__ pack, int passes, int stored, T omega,
@@ -454,16 +458,15 @@ __global__ void __launch_bounds__(kTileT)
       }
     }
     const T dE = op[e], dW = op[cap + e], dN = op[2 * cap + e], dS = op[3 * cap + e];
-    if (kPow2) {
+    if constexpr (kPow2) {
       v = v + qe * dE;
       v = v + qw * dW;
       v = v + qn * dN;
       v = v + qs * dS;
     } else {
-      v = v + div_c<false>(qe * dE, H.dx);
-      v = v + div_c<false>(qw * dW, H.dx);
-      v = v + div_c<false>(qn * dN, H.dy);
-      v = v + div_c<false>(qs * dS, H.dy);
+      T d[4] = {qe * dE, qw * dW, qn * dN, qs * dS};
+      div_group<2, 4, false>(d, H.dx, H.dy);
+      v = (((v + d[0]) + d[1]) + d[2]) + d[3];
     }
     v = v * op[4 * cap + e];
     if (unit_omega) win[c] = v;
