@@ -217,6 +217,7 @@ struct bsam_hier_s {
   int act_mode = 0;                // kActNone (one instance) / kActChunk (batch)
   DBuf<LevelX> levelx;             // per-level descriptors for the residual
   DBuf<ResTask> rtasks;            // residual warp tasks
+  int res_rows = kResRowsMax;      // cells of a column per item of theirs
   DBuf<InstRes> instres;           // per-instance residual reduction plan
   DBuf<SlotRange> sranges;
   DBuf<CoarsestD> coarsest;        // one coarsest operator per instance
@@ -329,6 +330,19 @@ inline int nblk(int n) { return (n + kBlock - 1) / kBlock; }
 // 114,756: 3.15 / 2.78, 379,536: 5.87 / 5.19, 262,144 (one patch): 4.82 /
 // 3.59, 1,048,576: 11.8 / 9.06; but 4,096: 1.72 / 1.88, 11,328: 2.40 / 2.40.
 constexpr int64_t kIntMinCells = 16384;
+
+// levels below this take four lanes per footprint cell in the coarse load
+// (load_fp_quad), larger ones, whose FP64 pipes it would keep busy with
+// fluxes formed twice, one.  Solve, ms without / levels below 16,384 / below
+// 65,536 cells: ragged FP64 2.67 / 2.60 / 2.57, disc 1.32 / 1.26 / 1.25, ragged
+// mixed 1.79 / 1.69 / 1.69, starfish (its levels reach 379,536) 3.13 / 3.12 / 3.13.
+constexpr int64_t kQuadMaxCells = 65536;
+
+// hierarchies below this many cells take one cell per residual item, larger
+// ones kResRowsMax cells of a column, whose inner fluxes are formed once.
+// Solve, ms with columns / single cells: 1,280 cells 0.408 / 0.398, 16,384
+// 1.316 / 1.288, 75,000 2.67 / 2.64, 550,000 3.13 / 3.18.
+constexpr int64_t kResRowCells = 131072;
 
 // kernels whose kBlock grid has fewer blocks than this run with 64-thread
 // (or one-chunk) blocks: an SM issues about two FP64 operations per clock,
@@ -1070,15 +1084,17 @@ void launch_coarse_load(bsam_hier h, int k, int home = 0) {
   // instances left a 256-thread block of 40 operations a thread is 3 us of its
   // SM's FP64 pipe (14 of 64 instances, 473 blocks: 9.9 us, 1,887: 4.5)
   const bool spread = D.nblocks < 8 * sm_count();
+  const bool quad = L.ncells < kQuadMaxCells;
   const int kt = spread ? 64 : kBlock;
   auto nb = [&](int n) { return (n + kt - 1) / kt; };
   auto go = [&](auto kern) {
-    launch_k(h, kern, nb(L.ring_n) + nb(D.n) + nb(ntgt), kt, leveld(h, k), leveld(h, k - 1), D, fields_at<T>(h, home),
+    launch_k(h, kern, nb(L.ring_n) + nb(quad ? 4 * D.n : D.n) + nb(ntgt), kt, leveld(h, k), leveld(h, k - 1), D, fields_at<T>(h, home),
              (const int *)h->ring.p, ri, L.ring_off, L.ring_n, corr_csr(h, L), ntgt);
   };
   auto pick = [&](auto pow2, auto ints) {
     constexpr bool p2 = decltype(pow2)::value, in = decltype(ints)::value;
-    if (spread) go(k_load<T, p2, in, 64>);
+    if (quad) go(k_load<T, p2, false, 64, true>);
+    else if (spread) go(k_load<T, p2, in, 64>);
     else go(k_load<T, p2, in>);
   };
   const bool p2 = L.pow2 && h->lev[k - 1].pow2;
@@ -1217,7 +1233,8 @@ void launch_residual(bsam_hier h, int mode, const LoopCond &c = LoopCond()) {
     const int g64 = (h->nres + 1) / 2;
     auto pick = [&](auto l2, auto pow2, auto ints) {
       constexpr bool a = decltype(l2)::value, p2 = decltype(pow2)::value, in = decltype(ints)::value;
-      if (small) go(k_residual<a, p2, in, 64>, g64, 64);
+      if (h->res_rows == 1) go(k_residual<a, p2, in, 64, 1>, g64, 64);
+      else if (small) go(k_residual<a, p2, in, 64>, g64, 64);
       else go(k_residual<a, p2, in>, g256, kBlock);
     };
     const std::true_type y{};
@@ -2036,13 +2053,22 @@ struct Builder {
       if (r[PD_CCNE] == 1) corners.push_back({G_PHYS_CORNER, Q(mx + 2, my + 2), Q(mx + 1, my + 2), Q(mx + 2, my + 1), Q(mx + 1, my + 1), 0, 0, cur});
     }
     if (outside) return fail(BSAM_ERR_ARG, "ghost destination outside its level's patches");
+    // the rules by kind (each gives its ghost's final value, so their order is
+    // free): a warp that fills ghosts of several kinds goes through the FP64
+    // chain of each (ragged solve 2.58 -> 2.50 ms, starfish 3.10 -> 3.07)
+    int first[10] = {};
+    for (const G &g : tmp) ++first[g.t + 1];
+    for (int t = 0; t < 9; ++t) first[t + 1] += first[t];
+    std::vector<int> pos(tmp.size());
+    std::vector<G> sorted(tmp.size());
+    for (size_t i = 0; i < tmp.size(); ++i) sorted[pos[i] = first[tmp[i].t]++] = tmp[i];
     L.g1_off = (int)gt.size();
     for (G &g : corners) {
       if (rule_at(g.dst) >= 0) return fail(BSAM_ERR_ARG, "physical corner also written by another ghost stage");
       const int i1 = rule_at(g.a), i2 = rule_at(g.b);
       if (i1 < 0 || i2 < 0) return fail(BSAM_ERR_ARG, "physical corner next to a ghost without a rule");
-      g.a = L.g1_off + i1;
-      g.b = L.g1_off + i2;
+      g.a = L.g1_off + pos[i1];
+      g.b = L.g1_off + pos[i2];
     }
     auto emit = [&](const std::vector<G> &v) {
       for (const G &g : v) {
@@ -2050,7 +2076,7 @@ struct Builder {
         gc.push_back(g.c); gd.push_back(g.dd); ge.push_back(g.e); gi.push_back(g.inst);
       }
     };
-    emit(tmp);
+    emit(sorted);
     emit(ringi);
     emit(corners);
     L.g1_n = (int)gt.size() - L.g1_off;
@@ -2408,6 +2434,7 @@ int do_upload(bsam_hier h, const bsam_hier_desc *d) {
   // the longest, come first in the list; then the QC refresh tasks of the
   // levels above each instance's root
   constexpr int kTask = 128;
+  h->res_rows = d->n_cells < kResRowCells ? 1 : kResRowsMax;
   std::vector<ResTask> tasks, cells;
   std::vector<SlotRange> ranges;
   std::vector<InstRes> ir(h->ninst);
@@ -2421,13 +2448,13 @@ int do_upload(bsam_hier h, const bsam_hier_desc *d) {
       for (int p = L.p0; p < L.p1; ++p) {
         if (pinst[p] != i) continue;
         const int32_t *r = B.P(p);
-        const int n = r[PD_MX] * r[PD_MY], nc = r[PD_MX] * ((r[PD_MY] + kResRows - 1) / kResRows);
+        const int n = r[PD_MX] * r[PD_MY], nc = r[PD_MX] * ((r[PD_MY] + h->res_rows - 1) / h->res_rows);
         for (int c = 0; c < n; ++c) h->inst_visible[i] += (d->covered[r[PD_COFF] + c] == 0);
         // items all of whose cells a finer level covers contribute nothing
         const uint8_t *cov = d->covered + r[PD_COFF];
         auto visible = [&](int e) {
-          const int x = e % r[PD_MX], y0 = e / r[PD_MX] * kResRows;
-          for (int y = y0; y < std::min(y0 + kResRows, (int)r[PD_MY]); ++y)
+          const int x = e % r[PD_MX], y0 = e / r[PD_MX] * h->res_rows;
+          for (int y = y0; y < std::min(y0 + h->res_rows, (int)r[PD_MY]); ++y)
             if (!cov[x + y * r[PD_MX]]) return true;
           return false;
         };

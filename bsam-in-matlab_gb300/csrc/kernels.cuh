@@ -1758,6 +1758,61 @@ __device__ __forceinline__ void load_fp_item(const LevelD &L, const LevelD &Lc, 
   f.F[dst] = T(rr + lc);
 }
 
+// The same with a footprint cell on four lanes, one fine cell each, which
+// also form one flux each of the coarse operator, for levels whose launch
+// waits for one thread's 84 to 110 operations (a warp's FP64 operation takes
+// its SM 19 cycles whatever else waits) and for that much straight-line code:
+// 40 to 50 operations here.  A level of 1,000 to 6,000 cells 3.4 to 4.0 us ->
+// 2.2 to 3.0, ragged (with divisions) mixed 6.6 -> 4.7.
+template <class T, bool kPow2, bool kChain>
+__device__ __forceinline__ void load_fp_quad(const LevelD &L, const LevelD &Lc, const Decomp &D, const FieldsT<T> &f,
+                                             int g4) {
+  const int g = g4 >> 2, t = g4 & 3;
+  if (g >= D.n) {
+    if (kChain) chain_wait();
+    return;
+  }
+  const int p = find_patch(D, g / kBlock, g);
+  const PatchD &P = L.patches[p];
+  if (!f.active[P.inst]) {
+    if (kChain) chain_wait();
+    return;
+  }
+  const int mx = P.mx, cmx = mx >> 1, cmy = P.my >> 1, ldq = mx + 2;
+  const int s = g - __ldg(D.beg + p);
+  const int cj = s / cmx, ci = s - cj * cmx;
+  const int li = 2 * ci + (t & 1), lj = 2 * cj + (t >> 1), cell = P.c_off + li + lj * mx;
+  const T *DeW = f.DeW + P.dew_off + li + lj * (mx + 1), *DnS = f.DnS + P.dns_off + li + lj * mx;
+  double dx[2] = {dbl(__ldg(DeW + 1)), dbl(__ldg(DeW))}, dy[2] = {dbl(__ldg(DnS + mx)), dbl(__ldg(DnS))};
+  const double cf = dbl(__ldg(f.CC + cell));
+  // the lane's face of the coarse cell, E W N S: its neighbour, ring cells
+  // from the parent's Q
+  const int ldc = cmx + 2, w = (ci + 1) + (cj + 1) * ldc, step = (t & 1 ? -1 : 1) * (t < 2 ? 1 : ldc);
+  const bool edge = t == 0 ? ci == cmx - 1 : t == 1 ? ci == 0 : t == 2 ? cj == cmy - 1 : cj == 0;
+  const T *nb = edge ? f.Q + __ldg(f.win + P.win_off + w + step) : f.QC + P.qc_off + w + step;
+  const T *PDeW = f.pcoef + P.pc_off, *PDnS = PDeW + (cmx + 1) * cmy, *PCC = PDnS + cmx * (cmy + 1);
+  double pd[1] = {dbl(__ldg(t < 2 ? PDeW + ci + (t == 0) + cj * (cmx + 1) : PDnS + ci + (cj + (t == 2)) * cmx))};
+  const double pC = dbl(__ldg(PCC + s));
+  const int dst = __ldg(f.fp + 2 * (P.fp_off + s) + 1);
+  if (kPow2) {
+    const DivC &Dp = t < 2 ? Lc.dx : Lc.dy;
+    scale_faces(dx, L.dx, faces_in(dx, L.dx));
+    scale_faces(dy, L.dy, faces_in(dy, L.dy));
+    scale_faces(pd, Dp, faces_in(pd, Dp));
+  }
+  if (kChain) chain_wait();
+  const T *Q = f.Q + P.q_off + f.lsh + (li + 1) + (lj + 1) * ldq;
+  const double v = dbl(Q[0]), ve = dbl(Q[1]), vw = dbl(Q[-1]), vn = dbl(Q[ldq]), vs = dbl(Q[-ldq]);
+  const double F = dbl(f.F[cell]), q = dbl(f.QC[P.qc_off + w]), qb = dbl(*nb);
+  const double fl = pd[0] * ((t & 1) ? q - qb : qb - q);
+  const double rf = F - op_flux<kPow2>(dx[0] * (ve - v), dx[1] * (v - vw), dy[0] * (vn - v), dy[1] * (v - vs), cf, v, L);
+  const unsigned quad = 0xfu << (threadIdx.x & 28);
+  auto from = [&](double x, int l) { return __shfl_sync(quad, x, l, 4); };
+  const double rr = 0.25 * (((from(rf, 0) + from(rf, 1)) + from(rf, 2)) + from(rf, 3));
+  const double lc = op_flux<kPow2>(from(fl, 0), from(fl, 1), from(fl, 2), from(fl, 3), pC, q, Lc);
+  if (t == 0) f.F[dst] = T(rr + lc);
+}
+
 template <class T, bool kPow2, bool kChain>
 __device__ __forceinline__ void load_corr_item(const LevelD &L, const LevelD &Lc, const FieldsT<T> &f, const CorrCSR &C,
                                                int n_tgt, int t) {
@@ -1782,12 +1837,12 @@ __device__ __forceinline__ void load_corr_item(const LevelD &L, const LevelD &Lc
 // kT threads per block (kBlock, or 64 on a level whose kBlock grid leaves
 // SMs idle: a footprint cell is ~84 FP64 operations, and an SM issues about
 // two per clock); the decomposition's per-block patch table is kBlock-based
-template <class T, bool kPow2, bool kInt, int kT = kBlock>
+template <class T, bool kPow2, bool kInt, int kT = kBlock, bool kQuad = false>
 __global__ void __launch_bounds__(kT) k_load(LevelD L, LevelD Lc, Decomp D, FieldsT<T> f, const int *__restrict__ ring,
                                              const int *__restrict__ ring_inst, int ring_off, int n_ring, CorrCSR C,
                                              int n_tgt) {
   const int nb_ring = (n_ring + kT - 1) / kT;
-  const int nb_fp = (D.n + kT - 1) / kT;
+  const int nb_fp = ((kQuad ? 4 : 1) * D.n + kT - 1) / kT;
   int b = blockIdx.x;
   if (b < nb_ring) {
     load_ring_item<T, true>(f, ring, ring_inst, ring_off, n_ring, b * kT + threadIdx.x);
@@ -1795,7 +1850,8 @@ __global__ void __launch_bounds__(kT) k_load(LevelD L, LevelD Lc, Decomp D, Fiel
   }
   b -= nb_ring;
   if (b < nb_fp) {
-    load_fp_item<T, kPow2, kInt, true>(L, Lc, D, f, b * kT + threadIdx.x);
+    if constexpr (kQuad) load_fp_quad<T, kPow2, true>(L, Lc, D, f, b * kT + threadIdx.x);
+    else load_fp_item<T, kPow2, kInt, true>(L, Lc, D, f, b * kT + threadIdx.x);
     return;
   }
   b -= nb_fp;
@@ -2008,7 +2064,7 @@ __global__ void __launch_bounds__(32 * kBWarps, 7) k_coarsest_batch(const double
 //   kind 0  r = FTrue - op(Q) on visible cells of a patch in the norms,
 //           correction targets excluded while the corrections are on; an item
 //           is kResRows cells of one column, whose inner y fluxes are formed
-//           once
+//           once, or on small hierarchies a single cell
 //   kind 1  r at correction targets of a level, corrections added in order,
 //           the coarse values taken as the refreshed QC holds them
 // and, in a launch of their own (k_qc_refresh), tasks of up to 128 items:
@@ -2052,11 +2108,11 @@ __device__ __forceinline__ double pmax(double a, double b) {
   return __longlong_as_double(m < 0 ? 0 : m);
 }
 
-constexpr int kResRows = 4;
+constexpr int kResRowsMax = 4;
 
 // kT threads per block (kBlock, or 64 where the kBlock grid would leave
 // SMs with unequal shares of the FP64 work)
-template <bool kL2, bool kPow2, bool kInt, int kT = kBlock>
+template <bool kL2, bool kPow2, bool kInt, int kT = kBlock, int kResRows = kResRowsMax>
 __global__ void __launch_bounds__(kT) k_residual(const LevelX *__restrict__ X, const PatchD *__restrict__ patches,
                                                  const ResTask *__restrict__ tasks, int ntask, Fields f, double *slots,
                                                  int nslots, unsigned long long *norms, int want_fn, int mass_corr,

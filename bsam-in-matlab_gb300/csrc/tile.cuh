@@ -354,8 +354,8 @@ __host__ __device__ inline size_t tile_smem(int win, int cap, int nf) {
 // reads the coarse-fine ghosts stored in src, as the last fill left them.
 // Five blocks per SM for FP32: left alone the compiler holds it to 32
 // registers, with its loads one after the other (114,756 cells 1.71 us a pass,
-// with 40 registers 1.70, with 48 1.54); FP64 keeps the 40 to 56 it takes by
-// itself (64: no faster).
+// with 40 registers 1.70, with 48 1.54).  FP64 takes what it wants (ragged
+// solve 2.64 ms with 70 to 88 registers or with 85, 2.68 with 64, 2.73 with 48).
 template <class T, bool kPow2>
 __global__ void __launch_bounds__(kTileT, sizeof(T) == 4 ? 5 : 1)
     k_relax_tile(LevelD L, const TileD *__restrict__ tiles, const TileTab *__restrict__ tab,
