@@ -1116,6 +1116,10 @@ void launch_prolong(bsam_hier h, int k, int correct, int home = 0) {
     launch_k(h, kern, (D.n + kt - 1) / kt, kt, leveld(h, k), D, fields_at<T>(h, home), correct);
   };
   const bool small = D.nblocks < spread_limit(h);
+  if (L.ncells < 2 * kQuadMaxCells) {
+    launch_k(h, k_prolong<T, false, 64, true>, (4 * D.n + 63) / 64, 64, leveld(h, k), D, fields_at<T>(h, home), correct);
+    return;
+  }
   if (sizeof(T) == sizeof(double) && L.ncells >= kIntMinCells) {
     if (small) go(k_prolong<T, true, 64>, 64);
     else go(k_prolong<T, true>, kBlock);
