@@ -208,6 +208,7 @@ struct bsam_hier_s {
   // footprint coded -1 - (entry of ga_rt)
   DBuf<int> ga_a, ga_b, ga_c;
   DBuf<int2> ga_rt;
+  DBuf<CornerRec> g_corner, ga_corner;   // physical corners: plain and fused-fill operands
   DBuf<PatchD> patches;
   DBuf<ResAcc> acc;
   DBuf<Rule> perim;                // per-patch perimeter ghost rules (inline)
@@ -413,7 +414,7 @@ enum { K_RELAX, K_GHOST, K_RESTRICT, K_RING, K_LOAD, K_CORR, K_PROLONG, K_COARSE
 // ---------------------------------------------------------------------------
 GhostItems ghost_items(bsam_hier h) {
   return GhostItems{h->g_type.p, h->g_dst.p, h->g_a.p, h->g_b.p, h->g_c.p, h->g_d.p, h->g_e.p,
-                    h->ninst > 1 ? h->g_inst.p : nullptr};
+                    h->ninst > 1 ? h->g_inst.p : nullptr, h->g_corner.p};
 }
 
 // the arrays of the FP64 solve or of the FP32 correction cycle
@@ -1054,7 +1055,7 @@ void launch_restrict_fill(bsam_hier h, int k, int fill_k = FILL_NONE, int need =
   Decomp D = decomp(h, L.coarse);
   FieldsT<T> f = fields_at<T>(h, home);
   Launch l(h, K_RESTRICT, 12.0 * tscale<T>() * (double)L.ncells, k);
-  const GhostAlt A{h->ga_a.p, h->ga_b.p, h->ga_c.p, h->ga_rt.p, home};
+  const GhostAlt A{h->ga_a.p, h->ga_b.p, h->ga_c.p, h->ga_rt.p, h->ga_corner.p, home};
   const int fn = fill_k ? L.g1_n : 0, fring = fill_k == FILL_TOP ? 1 : 0, fzero = fill_k == FILL_ZERO ? 1 : 0;
   const bool small = nblk(D.n) + nblk(Lc.g1_n) + nblk(fn) < spread_limit(h);
   const int kt = small ? 64 : kBlock;
@@ -2641,6 +2642,43 @@ int do_upload(bsam_hier h, const bsam_hier_desc *d) {
       h->lev[k].fuse_pre = ok;
       h->lev[k].fuse_top = ok && ring_ok;
     }
+    std::vector<CornerRec> crn, crna;
+    for (size_t i = 0; i < B.gt.size(); ++i) {
+      if (B.gt[i] != G_PHYS_CORNER) continue;
+      CornerRec plain{}, alt{};
+      for (int m = 0; m < 2; ++m) {
+        const int r = m ? B.gb[i] : B.ga[i];
+        const int8_t t = B.gt[r];
+        const bool ub = t == G_QIF || t == G_QIF_END || t == G_LIF || t == G_DIRICHLET;
+        const bool uc = t == G_QIF || t == G_QIF_END || t == G_LIF || t == G_LIF_CORNER, ue = t == G_QIF_END;
+        GhostRule &P = plain.r[m], &A = alt.r[m];
+        P.ty = t;
+        P.a = B.ga[r];
+        P.b = ub ? B.gb[r] : P.a;
+        P.c = uc ? B.gc[r] : P.a;
+        P.d = ue ? B.gd[r] : P.a;
+        P.e = ue ? B.ge[r] : P.a;
+        P.g = t == G_DIRICHLET || t == G_NEUMANN ? B.ge[r] : 0;
+        P.nb = t == G_NEUMANN ? B.gb[r] : 0;
+        P.x = m ? 0 : B.gc[i];
+        auto cells = [&](int v, int &at, int &ld) {
+          at = v < 0 ? rt[-1 - v].x : v;
+          ld = v < 0 ? rt[-1 - v].y : 0;
+        };
+        A = P;
+        cells(aa[r], A.a, A.la);
+        if (ub) cells(ab[r], A.b, A.lb);
+        if (uc) cells(ac[r], A.c, A.lc);
+      }
+      alt.r[0].x = ac[i] < 0 ? rt[-1 - ac[i]].x : ac[i];
+      alt.r[1].x = ac[i] < 0 ? rt[-1 - ac[i]].y : 0;
+      B.gd[i] = (int)crn.size();
+      crn.push_back(plain);
+      crna.push_back(alt);
+    }
+    if (crn.empty()) crn.resize(1), crna.resize(1);
+    if ((rc = h->g_corner.upload(crn.data(), crn.size(), s)) || (rc = h->ga_corner.upload(crna.data(), crna.size(), s)))
+      return rc;
     if (rt.empty()) rt.push_back(make_int2(0, 0));
     if ((rc = h->ga_a.upload(aa.data(), aa.size(), s)) || (rc = h->ga_b.upload(ab.data(), ab.size(), s)) ||
         (rc = h->ga_c.upload(ac.data(), ac.size(), s)) || (rc = h->ga_rt.upload(rt.data(), rt.size(), s)))
@@ -2716,6 +2754,8 @@ void release(bsam_hier h) {
   h->norms.release();
   h->ct_rec.release();
   h->ga_rt.release();
+  h->g_corner.release();
+  h->ga_corner.release();
   h->flux_faces.release();
   for (LevelPlan &L : h->lev)
     for (TilePlan &P : L.tile) P.release();

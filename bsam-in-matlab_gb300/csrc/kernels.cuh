@@ -367,10 +367,22 @@ enum GhostType : int8_t {
   G_DIRICHLET = 5, G_NEUMANN = 6, G_RING = 7, G_PHYS_CORNER = 8
 };
 
+// A physical corner's two face rules resolved at upload, with the operand
+// slots as a kernel holds them (GhostPrep): read through the items, one
+// after the other, they kept the corner's warp 3 us behind every other.
+struct __align__(16) GhostRule {
+  int ty, a, b, c, d, e, la, lb, lc;
+  int g, nb, x;                // boundary datum, Neumann side; rule 0: the corner's interior operand, 1: its stride
+};
+struct CornerRec {
+  GhostRule r[2];
+};
+
 struct GhostItems {
   const int8_t *type;
-  const int *dst, *a, *b, *c, *d, *e;
+  const int *dst, *a, *b, *c, *d, *e;   // a corner's d: its CornerRec
   const int *inst;             // instance per item (batches only, else null)
+  const CornerRec *corner;
 };
 
 // the value of a COPY / QIF / QIF_END / LIF rule from its five operands
@@ -405,6 +417,7 @@ __device__ __forceinline__ T rule_value(int type, T qa, T qb, T qc, T qd, T qe) 
 struct GhostAlt {
   const int *a, *b, *c;        // operand slots (d and e are parent cells: never restricted)
   const int2 *rt;              // (first fine cell in Q, fine row stride)
+  const CornerRec *corner;     // with these operands
   int sh;                      // where the finer level lives (FieldsT::lsh)
 };
 
@@ -412,8 +425,17 @@ template <class T>
 struct GhostPrep {
   int8_t ty;
   int dst, a, b, c, d, e;
+  int la, lb, lc;              // GhostAlt: row stride of the four fine cells from a / b / c on, 0: a plain cell
   T g;                         // a physical rule's boundary part: 8/3 g or h g
 };
+
+__device__ __forceinline__ int ghost_cells(const GhostAlt *A, int code, int &ld) {
+  ld = 0;
+  if (code >= 0) return code;
+  const int2 r = __ldg(A->rt + (-1 - code));
+  ld = r.y;
+  return r.x + A->sh;
+}
 
 template <class T, bool kAlt = false>
 __device__ __forceinline__ GhostPrep<T> ghost_prep(const GhostItems &G, int i, int8_t ty, int dst, const T *bcg, T hx,
@@ -421,18 +443,16 @@ __device__ __forceinline__ GhostPrep<T> ghost_prep(const GhostItems &G, int i, i
   GhostPrep<T> P;
   P.ty = ty;
   P.dst = dst;
-  const int a = kAlt ? __ldg(A->a + i) : __ldg(G.a + i);
-  P.a = a;
+  P.la = P.lb = P.lc = 0;
+  const int pa = __ldg(G.a + i);
   const bool ub = ty == G_QIF || ty == G_QIF_END || ty == G_LIF || ty == G_DIRICHLET;
   const bool uc = ty == G_QIF || ty == G_QIF_END || ty == G_LIF || ty == G_LIF_CORNER;
   const bool ue = ty == G_QIF_END;
-  P.b = ub ? (kAlt ? __ldg(A->b + i) : __ldg(G.b + i)) : a;
-  P.c = uc ? (kAlt ? __ldg(A->c + i) : __ldg(G.c + i)) : a;
-  // d and e (parent cells of QIF_END) are read directly: unused, they
-  // repeat the item's plain first operand (a cell of Q in every kind that
-  // reaches ghost_value)
-  const int pa = kAlt ? __ldg(G.a + i) : a;
-  P.d = ue ? __ldg(G.d + i) : pa;
+  // slots the kind does not use repeat the item's plain first operand
+  P.a = kAlt ? ghost_cells(A, __ldg(A->a + i), P.la) : pa;
+  P.b = !ub ? pa : kAlt ? ghost_cells(A, __ldg(A->b + i), P.lb) : __ldg(G.b + i);
+  P.c = !uc ? pa : kAlt ? ghost_cells(A, __ldg(A->c + i), P.lc) : __ldg(G.c + i);
+  P.d = ue ? __ldg(G.d + i) : pa;            // parent cells: never restricted
   P.e = ue ? __ldg(G.e + i) : pa;
   P.g = T(0);
   if (ty == G_DIRICHLET) P.g = T(8.0 / 3.0) * __ldg(bcg + __ldg(G.e + i));
@@ -440,42 +460,75 @@ __device__ __forceinline__ GhostPrep<T> ghost_prep(const GhostItems &G, int i, i
   return P;
 }
 
+// a corner's face rule from its record; x: the record's last word
+template <class T, bool kAlt>
+__device__ __forceinline__ GhostPrep<T> rule_prep(const GhostRule *R, const T *bcg, T hx, T hy, int sh, int &x) {
+  const int4 *p = reinterpret_cast<const int4 *>(R);
+  const int4 u = __ldg(p), v = __ldg(p + 1), w = __ldg(p + 2);
+  GhostPrep<T> P;
+  P.ty = (int8_t)u.x;
+  P.dst = 0;
+  P.la = kAlt ? v.z : 0;
+  P.lb = kAlt ? v.w : 0;
+  P.lc = kAlt ? w.x : 0;
+  P.a = u.y + (P.la ? sh : 0);
+  P.b = u.z + (P.lb ? sh : 0);
+  P.c = u.w + (P.lc ? sh : 0);
+  P.d = v.x;
+  P.e = v.y;
+  x = w.w;
+  P.g = T(0);
+  if (P.ty == G_DIRICHLET) P.g = T(8.0 / 3.0) * __ldg(bcg + w.y);
+  else if (P.ty == G_NEUMANN) P.g = (w.z ? hy : hx) * __ldg(bcg + w.y);
+  return P;
+}
+
 // an item as a fill kernel holds it across its programmatic-launch wait: a
-// physical corner also holds its two face rules (their item and boundary
-// loads cost a corner's fill 0.5 us after the wait)
+// physical corner also holds its two face rules
 template <class T>
 struct GhostPre {
-  GhostPrep<T> P, P1, P2;
-  int pc;                      // corner: the interior operand
+  GhostPrep<T> P, P1, P2;      // corner: P.c (P.lc) is the interior operand
 };
 template <class T, bool kAlt = false>
 __device__ __forceinline__ GhostPre<T> ghost_pre(const GhostItems &G, int i, int8_t ty, int dst, const T *bcg, T hx,
                                                  T hy, const GhostAlt *A = nullptr) {
   GhostPre<T> X;
   if (ty == G_PHYS_CORNER) {
-    const int r1 = __ldg(G.a + i), r2 = __ldg(G.b + i);
+    const CornerRec *R = (kAlt ? A->corner : G.corner) + __ldg(G.d + i);
+    const int sh = kAlt ? A->sh : 0;
     X.P.ty = ty;
     X.P.dst = dst;
-    X.pc = kAlt ? __ldg(A->c + i) : __ldg(G.c + i);
-    X.P1 = ghost_prep<T, kAlt>(G, r1, __ldg(G.type + r1), 0, bcg, hx, hy, A);
-    X.P2 = ghost_prep<T, kAlt>(G, r2, __ldg(G.type + r2), 0, bcg, hx, hy, A);
+    X.P1 = rule_prep<T, kAlt>(&R->r[0], bcg, hx, hy, sh, X.P.c);
+    X.P2 = rule_prep<T, kAlt>(&R->r[1], bcg, hx, hy, sh, X.P.lc);
+    if (!kAlt) X.P.lc = 0;
+    if (X.P.lc) X.P.c += sh;
   } else {
     X.P = ghost_prep<T, kAlt>(G, i, ty, dst, bcg, hx, hy, A);
   }
   return X;
 }
 
-// a solution operand: a cell of Q, or (code < 0, fused fills only) the
-// restriction of its four fine cells
+// a solution operand's cells: one, or (fused fills only) the four whose
+// restriction it is
 template <class T, bool kCG, bool kAlt>
-__device__ __forceinline__ T ghost_operand(const T *Q, int code, const GhostAlt *A) {
-  if (kAlt && code < 0) {
-    const int2 r = __ldg(A->rt + (-1 - code));
-    const T *q = Q + r.x + A->sh;
-    return T(0.25) * (((ld_sol<kCG>(q) + ld_sol<kCG>(q + 1)) + ld_sol<kCG>(q + r.y)) + ld_sol<kCG>(q + r.y + 1));
+struct GhostCells {
+  T v[kAlt ? 4 : 1];
+  __device__ __forceinline__ void load(const T *Q, int i, int ld) {
+    v[0] = ld_sol<kCG>(Q + i);
+    if (kAlt && ld) {
+      v[kAlt ? 1 : 0] = ld_sol<kCG>(Q + i + 1);
+      v[kAlt ? 2 : 0] = ld_sol<kCG>(Q + i + ld);
+      v[kAlt ? 3 : 0] = ld_sol<kCG>(Q + i + ld + 1);
+    }
   }
-  return ld_sol<kCG>(Q + code);
-}
+  __device__ __forceinline__ T value(int ld) const {
+    if constexpr (kAlt) {
+      const T r = T(0.25) * (((v[0] + v[1]) + v[2]) + v[3]);
+      return ld ? r : v[0];
+    }
+    return v[0];
+  }
+};
 
 // a ghost's value from its operands and boundary part (every kind but the
 // ring refresh and the physical corner)
@@ -490,14 +543,48 @@ __device__ __forceinline__ T ghost_formula(int ty, T qa, T qb, T qc, T qd, T qe,
   }
 }
 
-// the value of a prepared item that is not a ring refresh or a corner
-template <class T, bool kCG, bool kAlt>
-__device__ __forceinline__ T ghost_value(const GhostPrep<T> &P, const T *Q, const GhostAlt *A) {
-  const T qa = ghost_operand<T, kCG, kAlt>(Q, P.a, A), qb = ghost_operand<T, kCG, kAlt>(Q, P.b, A);
-  const T qc = ghost_operand<T, kCG, kAlt>(Q, P.c, A);
-  const T qd = ld_sol<kCG>(Q + P.d), qe = ld_sol<kCG>(Q + P.e);
-  return ghost_formula<T>(P.ty, qa, qb, qc, qd, qe, P.g);
+// the same without a branch per kind, for the few lanes of a corner's warp
+// that hold rules of different kinds: sums of two or three products by
+// constants (by 1 where a kind has none, which is exact)
+template <class T>
+__device__ __forceinline__ T ghost_formula_flat(int ty, T qa, T qb, T qc, T qd, T qe, T g) {
+  const T A1 = T(-1.0 / 5.0), A2 = T(2.0 / 3.0), A3 = T(8.0 / 15.0);
+  const T B1 = T(5.0 / 32.0), B2 = T(15.0 / 16.0), B3 = T(-3.0 / 32.0);
+  const T c23 = T(2.0 / 3.0), c13 = T(1.0 / 3.0);
+  if (ty == G_QIF_END) qc = (B1 * qc + B2 * qd) + B3 * qe;
+  T x = qa, y = qb, z = qc, cx = A1, cy = A2, cz = A3;       // QIF, QIF_END
+  if (ty == G_LIF) { x = qc; y = qa; z = qb; cx = cy = c23; cz = -c13; }
+  else if (ty == G_LIF_CORNER) { x = qc; y = qa; cx = c23; cy = c13; }
+  else if (ty == G_DIRICHLET) { x = g; y = qa; z = qb; cx = 1; cy = -2; cz = c13; }
+  else if (ty == G_NEUMANN) { y = g; cx = cy = 1; }
+  const T two = cx * x + cy * y, three = two + cz * z;
+  return ty == G_COPY ? qa : (ty == G_LIF_CORNER || ty == G_NEUMANN) ? two : three;
 }
+
+// the operands of a prepared item that is not a ring refresh or a corner,
+// all requested before the first is used, and its value
+template <class T, bool kCG, bool kAlt>
+struct GhostVals {
+  GhostCells<T, kCG, kAlt> a, b, c;
+  T d, e;
+  __device__ __forceinline__ void load(const GhostPrep<T> &P, const T *Q) {
+    a.load(Q, P.a, P.la);
+    b.load(Q, P.b, P.lb);
+    c.load(Q, P.c, P.lc);
+    d = ld_sol<kCG>(Q + P.d);
+    e = ld_sol<kCG>(Q + P.e);
+  }
+  template <bool kFlat = false>
+  __device__ __forceinline__ T value(const GhostPrep<T> &P) const {
+    T qa = a.v[0], qb = b.v[0], qc = c.v[0];
+    if (kAlt && (P.la | P.lb | P.lc)) {      // the three restrictions side by side
+      qa = a.value(P.la);
+      qb = b.value(P.lb);
+      qc = c.value(P.lc);
+    }
+    return kFlat ? ghost_formula_flat<T>(P.ty, qa, qb, qc, d, e, P.g) : ghost_formula<T>(P.ty, qa, qb, qc, d, e, P.g);
+  }
+};
 
 // A level's own fill where the level lives at Q + sh: operands inside the
 // level's range [lo, lo + n) of Q and the ghosts move by sh, parent cells
@@ -511,9 +598,6 @@ __device__ __forceinline__ void ghost_apply_home(const GhostPre<T> &X, T *Q, T *
     if ((unsigned)(j - M.lo) < (unsigned)M.n) return Q[j + M.sh];
     return kZero && zero ? T(0) : Q[j];
   };
-  auto value = [&](const GhostPrep<T> &R) -> T {
-    return ghost_formula<T>(R.ty, op(R.a), op(R.b), op(R.c), op(R.d), op(R.e), R.g);
-  };
   if (X.P.ty == G_RING) {
     QC[X.P.dst] = Q[X.P.a];
     return;
@@ -521,21 +605,36 @@ __device__ __forceinline__ void ghost_apply_home(const GhostPre<T> &X, T *Q, T *
   // a corner: (face ghost 1 + face ghost 2) - interior, the face ghosts
   // evaluated by their own final rules (ebFillGhosts.m:84-89 reads them after
   // stage 3)
-  Q[X.P.dst + M.sh] = X.P.ty == G_PHYS_CORNER ? (value(X.P1) + value(X.P2)) - op(X.pc) : value(X.P);
+  if (X.P.ty == G_PHYS_CORNER) {
+    const GhostPrep<T> &R = X.P1, &S = X.P2;
+    const T ra = op(R.a), rb = op(R.b), rc = op(R.c), rd = op(R.d), re = op(R.e);
+    const T sa = op(S.a), sb = op(S.b), sc = op(S.c), sd = op(S.d), se = op(S.e), in = op(X.P.c);
+    Q[X.P.dst + M.sh] = (ghost_formula_flat<T>(R.ty, ra, rb, rc, rd, re, R.g) +
+                         ghost_formula_flat<T>(S.ty, sa, sb, sc, sd, se, S.g)) - in;
+    return;
+  }
+  const GhostPrep<T> &R = X.P;
+  Q[R.dst + M.sh] = ghost_formula<T>(R.ty, op(R.a), op(R.b), op(R.c), op(R.d), op(R.e), R.g);
 }
 
 template <class T, bool kCG = false, bool kAlt = false>
-__device__ __forceinline__ void ghost_apply(const GhostPre<T> &X, T *Q, T *QC, const GhostAlt *A = nullptr) {
+__device__ __forceinline__ void ghost_apply(const GhostPre<T> &X, T *Q, T *QC) {
   if (X.P.ty == G_RING) {
     QC[X.P.dst] = ld_sol<kCG>(Q + X.P.a);
     return;
   }
+  GhostVals<T, kCG, kAlt> V;
   if (X.P.ty == G_PHYS_CORNER) {
-    const T v1 = ghost_value<T, kCG, kAlt>(X.P1, Q, A), v2 = ghost_value<T, kCG, kAlt>(X.P2, Q, A);
-    Q[X.P.dst] = (v1 + v2) - ghost_operand<T, kCG, kAlt>(Q, X.pc, A);
+    GhostVals<T, kCG, kAlt> W;
+    GhostCells<T, kCG, kAlt> C;
+    V.load(X.P1, Q);
+    W.load(X.P2, Q);
+    C.load(Q, X.P.c, X.P.lc);
+    Q[X.P.dst] = (V.template value<true>(X.P1) + W.template value<true>(X.P2)) - C.value(X.P.lc);
     return;
   }
-  Q[X.P.dst] = ghost_value<T, kCG, kAlt>(X.P, Q, A);
+  V.load(X.P, Q);
+  Q[X.P.dst] = V.value(X.P);
 }
 
 // kT threads per block: kBlock, or 64 on a level whose kBlock grid leaves
@@ -1517,8 +1616,17 @@ __global__ void __launch_bounds__(kT) k_restrict(LevelD L, Decomp D, FieldsT<T> 
 // and level k-1 is first written by this very launch, so every parent-level
 // operand of level k's pre-smoothing fill is 0, which the items use instead
 // of reading cells the launch may be writing.
+//
+// Bound by latency: a launch was as long as the warp of its physical corners,
+// whose two face rules were looked up one after the other and evaluated kind
+// by kind (a ragged level's parent fill 6.2 us, every other warp done in 1.6);
+// with CornerRec, ghost_formula_flat and the operands' restrictions side by
+// side 4.2 us; FP64 levels of 1,000 to 6,000 cells 3.0-3.7 -> 2.5-3.1.  Three
+// 256-thread blocks per SM: the operands of a fused fill would take 98
+// registers and hold back the restriction's warps (batch of 64 20.3 ms, with
+// 80 registers 19.5).
 template <class T, int kT = kBlock>
-__global__ void __launch_bounds__(kT) k_restrict_fill(LevelD L, Decomp D, FieldsT<T> f, int to_parent, int nb_r,
+__global__ void __launch_bounds__(kT, kT == kBlock ? 3 : 1) k_restrict_fill(LevelD L, Decomp D, FieldsT<T> f, int to_parent, int nb_r,
                                                      GhostItems G, GhostAlt A, int g_off, int g_n, double hx_,
                                                      double hy_, const int *__restrict__ active,
                                                      const int *__restrict__ inst_nlev, int need, int f_off, int f_n,
@@ -1549,7 +1657,7 @@ __global__ void __launch_bounds__(kT) k_restrict_fill(LevelD L, Decomp D, Fields
   if (!skip) X = ghost_pre<T, true>(G, i, G.type[i], G.dst[i], f.bcg, T(hx_), T(hy_), &A);
   chain_wait();
   if (skip) return;
-  ghost_apply<T, false, true>(X, f.Q, f.QC, &A);
+  ghost_apply<T, false, true>(X, f.Q, f.QC);
 }
 // ---------------------------------------------------------------------------
 // ebFaceCorrections (ebFaceCorrections.m:18-61): the correction of one coarse
