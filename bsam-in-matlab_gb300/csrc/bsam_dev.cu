@@ -795,7 +795,9 @@ int relax_form(bsam_hier h, int k) {
 //   FP32   1,024: 1.37 / 0.86 / 0.86 / 1.03        4,096: 1.37 / 0.86 / 0.87 / 1.03
 //         11,328: 2.05 / 1.03 / 1.04 / 1.11       33,668: 2.22 / 1.30 / 1.20 / 1.20
 //        114,756: 2.22 / 2.57 / 2.05 / 1.54      379,536: 2.74 / 6.5 / 4.4 / 3.4
-// (the tuner times the form against the others on the level itself).
+// (the tuner times the form against the others on the level itself; the FP64
+// figures of 11,328 and 33,668 cells are from before a pass formed its special
+// sides together, which took 16x8 there from 1.88 / 2.40 to 1.71 / 2.22).
 void tile_size(bsam_hier h, int k, int p, int *tw, int *th) {
   const int64_t n = h->lev[k].ncells;
   *tw = *th = 0;

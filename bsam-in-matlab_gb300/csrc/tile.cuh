@@ -54,7 +54,8 @@ struct __align__(16) TileTab {
   int ent, face, nf, pad;
   int nA[kTileGroups], x0;     // x0 .. y1 (counting): the needed cells' bounds in the widest window
   int nB[kTileGroups], y0;
-  int x1, y1, pad1, pad2;
+  int fA[kTileGroups], x1;     // the special ones' TileFaces, counted in the same way
+  int fB[kTileGroups], y1;
 };
 
 // an update: window position | flags << 16 (bit 15: has a TileFace, index in
@@ -228,10 +229,11 @@ __global__ void __launch_bounds__(kTileBuildT) k_tile_build(TileBuild B) {
   const TileTab tb = B.tab[blockIdx.x];
   if (t == 0) s_base = 0;
   __syncthreads();
-  int count[4 * kTileGroups + 1], nface = 0;
+  int count[4 * kTileGroups + 1], faces[4 * kTileGroups + 1], nface = 0;
   for (int cls = 0; cls < 4 * kTileGroups; ++cls) {
     const int begin = s_base;
     count[cls] = begin;
+    faces[cls] = nface;
     const int ccol = cls < 2 * kTileGroups ? mA : 1 - mA, cg = (cls % (2 * kTileGroups)) >> 1;
     const bool csp = ((cls & 1) ^ (cg & 1)) != 0;
     for (int c0 = 0; c0 < W; c0 += kTileBuildT) {
@@ -283,6 +285,7 @@ __global__ void __launch_bounds__(kTileBuildT) k_tile_build(TileBuild B) {
               const int hi = pos == 0 ? 0 : 1, side = 2 * ax + hi;
               if (P.bc[side]) {
                 S.kind = (uint16_t)P.bc[side];
+                S.a = (uint16_t)(c + (ax == 0 ? 1 : td.wx) * (hi ? -1 : 1));   // the neighbour across the cell
                 S.c = P.bcg_off + (ax == 0 ? hi * P.my + lj : 2 * P.my + hi * P.mx + li);
               } else {
                 const Rule &R = rule_of(P, side, li, lj);
@@ -311,6 +314,7 @@ __global__ void __launch_bounds__(kTileBuildT) k_tile_build(TileBuild B) {
     if (csp) nface += s_base - begin;
   }
   count[4 * kTileGroups] = s_base;
+  faces[4 * kTileGroups] = nface;
   if (t == 0) {
     if (nface > kTileFaces) s_bad = 1;
     if (s_bad) *B.bad = 1;
@@ -320,6 +324,8 @@ __global__ void __launch_bounds__(kTileBuildT) k_tile_build(TileBuild B) {
       for (int g = 0; g < kTileGroups; ++g) {
         o.nA[g] = count[2 * g + 2];
         o.nB[g] = count[2 * kTileGroups + 2 * g + 2] - count[2 * kTileGroups];
+        o.fA[g] = faces[2 * g + 2];
+        o.fB[g] = faces[2 * kTileGroups + 2 * g + 2] - faces[2 * kTileGroups];
       }
       o.x0 = s_lo[0];
       o.x1 = s_hi[0];
@@ -372,7 +378,7 @@ __global__ void __launch_bounds__(kTileT, sizeof(T) == 4 ? 5 : 1)
   }
   T *win = reinterpret_cast<T *>(tile_raw);
   T *op = win + win_cap;                      // rows dE dW dN dS InvDiagS F
-  T *fst = op + 6 * cap;                      // special sides: constant part, stored ghost
+  T *fst = op + 6 * cap;                      // special sides: constant part, ghost
   uint32_t *code = reinterpret_cast<uint32_t *>(fst + 4 * nf_cap);
   int *wqs = reinterpret_cast<int *>(code + cap);
   uint32_t *fk = reinterpret_cast<uint32_t *>(wqs + win_cap);
@@ -423,18 +429,28 @@ __global__ void __launch_bounds__(kTileT, sizeof(T) == 4 ? 5 : 1)
       else v = c23 * qc;
     }
     fst[i] = v;
+    if (k == 2) fst[2 * nf_cap + i] = v;
   }
   cp_async_wait();
   __syncthreads();
-  // an update; `first`: coarse-fine sides take the stored ghost
-  auto update = [&](int e, bool first) {
+  // the ghost of special side i, which is neither a Neumann side (constant)
+  // nor takes the stored ghost
+  auto side = [&](int i) -> T {
+    const uint32_t ka = fk[2 * i];
+    const int k = ka & 0x7f;
+    const T s = fst[i], qa = win[ka >> 16];
+    if (k == 1) return s + c13 * qa;
+    const T qb = win[fk[2 * i + 1]];
+    return k == 8 + G_LIF ? (s + c23 * qa) - c13 * qb : (A1 * qa + A2 * qb) + s;
+  };
+  // an update
+  auto update = [&](int e) {
     const uint32_t sf = code[e];
     const int c = sf & 0xffff;
     T qe = win[c + 1], qw = win[c - 1], qn = win[c + wx], qs = win[c - wx];
     T v = op[kPackRows * cap + e];
     if (sf & kTileSpecial) {
       const int fi = (sf >> 16) & (kTileFaces - 1);
-      const T we = qe, ww = qw, wn = qn, ws = qs;
 #pragma unroll
       for (int ax = 0; ax < 2; ++ax) {
         const int i = 2 * fi + ax;
@@ -442,17 +458,7 @@ __global__ void __launch_bounds__(kTileT, sizeof(T) == 4 ? 5 : 1)
         const int k = ka & 0x7f;
         if (k == 0) continue;
         const bool lo = (ka & 0x80) != 0;
-        const T s = fst[i];
-        T g;
-        // a partial Dirichlet ghost reads the neighbour across the cell
-        if (k == 1) g = s + c13 * (ax == 0 ? (lo ? we : ww) : (lo ? wn : ws));
-        else if (k == 2) g = s;
-        else if (first) g = fst[2 * nf_cap + i];
-        else {
-          const T qa = win[ka >> 16], qb = win[fk[2 * i + 1]];
-          if (k == 8 + G_LIF) g = (s + c23 * qa) - c13 * qb;
-          else g = (A1 * qa + A2 * qb) + s;
-        }
+        const T g = fst[2 * nf_cap + i];
         if (ax == 0) { if (lo) qw = g; else qe = g; }
         else { if (lo) qs = g; else qn = g; }
       }
@@ -479,7 +485,20 @@ __global__ void __launch_bounds__(kTileT, sizeof(T) == 4 ? 5 : 1)
     const int e0 = a ? 0 : nA;
     const int e1 = e0 + (g == 0 ? (a ? tb.nA[0] : tb.nB[0]) : g == 1 ? (a ? tb.nA[1] : tb.nB[1]) : (a ? tb.nA[2] : tb.nB[2]));
     const bool first = stored && p == kTilePasses - passes + 1;
-    for (int e = e0 + t; e < e1; e += kTileT) update(e, first);
+    // the pass's special sides first, by the block's first threads together:
+    // in the updates both axes' rules stood one after the other in front of
+    // the chain of every warp with a special cell (5,200 to 5,800 cells in
+    // patches 1.88 us a pass -> 1.54, 33,668 cells 2.40 -> 2.22; FP32 the same)
+    const int f0 = a ? 0 : tb.fA[kTileGroups - 1];
+    const int f1 = f0 + (g == 0 ? (a ? tb.fA[0] : tb.fB[0]) : g == 1 ? (a ? tb.fA[1] : tb.fB[1]) : (a ? tb.fA[2] : tb.fB[2]));
+    if (f1 > f0) {
+      for (int i = 2 * f0 + t; i < 2 * f1; i += kTileT) {
+        const int k = fk[2 * i] & 0x7f;
+        if (k != 0 && k != 2 && !(first && k != 1)) fst[2 * nf_cap + i] = side(i);
+      }
+      __syncthreads();
+    }
+    for (int e = e0 + t; e < e1; e += kTileT) update(e);
     __syncthreads();
   }
   for (int i = t; i < td.w * td.h; i += kTileT) {
