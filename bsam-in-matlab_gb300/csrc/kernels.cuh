@@ -2257,9 +2257,12 @@ __device__ __forceinline__ double pmax(double a, double b) {
 constexpr int kResRowsMax = 4;
 
 // kT threads per block (kBlock, or 64 where the kBlock grid would leave
-// SMs with unequal shares of the FP64 work)
+// SMs with unequal shares of the FP64 work; 14 of those per SM, with 72
+// registers: with the 80 to 96 it takes by itself the starfish's 13.9 blocks
+// per SM ran in two rounds, the second half empty, 16.5 us; 12 or 16 per SM no
+// faster, solve 2.99 -> 2.96 ms, 1024^2 24.8 -> 24.7 for 60 V-cycles)
 template <bool kL2, bool kPow2, bool kInt, int kT = kBlock, int kResRows = kResRowsMax>
-__global__ void __launch_bounds__(kT) k_residual(const LevelX *__restrict__ X, const PatchD *__restrict__ patches,
+__global__ void __launch_bounds__(kT, kT == 64 && kResRows == kResRowsMax ? 14 : 1) k_residual(const LevelX *__restrict__ X, const PatchD *__restrict__ patches,
                                                  const ResTask *__restrict__ tasks, int ntask, Fields f, double *slots,
                                                  int nslots, unsigned long long *norms, int want_fn, int mass_corr,
                                                  float *__restrict__ rout) {
