@@ -2783,6 +2783,31 @@ int set_device(bsam_hier h) {
 }  // namespace
 
 // ===========================================================================
+// the two sums of k_sums per level from the root up, each the sum of its
+// blocks' partials in order
+template <bool kMass>
+static int level_sums(bsam_hier h, std::vector<double> &part, std::vector<int> &starts) {
+  int o = 0;
+  for (int k = h->root; k <= h->nlev;) {
+    SumSpans S{};
+    const int o0 = o;
+    for (; k <= h->nlev && S.n < kMaxSums; ++k, ++S.n) {
+      const LevelPlan &L = h->lev[k];
+      starts.push_back(o);
+      S.b0[S.n] = o - o0;
+      S.patches[S.n] = h->patches.p + L.p0;
+      S.D[S.n] = decomp(h, L.cell);
+      o += L.cell.nblocks;
+    }
+    S.b0[S.n] = o - o0;
+    if (o > o0) k_sums<kMass><<<(unsigned)(o - o0), kBlock, 0, h->stream>>>(S, fields(h), h->partials.p + 2 * o0);
+  }
+  CK(cudaGetLastError());
+  part.resize((size_t)2 * o);
+  CK(cudaMemcpyAsync(part.data(), h->partials.p, sizeof(double) * part.size(), cudaMemcpyDeviceToHost, h->stream));
+  return BSAM_OK;
+}
+
 extern "C" {
 
 const char *bsam_last_error(void) { return g_err.c_str(); }
@@ -3162,7 +3187,13 @@ int bsam_tag_level(bsam_hier h, int level, int indicator, double threshold, int 
       Decomp D = decomp(h, L.coarse);
       k_tag_rte<<<D.nblocks, kBlock, 0, h->stream>>>(leveld(h, level), D, fields(h), threshold, T, cover, n1);
     }
-    k_tag_buffer<<<(unsigned)((n + kBlock - 1) / kBlock), kBlock, 0, h->stream>>>(T, cover, out, n0, n1, buffer);
+    if (n1 % 4 == 0 && buffer <= 4) {        // (then every row starts on a word)
+      const int w = n1 / 4;
+      k_tag_buffer4<<<(unsigned)((n / 4 + kBlock - 1) / kBlock), kBlock, 0, h->stream>>>(
+          (const uint32_t *)T, (const uint32_t *)cover, (uint32_t *)out, n0, w, buffer);
+    } else {
+      k_tag_buffer<<<(unsigned)((n + kBlock - 1) / kBlock), kBlock, 0, h->stream>>>(T, cover, out, n0, n1, buffer);
+    }
     h->launch_count += 2;
     e = cudaGetLastError();
   }
@@ -3285,24 +3316,12 @@ int bsam_batch_set_stop(bsam_hier h, int inst, int max_vcycles, double rel_tol) 
 }
 
 int bsam_composite_mean(bsam_hier h, double *mean, double *area) {
-  double out[4];
-  (void)out;
   if (!h) return fail(BSAM_ERR_ARG, "null hierarchy");
   int rc = set_device(h);
   if (rc) return rc;
-  Fields f = fields(h);
-  int o = 0;
   std::vector<int> starts;
-  for (int k = h->root; k <= h->nlev; ++k) {
-    const LevelPlan &L = h->lev[k];
-    Decomp D = decomp(h, L.cell);
-    starts.push_back(o);
-    k_sums<<<D.nblocks, kBlock, 0, h->stream>>>(leveld(h, k), D, f, h->partials.p + 4 * o);
-    o += D.nblocks;
-  }
-  CK(cudaGetLastError());
-  std::vector<double> part((size_t)4 * o);
-  CK(cudaMemcpyAsync(part.data(), h->partials.p, sizeof(double) * part.size(), cudaMemcpyDeviceToHost, h->stream));
+  std::vector<double> part;
+  if ((rc = level_sums<false>(h, part, starts))) return rc;
   CK(cudaStreamSynchronize(h->stream));
   double tot = 0, ar = 0;
   int li = 0;
@@ -3311,8 +3330,8 @@ int bsam_composite_mean(bsam_hier h, double *mean, double *area) {
     const double da = L.hx * L.hy;
     double su = 0, nv = 0;
     for (int b = starts[li]; b < starts[li] + L.cell.nblocks; ++b) {
-      su = su + part[4 * b];
-      nv = nv + part[4 * b + 3];
+      su = su + part[2 * b];
+      nv = nv + part[2 * b + 1];
     }
     tot = tot + su * da;
     ar = ar + nv * da;
@@ -3366,19 +3385,9 @@ int bsam_mass_check(bsam_hier h, double out[4]) {
   if (!h || !out) return fail(BSAM_ERR_ARG, "null argument");
   int rc = set_device(h);
   if (rc) return rc;
-  Fields f = fields(h);
-  int o = 0;
   std::vector<int> starts;
-  for (int k = h->root; k <= h->nlev; ++k) {
-    const LevelPlan &L = h->lev[k];
-    Decomp D = decomp(h, L.cell);
-    starts.push_back(o);
-    k_sums<<<D.nblocks, kBlock, 0, h->stream>>>(leveld(h, k), D, f, h->partials.p + 4 * o);
-    o += D.nblocks;
-  }
-  CK(cudaGetLastError());
-  std::vector<double> part((size_t)4 * o);
-  CK(cudaMemcpyAsync(part.data(), h->partials.p, sizeof(double) * part.size(), cudaMemcpyDeviceToHost, h->stream));
+  std::vector<double> part;
+  if ((rc = level_sums<true>(h, part, starts))) return rc;
   // boundary flux: the terms of the uncovered physical faces on the device,
   // summed here side by side in the reference's loop order
   if ((rc = ensure_flux_faces(h))) return rc;
@@ -3399,8 +3408,8 @@ int bsam_mass_check(bsam_hier h, double out[4]) {
     const double da = L.hx * L.hy;
     double sm = 0, sa = 0;
     for (int b = starts[li]; b < starts[li] + L.cell.nblocks; ++b) {
-      sm = sm + part[4 * b + 1];
-      sa = sa + part[4 * b + 2];
+      sm = sm + part[2 * b];
+      sa = sa + part[2 * b + 1];
     }
     lhs = lhs + sm * da;
     scale = scale + sa * da;

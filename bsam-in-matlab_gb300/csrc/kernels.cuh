@@ -2482,7 +2482,7 @@ __global__ void __launch_bounds__(kStep) k_solve_step(const InstRes *__restrict_
 // A residual report of every instance (one block per instance): max-norms
 // over its slots, L2 per level from that level's slots in a fixed tree order
 // weighted by the cell area, rel = linf / max(fnorm, realmin).
-constexpr int kFinal = 512;
+constexpr int kFinal = 512, kFinalRanges = 8;
 __global__ void __launch_bounds__(kFinal) k_residual_final(const InstRes *__restrict__ ir,
                                                           const SlotRange *__restrict__ ranges, const double *slots,
                                                           int nslots, ResAcc *acc) {
@@ -2490,22 +2490,38 @@ __global__ void __launch_bounds__(kFinal) k_residual_final(const InstRes *__rest
   const int inst = blockIdx.x, t = threadIdx.x;
   const InstRes R = ir[inst];
   double li = 0, fn = 0, l2sq = 0;
-  __shared__ double s_p[kFinal], s_a[kFinal], s_b[kFinal];
-  for (int r = R.range0; r < R.range1; ++r) {
-    const int s0 = ranges[r].s0, s1 = ranges[r].s1;
-    double p = 0;
-    for (int i = s0 + t; i < s1; i += kFinal) {
-      p = p + slots[nslots + i];
-      li = pmax(li, slots[i]);
-      fn = pmax(fn, slots[2 * nslots + i]);
+  // up to kFinalRanges levels' trees side by side, the last five steps of
+  // each in a warp of its own (a report of a starfish 73 us through the call
+  // with one level after the other, 65 side by side)
+  __shared__ double s_p[kFinalRanges][kFinal], s_a[kFinal], s_b[kFinal], s_l2[kFinalRanges];
+  for (int r0 = R.range0; r0 < R.range1; r0 += kFinalRanges) {
+    const int nr = min(kFinalRanges, R.range1 - r0);
+    for (int r = 0; r < nr; ++r) {
+      const int s0 = ranges[r0 + r].s0, s1 = ranges[r0 + r].s1;
+      double p = 0;
+      for (int i = s0 + t; i < s1; i += kFinal) {
+        p = p + slots[nslots + i];
+        li = pmax(li, slots[i]);
+        fn = pmax(fn, slots[2 * nslots + i]);
+      }
+      s_p[r][t] = p;
     }
-    s_p[t] = p;
     __syncthreads();
-    for (int off = kFinal / 2; off >= 1; off >>= 1) {
-      if (t < off) s_p[t] = s_p[t] + s_p[t + off];
+    for (int off = kFinal / 2; off >= 32; off >>= 1) {
+      for (int i = t; i < nr * off; i += kFinal) {
+        double *q = s_p[i / off] + (i & (off - 1));
+        q[0] = q[0] + q[off];
+      }
       __syncthreads();
     }
-    l2sq = l2sq + s_p[0] * ranges[r].area;
+    for (int r = t >> 5; r < nr; r += kFinal / 32) {
+      double p = s_p[r][t & 31];
+#pragma unroll
+      for (int off = 16; off >= 1; off >>= 1) p = p + __shfl_down_sync(0xffffffffu, p, off);
+      if ((t & 31) == 0) s_l2[r] = p;
+    }
+    __syncthreads();
+    for (int r = 0; r < nr; ++r) l2sq = l2sq + s_l2[r] * ranges[r0 + r].area;
     __syncthreads();
   }
   s_a[t] = li;
@@ -2819,6 +2835,41 @@ __global__ void __launch_bounds__(kBlock) k_tag_buffer(const uint8_t *__restrict
   out[g] = (t && a) ? 1 : 0;
 }
 
+// the same for four cells of a row per thread, as bytes of a word: n1 a
+// multiple of four and b at most four.  The rows' words are combined first
+// (or of the tags, and of the cover), then the bytes beside a cell: 9 words
+// per row and a few shifts instead of 34 bytes per cell (b = 2); the tags of
+// 1024 x 1024 cells 156 us through the call -> 131
+__global__ void __launch_bounds__(kBlock) k_tag_buffer4(const uint32_t *__restrict__ T, const uint32_t *__restrict__ cover,
+                                                        uint32_t *out, int n0, int w, int b) {
+  const long long g = (long long)blockIdx.x * kBlock + threadIdx.x;
+  if (g >= (long long)n0 * w) return;
+  const int i = (int)(g / w), j = (int)(g - (long long)i * w);
+  // tags and covers hold 0 or 1 per byte; outside: untagged, covered
+  uint32_t tl = 0, tc = 0, tr = 0, al = 0x01010101u, ac = 0x01010101u, ar = 0x01010101u;
+  for (int ii = max(i - b, 0); ii <= min(i + b, n0 - 1); ++ii) {
+    const uint32_t *r = T + (size_t)ii * w + j;
+    tc |= r[0];
+    if (j > 0) tl |= r[-1];
+    if (j + 1 < w) tr |= r[1];
+  }
+#pragma unroll
+  for (int d = -1; d <= 1; ++d) {
+    const int ii = i + d;
+    if (ii < 0 || ii >= n0) continue;
+    const uint32_t *r = cover + (size_t)ii * w + j;
+    ac &= r[0];
+    if (j > 0) al &= r[-1];
+    if (j + 1 < w) ar &= r[1];
+  }
+  uint32_t t = tc;
+#pragma unroll
+  for (int d = 1; d <= 4; ++d)               // the byte d to the right, d to the left
+    if (d <= b) t |= __funnelshift_rc(tc, tr, 8 * d) | __funnelshift_lc(tl, tc, 8 * d);
+  const uint32_t a = ac & __funnelshift_r(ac, ar, 8) & __funnelshift_l(al, ac, 8);
+  out[g] = t & a;
+}
+
 // FP32 copy of an FP64 array (coefficient copies of the mixed form)
 __global__ void __launch_bounds__(kBlock) k_to_f32(const double *__restrict__ a, float *__restrict__ b, long long n) {
   chain_wait_static();
@@ -2827,36 +2878,55 @@ __global__ void __launch_bounds__(kBlock) k_to_f32(const double *__restrict__ a,
 }
 
 // ---------------------------------------------------------------------------
-// Composite sums over visible cells (ebCompositeMean.m, ebMassCheck.m lhs):
-// per-block partials of sum(u), sum(C u - FTrue), sum(|FTrue|)
-__global__ void __launch_bounds__(kBlock) k_sums(LevelD L, Decomp D, Fields f, double *partials) {
-  chain_wait();
-  const int g = blockIdx.x * kBlock + threadIdx.x;
-  double su = 0, sm = 0, sa = 0, nv = 0;
+// Composite sums over visible cells, per-block partials of two quantities:
+// sum(u) and the number of cells (ebCompositeMean.m), or sum(C u - FTrue) and
+// sum(|FTrue|) (ebMassCheck.m lhs).  Several levels in one launch, the blocks
+// of each as a launch of its own would have them; a launch per level, each
+// with all four sums, made the mean of a starfish 62 us through the call and its
+// mass check 77, one launch of two sums 30 and 47.
+constexpr int kMaxSums = 16;
+struct SumSpans {
+  int n, b0[kMaxSums + 1];     // first block per level
+  const PatchD *patches[kMaxSums];
+  Decomp D[kMaxSums];
+};
+template <bool kMass>
+__global__ void __launch_bounds__(kBlock) k_sums(const __grid_constant__ SumSpans S, Fields f, double *partials) {
+  int l = 0;
+  while ((int)blockIdx.x >= S.b0[l + 1]) ++l;
+  const Decomp &D = S.D[l];
+  const int b = blockIdx.x - S.b0[l], g = b * kBlock + threadIdx.x, t = threadIdx.x;
+  double x = 0, y = 0;
   if (g < D.n) {
-    const int p = find_patch(D, blockIdx.x, g);
-    const PatchD &P = L.patches[p];
+    const int p = find_patch(D, b, g);
+    const PatchD &P = S.patches[l][p];
     const int s = g - __ldg(D.beg + p);
     const int lj = s / P.mx, lx = s - lj * P.mx;
     const int cc = P.c_off + s;
     if (!(f.flags[cc] & 1)) {
       const double u = f.Q[P.q_off + (lx + 1) + (lj + 1) * (P.mx + 2)];
-      su = u;
-      sm = f.CC[cc] * u - f.FTrue[cc];
-      sa = fabs(f.FTrue[cc]);
-      nv = 1;
+      x = kMass ? f.CC[cc] * u - f.FTrue[cc] : u;
+      y = kMass ? fabs(f.FTrue[cc]) : 1.0;
     }
   }
-  __shared__ double sh[4][kBlock];
-  sh[0][threadIdx.x] = su; sh[1][threadIdx.x] = sm; sh[2][threadIdx.x] = sa; sh[3][threadIdx.x] = nv;
+  // halving tree: thread t < off adds thread t + off
+  __shared__ double sh[2][kBlock];
+  sh[0][t] = x;
+  sh[1][t] = y;
   __syncthreads();
-  for (int off = kBlock / 2; off >= 1; off >>= 1) {
-    if (threadIdx.x < off)
-      for (int q = 0; q < 4; ++q) sh[q][threadIdx.x] = sh[q][threadIdx.x] + sh[q][threadIdx.x + off];
+#pragma unroll
+  for (int off = kBlock / 2; off >= 32; off >>= 1) {
+    if (t < 2 * off) {         // the second sum's threads follow the first's
+      double *r = sh[t / off];
+      r[t & (off - 1)] = r[t & (off - 1)] + r[(t & (off - 1)) + off];
+    }
     __syncthreads();
   }
-  if (threadIdx.x == 0)
-    for (int q = 0; q < 4; ++q) partials[4 * blockIdx.x + q] = sh[q][0];
+  if (t >= 64) return;
+  double v = sh[t >> 5][t & 31];
+#pragma unroll
+  for (int off = 16; off >= 1; off >>= 1) v = v + __shfl_down_sync(0xffffffffu, v, off);
+  if ((t & 31) == 0) partials[2 * blockIdx.x + (t >> 5)] = v;
 }
 
 // Boundary flux terms of the mass balance (ebMassCheck.m:30-60), one per
