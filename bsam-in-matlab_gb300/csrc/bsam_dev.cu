@@ -1419,8 +1419,8 @@ int launch_iteration(bsam_hier h, int mode, const LoopCond &cond = LoopCond()) {
 // of kTuneMinCells or more fills the device with one launch per colour pass
 // and one cell per thread (2 or 4 cells, or persistent blocks, measured no
 // faster in either precision and are only forced); a smaller level times one
-// launch per colour pass, the tile form (kn 6) and, where its Q range fits,
-// the shared-memory cluster launch (kn 5).  Each candidate's relaxation (npre
+// launch per colour pass against the tile form (kn 6) or, where its tables
+// cannot be had and the Q range fits, the shared-memory cluster launch (kn 5).  Each candidate's relaxation (npre
 // sweeps and the closing fill) is timed best of three with CUDA events on the
 // stream, in the precision the cycle runs in; the fastest is kept.  The
 // choice does not change a single bit of the result (each update's arithmetic

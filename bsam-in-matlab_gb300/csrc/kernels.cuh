@@ -1943,8 +1943,8 @@ __device__ __forceinline__ void load_corr_item(const LevelD &L, const LevelD &Lc
 }
 
 // kT threads per block (kBlock, or 64 on a level whose kBlock grid leaves
-// SMs idle: a footprint cell is ~84 FP64 operations, and an SM issues about
-// two per clock); the decomposition's per-block patch table is kBlock-based
+// SMs idle: a footprint cell is 45 to 85 FP64 operations, and an SM issues
+// about two per clock); the decomposition's per-block patch table is kBlock-based
 template <class T, bool kPow2, bool kInt, int kT = kBlock, bool kQuad = false>
 __global__ void __launch_bounds__(kT) k_load(LevelD L, LevelD Lc, Decomp D, FieldsT<T> f, const int *__restrict__ ring,
                                              const int *__restrict__ ring_inst, int ring_off, int n_ring, CorrCSR C,
@@ -2226,7 +2226,7 @@ __global__ void __launch_bounds__(32 * kBWarps, 7) k_coarsest_batch(const double
 //
 // Bound by the FP64 pipe and latency: about 13 operations per cell (19 with
 // every flux formed twice, the scaling by 1/h^2 on the FP64 pipe and the
-// squares): starfish 34 us -> 18 us per iteration, its floor at the
+// squares): starfish 34 us -> 16 us per iteration, its floor at the
 // measured FP64 rate 10 us.
 struct ResAcc {
   double out[5];        // linf, l2, fnorm, rel, ncell
