@@ -2360,8 +2360,7 @@ __global__ void __launch_bounds__(kT, kT == 64 && kResRows == kResRowsMax ? 14 :
       Y = corr_target<double>(Xf.C, g, f);
     }
     chain_wait();
-    if (!mass_corr) return;
-    if (on) {
+    if (on) {                // corrections off: kind 0 took these cells, and zeros go to the task's slot
       const double *Q = f.Q + c;
       double r = ft - op_pre<kPow2>(Q[0], Q[1], Q[-1], Q[ldq], Q[-ldq], dE, dW, dN, dS, cf, Xk.L);
       r = add_corrections<kPow2>(r, Y, Xf.C, Xk.L, f, true);
