@@ -98,7 +98,8 @@ __global__ void __launch_bounds__(kThreads) k_segdist(const double *__restrict__
                                                       const double *__restrict__ x, const double *__restrict__ y,
                                                       double *__restrict__ best, int64_t n) {
   const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
-  const bool on = i < n;
+  // a NaN start stays: no distance compares below it
+  const bool on = i < n && !isnan(best[i]);
   const double px = on ? x[i] : 0.0, py = on ? y[i] : 0.0;
   double b = on ? best[i] : 0.0;
   const double M = fmax(scale, fmax(fabs(px), fabs(py)));
