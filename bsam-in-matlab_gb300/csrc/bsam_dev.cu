@@ -40,7 +40,10 @@ int fail(int code, const std::string &msg) {
   return code;
 }
 
+// (takes a failed call's error off the runtime as well: left there, the next
+// call that asks for launch errors would report it as its own)
 int cuda_fail(cudaError_t e, const char *what) {
+  cudaGetLastError();
   return fail(e == cudaErrorMemoryAllocation ? BSAM_ERR_NOMEM : BSAM_ERR_CUDA,
               std::string(what) + ": " + cudaGetErrorString(e));
 }
@@ -3349,6 +3352,7 @@ static int ensure_flux_faces(bsam_hier h) {
   CK(cudaMemcpyAsync(fl.data(), h->flags.p, fl.size(), cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
   std::vector<FluxFace> faces;
+  std::vector<FluxSide> sides;
   for (int k = h->root; k <= h->nlev; ++k) {
     const LevelPlan &L = h->lev[k];
     for (int p = L.p0; p < L.p1; ++p) {
@@ -3369,14 +3373,19 @@ static int ensure_flux_faces(bsam_hier h) {
           faces.push_back(f);
         }
         S.end = (int)faces.size();
-        h->flux_sides.push_back(S);
+        sides.push_back(S);
       }
     }
   }
   int rc;
-  if ((rc = h->flux_faces.upload(faces.data(), faces.size(), h->stream)) || (rc = h->flux_term.alloc(faces.size())))
+  if ((rc = h->flux_faces.upload(faces.data(), faces.size(), h->stream)) || (rc = h->flux_term.alloc(faces.size()))) {
+    cudaStreamSynchronize(h->stream);        // the faces' host copy goes
+    h->flux_faces.release();
+    h->flux_term.release();
     return rc;
+  }
   CK(cudaStreamSynchronize(h->stream));
+  h->flux_sides.swap(sides);
   h->flux_ready = true;
   return BSAM_OK;
 }
