@@ -814,23 +814,32 @@ void tile_size(bsam_hier h, int k, int p, int *tw, int *th) {
   }
 }
 
-// the levels' tiles, built on first use; usable or not in their state
+// the levels' tiles, built on first use; usable or not in their state.  A
+// level whose tables find no memory runs without them.
 int ensure_tiles(bsam_hier h, const std::vector<int> &levels, int p) {
   std::vector<TileCount> C(levels.size());
   int rc = BSAM_OK;
   bool any = false;
+  auto refused = [&](size_t i) {
+    TilePlan &P = h->lev[levels[i]].tile[p];
+    P.release();
+    P.state = -1;
+    C[i].k = 0;
+    rc = BSAM_OK;
+  };
   for (size_t i = 0; i < levels.size() && !rc; ++i) {
     const int k = levels[i];
     if (h->lev[k].tile[p].state) continue;
     int tw, th;
     tile_size(h, k, p, &tw, &th);
-    rc = begin_tiles(h, k, p, tw, th, C[i]);
+    if ((rc = begin_tiles(h, k, p, tw, th, C[i])) == BSAM_ERR_NOMEM) refused(i);
     any = true;
   }
   // the counts are on the host; later, the tables' host copies may go
   if (any) {
     if (cudaStreamSynchronize(h->stream) != cudaSuccess && !rc) rc = cuda_fail(cudaGetLastError(), "tile tables");
-    for (size_t i = 0; i < levels.size() && !rc; ++i) rc = end_tiles(h, p, C[i]);
+    for (size_t i = 0; i < levels.size() && !rc; ++i)
+      if ((rc = end_tiles(h, p, C[i])) == BSAM_ERR_NOMEM) refused(i);
     if (cudaStreamSynchronize(h->stream) != cudaSuccess && !rc) rc = cuda_fail(cudaGetLastError(), "tile tables");
   }
   for (TileCount &c : C) {
@@ -841,13 +850,13 @@ int ensure_tiles(bsam_hier h, const std::vector<int> &levels, int p) {
 }
 
 // does level k's V-cycle run its relaxations in the tile form: chosen for the
-// level (6), with a relaxation on either side (the first moves the level to
+// level (6), its tables there, with a relaxation on either side (the first moves the level to
 // its second copy, the second back), and with the stored copies of the
 // siblings' cells in step with them when the first starts
 template <class T>
 bool tile_cycle(bsam_hier h, int k) {
-  return relax_form<T>(h, k) == 6 && h->opts.npre > 0 && h->opts.npost > 0 &&
-         (sizeof(T) == sizeof(float) || h->copies_synced);
+  return relax_form<T>(h, k) == 6 && h->lev[k].tile[sizeof(T) == sizeof(float) ? 1 : 0].state == 1 &&
+         h->opts.npre > 0 && h->opts.npost > 0 && (sizeof(T) == sizeof(float) || h->copies_synced);
 }
 
 // where level k lives between its two relaxations (FieldsT::lsh)
