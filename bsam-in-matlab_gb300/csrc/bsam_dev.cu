@@ -621,7 +621,6 @@ void launch_dsm(bsam_hier h, int ctas, size_t smem, Args... args) {
   cudaLaunchKernelEx(&cfg, k_relax_dsm<T, kPow2>, args...);
 }
 
-constexpr int kTileMaxBytes = 200 * 1024;
 constexpr int64_t kTuneMinCells = 131072;   // large levels: the forms that fill the device
 
 // k_relax_tile's variants may use up to kTileMaxBytes of shared memory
@@ -877,14 +876,8 @@ void launch_relax_tiles(bsam_hier h, int k, int nsweeps, bool first_fresh, bool 
   const int nl = ((nsweeps + kTileGroups - 1) / kTileGroups) | 1;
   const int unit = h->opts.omega == 1.0 ? 1 : 0;
   const T om = (T)h->opts.omega;
-  // FP64: a block's passes share its SM's pipe with any other block there, so
-  // the blocks of a grid that covers a good part of the SMs ask for as much
-  // shared memory as spreads them evenly (starfish -1.4%; a handful of blocks
-  // only pays for the larger request: a 1,024-cell solve +2%)
   size_t smem = tile_smem<T>(P.win_cap, P.cap, P.nf_cap);
-  const int per_sm = (P.ntiles + sm_count() - 1) / sm_count();
-  if (sizeof(T) == sizeof(double) && 4 * P.ntiles >= sm_count())
-    smem = std::max(smem, (size_t)std::min(kTileMaxBytes, 224 * 1024 / per_sm - 2048));
+  if (sizeof(T) == sizeof(double)) smem = tile_request(smem, P.ntiles, sm_count());
   T *a = f.Q, *b = f.Q + h->n_q;
   if (back) std::swap(a, b);
   for (int l = 0, done = 0; l < nl; ++l, std::swap(a, b)) {

@@ -3,6 +3,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <map>
 #include <mutex>
@@ -27,3 +28,18 @@ struct bsam_ctx_s {
 
 // records the message of a failed call for bsam_last_error(); returns code
 int bsam_internal_set_error(int code, const std::string &msg);
+
+// most dynamic shared memory of a k_relax_tile block
+constexpr int kTileMaxBytes = 200 * 1024;
+
+// what a block of an FP64 tile launch asks for, `need` at least: a block's
+// passes share its SM's FP64 pipe with any other block there, so the blocks of
+// a grid that covers a good part of the SMs ask for as much as spreads them
+// evenly (starfish -1.4%; a handful of blocks only pays for the larger request:
+// a 1,024-cell solve +2%).  With more blocks per SM than have a share, need.
+inline size_t tile_request(size_t need, int ntiles, int sms) {
+  if (4 * (int64_t)ntiles < sms) return need;
+  const int per_sm = (ntiles + sms - 1) / sms;
+  const int share = std::min(kTileMaxBytes, 224 * 1024 / per_sm - 2048);
+  return share > 0 ? std::max(need, (size_t)share) : need;
+}
