@@ -257,6 +257,7 @@ struct bsam_hier_s {
   // picked by the autotuner at the first solve (result-neutral)
   std::vector<int> relax_n[2];
   bool tuned[2] = {false, false};
+  bool retune[2] = {false, false};   // chosen while the tile form was (not) to be had, which the options changed
   DBuf<double> saveQ, saveQC, saveF;
   // bsam_mass_check: its boundary faces (structure only) and their terms
   bool flux_ready = false;
@@ -848,6 +849,17 @@ int ensure_tiles(bsam_hier h, const std::vector<int> &levels, int p) {
   return rc;
 }
 
+// marks launches of the solve's own flow (copies_synced)
+struct Synced {
+  bsam_hier h;
+  bool was;
+  explicit Synced(bsam_hier h_) : h(h_), was(h_->copies_synced) { h->copies_synced = true; }
+  ~Synced() { h->copies_synced = was; }
+};
+
+// a relaxation on either side, for the tile form's way out and back
+bool tiles_apply(const bsam_solve_opts &o) { return o.npre > 0 && o.npost > 0; }
+
 // does level k's V-cycle run its relaxations in the tile form: chosen for the
 // level (6), its tables there, with a relaxation on either side (the first moves the level to
 // its second copy, the second back), and with the stored copies of the
@@ -855,7 +867,7 @@ int ensure_tiles(bsam_hier h, const std::vector<int> &levels, int p) {
 template <class T>
 bool tile_cycle(bsam_hier h, int k) {
   return relax_form<T>(h, k) == 6 && h->lev[k].tile[sizeof(T) == sizeof(float) ? 1 : 0].state == 1 &&
-         h->opts.npre > 0 && h->opts.npost > 0 && (sizeof(T) == sizeof(float) || h->copies_synced);
+         tiles_apply(h->opts) && (sizeof(T) == sizeof(float) || h->copies_synced);
 }
 
 // where level k lives between its two relaxations (FieldsT::lsh)
@@ -1476,7 +1488,7 @@ float time_form(bsam_hier h, int k, int kn, int ns) {
 }
 
 template <class T>
-int tune_level(bsam_hier h, int k, int *best) {
+int tune_level(bsam_hier h, int k, bool with_tiles, int *best) {
   const int p = sizeof(T) == sizeof(float) ? 1 : 0;
   std::vector<int> &rn = h->relax_n[p];
   *best = 1;
@@ -1488,7 +1500,7 @@ int tune_level(bsam_hier h, int k, int *best) {
   // 2,000 cells by the tuner's margin, but not in the cycle, where the first
   // relaxation's fill rides with the restriction (8.1 against 6.5 us there,
   // 10.8 against 8.0 after the correction)
-  if (h->lev[k].tile[p].state == 1) cand.push_back(6);
+  if (with_tiles) cand.push_back(6);
   else if (h->lev[k].dsm_shift[p] >= 0) cand.push_back(5);
   if (cand.size() > 1) {
     time_form<T>(h, k, 1, ns);           // warm-up: the first form timed is not the one that pays for it
@@ -1506,11 +1518,11 @@ int tune_level(bsam_hier h, int k, int *best) {
   return BSAM_OK;
 }
 
-
-uint64_t tune_key(int precision, bool pow2, int chunks) {
+// with_tiles: chosen with the tile form among the candidates
+uint64_t tune_key(int precision, bool pow2, int chunks, bool with_tiles) {
   int b = 0;
   while ((chunks >> (b + 1)) > 0) ++b;
-  return ((uint64_t)precision << 40) | ((uint64_t)pow2 << 32) | (uint64_t)b;
+  return ((uint64_t)with_tiles << 48) | ((uint64_t)precision << 40) | ((uint64_t)pow2 << 32) | (uint64_t)b;
 }
 
 // FP32 arrays of the mixed form: allocated on first use, coefficient copies
@@ -1543,23 +1555,19 @@ int ensure_f32(bsam_hier h) {
   return BSAM_OK;
 }
 
-// the tables of the levels whose form is the tiles; a level that cannot take
-// them runs one launch per colour pass
-int take_tiles(bsam_hier h, int p) {
-  std::vector<int> &rn = h->relax_n[p], levels;
-  for (int k = 2; k <= h->nlev; ++k)
-    if (rn[k] == 6) levels.push_back(k);
-  if (int rc = ensure_tiles(h, levels, p)) return rc;
-  for (int k : levels)
-    if (h->lev[k].tile[p].state != 1) rn[k] = 1;
-  return BSAM_OK;
-}
+void drop_graph(bsam_hier h);
+
+// are the smoother's forms of the present cycle and options chosen
+bool forms_known(bsam_hier h) { return h->tuned[mixed(h) ? 1 : 0] && !h->retune[mixed(h) ? 1 : 0]; }
 
 // cached_only: only if nothing has to be timed
 int autotune(bsam_hier h, bool cached_only = false) {
   const int p = mixed(h) ? 1 : 0;
-  if (h->tuned[p]) return BSAM_OK;
+  if (forms_known(h)) return BSAM_OK;
+  const Synced synced(h);          // forms as a solve runs them, whoever asks
+  drop_graph(h);                   // of the former forms
   h->tuned[p] = true;
+  h->retune[p] = false;
   std::vector<int> &rn = h->relax_n[p];
   rn.assign(h->nlev + 1, 1);
   // the shared-memory form only where the level's Q range fits one cluster
@@ -1568,44 +1576,67 @@ int autotune(bsam_hier h, bool cached_only = false) {
     h->lev[k].dsm_shift[p] = sh;
     return sh >= 0;
   };
+  // the tables of the levels whose form is the tiles; those that cannot take
+  // them go to `without`, with one launch per colour pass
+  auto take_tiles = [&](std::vector<int> &without) {
+    std::vector<int> levels;
+    for (int k = 2; k <= h->nlev; ++k)
+      if (rn[k] == 6) levels.push_back(k);
+    const int rc = ensure_tiles(h, levels, p);
+    for (int k : levels)
+      if (rc || h->lev[k].tile[p].state != 1) {
+        rn[k] = 1;
+        without.push_back(k);
+      }
+    return rc;
+  };
+  std::vector<int> todo;
   if (const char *env = getenv("BSAM_RELAX_N")) {
     int kn = atoi(env);
     if (kn == 0 && cluster_ctas() == 0) kn = 1;
     rn.assign(h->nlev + 1, (kn >= 0 && kn <= 6) ? kn : 1);
     rn[1] = 1;
-    if (kn == 6)
-      if (int rc = take_tiles(h, p)) return rc;
+    if (int rc = take_tiles(todo)) return rc;
     for (int k = 2; k <= h->nlev; ++k)
       if (rn[k] == 5 && !dsm_ok(k)) rn[k] = 1;
     return BSAM_OK;
   }
   // levels already measured on this context (same precision, same h^2 form,
-  // chunk count within a factor of two) take the cached choice
+  // chunk count within a factor of two, the tile form to be had or not) take
+  // the cached choice
   bsam_ctx_s *c = h->ctx;
-  std::vector<int> todo;
-  {
+  auto known = [&](int k, bool with_tiles) {
     std::lock_guard<std::mutex> lk(c->tune_mu);
-    for (int k = 2; k <= h->nlev; ++k) {
-      if (!tunable(h, k)) continue;
-      auto it = c->relax_tune.find(tune_key(p, h->lev[k].pow2, h->lev[k].rc_n));
-      if (it == c->relax_tune.end()) todo.push_back(k);
-      else rn[k] = it->second == 5 && !dsm_ok(k) ? 1 : it->second;
-    }
-  }
-  if (!todo.empty() && cached_only) {
+    auto it = c->relax_tune.find(tune_key(p, h->lev[k].pow2, h->lev[k].rc_n, with_tiles));
+    if (it == c->relax_tune.end()) return false;
+    rn[k] = it->second == 5 && !dsm_ok(k) ? 1 : it->second;
+    return true;
+  };
+  auto later = [&]() {
     h->tuned[p] = false;
     rn.assign(h->nlev + 1, 1);
     return BSAM_OK;
+  };
+  const bool tiles = tiles_apply(h->opts);
+  for (int k = 2; k <= h->nlev; ++k)
+    if (tunable(h, k) && !known(k, tiles)) todo.push_back(k);
+  if (!todo.empty() && cached_only) return later();
+  if (tiles) {
+    if (int rc = ensure_tiles(h, todo, p)) return rc;
+    if (int rc = take_tiles(todo)) return rc;
+    auto has = [&](int k) { return h->lev[k].tile[p].state != 1 && known(k, false); };
+    todo.erase(std::remove_if(todo.begin(), todo.end(), has), todo.end());
   }
-  if (int rc = take_tiles(h, p)) return rc;
   if (todo.empty()) return BSAM_OK;
-  if (int rc = ensure_tiles(h, todo, p)) return rc;
+  if (cached_only) return later();
   // the FP64 smoother runs on the solution itself: keep a copy to put back
   // (the FP32 correction is zeroed at the start of every correction cycle)
   DBuf<double> keep;
   int rc = BSAM_OK;
   if (!p) {
-    if ((rc = keep.alloc(h->Q.n))) return rc;
+    rc = keep.alloc(h->Q.n);
+    if (rc == BSAM_ERR_NOMEM) return later();   // this solve without
+    if (rc) return rc;
     CK(cudaMemcpyAsync(keep.p, h->Q.p, sizeof(double) * h->Q.n, cudaMemcpyDeviceToDevice, h->stream));
   }
   const bool prof = h->profiling;
@@ -1613,10 +1644,11 @@ int autotune(bsam_hier h, bool cached_only = false) {
   h->profiling = false;
   for (int k : todo) {
     int best = 1;
-    rc = p ? tune_level<float>(h, k, &best) : tune_level<double>(h, k, &best);
+    const bool with = tiles && h->lev[k].tile[p].state == 1;
+    rc = p ? tune_level<float>(h, k, with, &best) : tune_level<double>(h, k, with, &best);
     if (rc) break;
     std::lock_guard<std::mutex> lk(c->tune_mu);
-    c->relax_tune[tune_key(p, h->lev[k].pow2, h->lev[k].rc_n)] = best;
+    c->relax_tune[tune_key(p, h->lev[k].pow2, h->lev[k].rc_n, with)] = best;
   }
   h->profiling = prof;
   h->launch_count = lc;
@@ -1628,14 +1660,6 @@ int autotune(bsam_hier h, bool cached_only = false) {
   }
   return rc;
 }
-
-// marks launches of the solve's own flow (copies_synced)
-struct Synced {
-  bsam_hier h;
-  bool was;
-  explicit Synced(bsam_hier h_) : h(h_), was(h_->copies_synced) { h->copies_synced = true; }
-  ~Synced() { h->copies_synced = was; }
-};
 
 int build_graph(bsam_hier h) {
   if (h->gexec) return BSAM_OK;
@@ -2957,6 +2981,7 @@ int bsam_set_opts(bsam_hier h, const bsam_solve_opts *opts) {
               opts->rel_tol == o.rel_tol && opts->precision == o.precision;
   for (const InstRes &r : h->hir) same = same && r.max_vcycles == o.max_vcycles && r.rel_tol == o.rel_tol;
   if (same) return BSAM_OK;
+  if (tiles_apply(*opts) != tiles_apply(o)) h->retune[0] = h->retune[1] = true;
   h->opts = *opts;
   drop_graph(h);
   rc = set_device(h);
@@ -3237,8 +3262,8 @@ int bsam_solve_cycles(bsam_hier h, double *res_hist, int hist_cap, int *vcycles,
   bool on_device = false;
   const Synced synced(h);
   // forms known from other hierarchies of this context: straight to the graph
-  if (!h->tuned[mixed(h) ? 1 : 0] && !host_loop() && (rc = autotune(h, true))) return rc;
-  if (h->tuned[mixed(h) ? 1 : 0] && !host_loop() && build_solve_graph(h)) {
+  if (!host_loop() && (rc = autotune(h, true))) return rc;
+  if (forms_known(h) && !host_loop() && build_solve_graph(h)) {
     // the whole solve in one graph launch (once the smoother is tuned)
     CK(cudaGraphLaunch(h->sexec, h->stream));
     h->solve_graphs++;
@@ -3497,6 +3522,7 @@ int bsam_time_relax(bsam_hier h, int level, int reps, double *us) {
   int rc = set_device(h);
   if (rc || (rc = ensure_f32(h))) return rc;
   if (!h->tuned[mixed(h) ? 1 : 0]) return fail(BSAM_ERR_STATE, "bsam_time_relax: the smoother is not tuned yet");
+  if ((rc = autotune(h))) return rc;         // (options changed since)
   const int ns = std::max(h->opts.npre, 1);
   CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
   const int64_t before = h->launch_count;
