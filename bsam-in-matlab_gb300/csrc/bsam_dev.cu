@@ -624,22 +624,21 @@ void launch_dsm(bsam_hier h, int ctas, size_t smem, Args... args) {
 
 constexpr int64_t kTuneMinCells = 131072;   // large levels: the forms that fill the device
 
-// k_relax_tile's variants may use up to kTileMaxBytes of shared memory
-template <class T, bool kPow2>
-bool tile_attr() {
-  static std::once_flag once;
-  static bool ok = false;
-  std::call_once(once, [] {
-    ok = cudaFuncSetAttribute(k_relax_tile<T, kPow2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              kTileMaxBytes) == cudaSuccess;
-    cudaGetLastError();
-  });
-  return ok;
+// lets level k's k_relax_tile use up to kTileMaxBytes of shared memory on the
+// current device (the limit belongs to a function on one device)
+bool tile_attr(bsam_hier h, int k, int p) {
+  auto set = [](auto kern) {
+    const bool ok =
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileMaxBytes) == cudaSuccess;
+    if (!ok) cudaGetLastError();
+    return ok;
+  };
+  if (p) return h->lev[k].pow2 ? set(k_relax_tile<float, true>) : set(k_relax_tile<float, false>);
+  return h->lev[k].pow2 ? set(k_relax_tile<double, true>) : set(k_relax_tile<double, false>);
 }
 
 template <class T, bool kPow2, class... Args>
 void launch_tile_k(bsam_hier h, int grid, size_t smem, Args... args) {
-  tile_attr<T, kPow2>();
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3(kTileT);
@@ -761,7 +760,8 @@ int end_tiles(bsam_hier h, int p, TileCount &C) {
   P.cap = (P.cap + 3) & ~3;
   P.win_cap = (P.win_cap + 3) & ~3;
   const size_t smem = p ? tile_smem<float>(P.win_cap, P.cap, P.nf_cap) : tile_smem<double>(P.win_cap, P.cap, P.nf_cap);
-  if (!C.hbad && ne < INT32_MAX && nf < INT32_MAX && wq < INT32_MAX && smem <= (size_t)kTileMaxBytes) {
+  if (!C.hbad && ne < INT32_MAX && nf < INT32_MAX && wq < INT32_MAX && smem <= (size_t)kTileMaxBytes &&
+      tile_attr(h, C.k, p)) {
     int rc;
     if ((rc = P.ent.alloc(std::max<size_t>((size_t)ne, 1))) || (rc = P.face.alloc(std::max<size_t>((size_t)nf, 1))) ||
         (rc = P.wq.alloc((size_t)wq)))
