@@ -174,6 +174,10 @@ struct bsam_hier_s {
   std::vector<double> hs;
   std::vector<LevelPlan> lev;     // index 1..nlev
   int64_t n_q = 0, n_cells = 0, n_qc = 0;
+  // the tile form's second copies, behind Q (and E) proper: a copy of the Q
+  // range of the levels that may take the form, at Q + second_home; 0: none
+  int64_t second_n = 0;
+  int second_home = 0;
   int ninst = 1;                   // instances (a single hierarchy is one instance)
   std::vector<int> inst_root, patch_inst;
   std::vector<int64_t> inst_visible;
@@ -672,7 +676,7 @@ int begin_tiles(bsam_hier h, int k, int p, int tw, int th, TileCount &C) {
   C.k = 0;
   P.release();
   P.state = -1;
-  if (tw < 1 || th < 1 || tw > kTileMax || th > kTileMax || 2 * h->n_q > INT32_MAX ||
+  if (tw < 1 || th < 1 || tw > kTileMax || th > kTileMax || !h->second_home ||
       (int64_t)L.rc_n * 2 * kPackRows * kChunk > INT32_MAX)
     return BSAM_OK;
   const int halo = L.qif ? kTileHalo : kTilePasses;
@@ -873,7 +877,7 @@ bool tile_cycle(bsam_hier h, int k) {
 // where level k lives between its two relaxations (FieldsT::lsh)
 template <class T>
 int level_home(bsam_hier h, int k) {
-  return k >= 2 && tile_cycle<T>(h, k) ? (int)h->n_q : 0;
+  return k >= 2 && tile_cycle<T>(h, k) ? h->second_home : 0;
 }
 
 // a relaxation of level k in the tile form: an odd number of launches of an
@@ -890,7 +894,7 @@ void launch_relax_tiles(bsam_hier h, int k, int nsweeps, bool first_fresh, bool 
   const T om = (T)h->opts.omega;
   size_t smem = tile_smem<T>(P.win_cap, P.cap, P.nf_cap);
   if (sizeof(T) == sizeof(double)) smem = tile_request(smem, P.ntiles, sm_count());
-  T *a = f.Q, *b = f.Q + h->n_q;
+  T *a = f.Q, *b = f.Q + h->second_home;
   if (back) std::swap(a, b);
   for (int l = 0, done = 0; l < nl; ++l, std::swap(a, b)) {
     const int passes = 2 * ((nsweeps - done + (nl - l) - 1) / (nl - l));
@@ -931,7 +935,7 @@ void launch_relax(bsam_hier h, int k, int nsweeps, bool first_fresh = false, boo
   const int kn = rn.empty() ? 1 : rn[k];
   if (tile_cycle<T>(h, k)) {   // to the level's second copy (`back`: from it)
     launch_relax_tiles<T>(h, k, nsweeps, first_fresh, back);
-    if (!defer_fill) launch_fill<T>(h, k, 0, back ? 0 : (int)h->n_q);
+    if (!defer_fill) launch_fill<T>(h, k, 0, back ? 0 : h->second_home);
     return;
   }
   if (kn == 5) {   // the whole relaxation (and its fill) in one cluster launch, solution in shared memory
@@ -1531,7 +1535,7 @@ int ensure_f32(bsam_hier h) {
   if (!mixed(h)) return BSAM_OK;
   int rc;
   if (!h->E.p) {
-    if ((rc = h->E.alloc(h->Q.n, h->Q.n)) || (rc = h->F32.alloc(h->F.n)) || (rc = h->QC32.alloc(std::max<size_t>(h->QC.n, 1))) ||
+    if ((rc = h->E.alloc(h->Q.n, (size_t)h->second_n)) || (rc = h->F32.alloc(h->F.n)) || (rc = h->QC32.alloc(std::max<size_t>(h->QC.n, 1))) ||
         (rc = h->DeW32.alloc(h->DeW.n)) || (rc = h->DnS32.alloc(h->DnS.n)) || (rc = h->CC32.alloc(h->CC.n)) ||
         (rc = h->ID32.alloc(h->ID.n)) || (rc = h->pcoef32.alloc(std::max<size_t>(h->pcoef.n, 1))) ||
         (rc = h->cfd32.alloc(std::max<size_t>(h->cfd.n, 1))) || (rc = h->bcg32.alloc(std::max<size_t>(h->bcg.n, 1))) ||
@@ -2297,6 +2301,24 @@ CorrRec corr_rec(const int32_t *r, const int32_t *win, int fc, int j) {
   return c;
 }
 
+// room for the second copies of the levels below kTuneMinCells cells (a
+// uniform 1024^2 hierarchy: 9% of Q; all of it before)
+void second_copies(bsam_hier h, const bsam_hier_desc *d) {
+  int64_t lo = INT64_MAX, hi = 0;
+  for (int k = 2; k <= d->nlev; ++k) {
+    const int32_t *L = d->levels + (size_t)(k - 1) * LDN;
+    if (L[LD_CELL1] - L[LD_CELL0] >= kTuneMinCells) continue;
+    for (int p = L[LD_P0]; p < L[LD_P1]; ++p) {
+      const int32_t *r = d->patches + (size_t)p * PDN;
+      lo = std::min<int64_t>(lo, r[PD_QOFF]);
+      hi = std::max<int64_t>(hi, r[PD_QOFF] + (int64_t)(r[PD_MX] + 2) * (r[PD_MY] + 2));
+    }
+  }
+  if (hi <= lo || d->n_q + (hi - lo) > INT32_MAX || d->n_q == lo) return;
+  h->second_n = hi - lo;
+  h->second_home = (int)(d->n_q - lo);
+}
+
 int do_upload(bsam_hier h, const bsam_hier_desc *d) {
   int rc = validate(d);
   if (rc) return rc;
@@ -2323,7 +2345,8 @@ int do_upload(bsam_hier h, const bsam_hier_desc *d) {
     const int32_t *r1 = d->patches + (size_t)i * PDN;
     asz += (int64_t)r1[PD_MX] * r1[PD_MY] * r1[PD_MX] * r1[PD_MY];
   }
-  if ((rc = h->Q.upload(d->Q, d->n_q, s, d->n_q)) || (rc = h->F.upload(d->F, d->n_cells, s)) ||
+  second_copies(h, d);
+  if ((rc = h->Q.upload(d->Q, d->n_q, s, (size_t)h->second_n)) || (rc = h->F.upload(d->F, d->n_cells, s)) ||
       (rc = h->FTrue.upload(d->FTrue, d->n_cells, s)) || (rc = h->CC.upload(d->CC, d->n_cells, s)) ||
       (rc = h->ID.upload(d->InvDiagS, d->n_cells, s)) || (rc = h->DeW.upload(d->DeW, d->n_dew, s)) ||
       (rc = h->DnS.upload(d->DnS, d->n_dns, s)) || (rc = h->QC.upload(d->QC, d->n_qc, s)) ||
