@@ -253,10 +253,8 @@ struct bsam_hier_s {
   struct Rec { int kind; cudaEvent_t a, b; double bytes; };
   std::vector<Rec> recs;
   int64_t launch_count = 0;
-  int64_t graph_launches = 0;
-  int64_t while_bodies = 0;        // iterations run inside WHILE graphs
-  int64_t solve_graphs = 0;        // solves run as one graph launch
-  int64_t preamble_kernels = 0;    // kernels of such a solve before its loop
+  int64_t outer_kernels = 0;       // kernels of a solve's one graph outside its conditional bodies
+  int64_t rhs_kernels = 0;         // and of its IF body
   // per precision and level: colour cells per smoother thread (1, 2, 4),
   // picked by the autotuner at the first solve (result-neutral)
   std::vector<int> relax_n[2];
@@ -1671,11 +1669,13 @@ int build_graph(bsam_hier h) {
   CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
   const int64_t before = h->launch_count;
   int rc = launch_iteration(h, RES_STEP);
+  const int64_t kernels = h->launch_count - before;
+  h->launch_count = before;                  // captured, not launched
   cudaGraph_t g = nullptr;
   cudaError_t e = cudaStreamEndCapture(h->stream, &g);
   if (rc) return rc;
   if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture");
-  h->kernels_per_cycle = h->launch_count - before;
+  h->kernels_per_cycle = kernels;
   h->graph = g;
   CK(cudaGraphInstantiate(&h->gexec, g, 0));
   return BSAM_OK;
@@ -1818,18 +1818,26 @@ bool build_solve_graph(bsam_hier h) {
       if (!mixed(h)) reset_force(h);
       for (int k = 1; k <= h->nlev; ++k) launch_fill(h, k);
       launch_residual(h, RES_START, LoopCond{wcond, icond, mixed(h) ? 2 : 1});
-      h->preamble_kernels = h->launch_count - before;
+      h->outer_kernels = h->launch_count - before;
+      h->rhs_kernels = 0;
       if (mixed(h))
         ok = add_conditional(h, helper, icond, cudaGraphCondTypeIf, [h]() {
+          const int64_t n = h->launch_count;
           launch_consistent(h);
           launch_residual(h, RES_RHS);
+          h->rhs_kernels = h->launch_count - n;
           return cudaGetLastError() == cudaSuccess ? BSAM_OK : BSAM_ERR_CUDA;
         });
       if (ok)
         ok = add_conditional(h, helper, wcond, cudaGraphCondTypeWhile, [h, wcond]() {
-          return launch_iteration(h, RES_STEP, LoopCond{wcond, wcond, 1});
+          const int64_t n = h->launch_count;
+          const int rc = launch_iteration(h, RES_STEP, LoopCond{wcond, wcond, 1});
+          h->kernels_per_cycle = h->launch_count - n;
+          return rc;
         });
+      const int64_t n = h->launch_count;
       if (ok) launch_qc_refresh(h);
+      h->outer_kernels += h->launch_count - n;
     }
     cudaGraph_t g = nullptr;
     const bool ended = cudaStreamEndCapture(h->stream, &g) == cudaSuccess;
@@ -3289,10 +3297,12 @@ int bsam_solve_cycles(bsam_hier h, double *res_hist, int hist_cap, int *vcycles,
   if (forms_known(h) && !host_loop() && build_solve_graph(h)) {
     // the whole solve in one graph launch (once the smoother is tuned)
     CK(cudaGraphLaunch(h->sexec, h->stream));
-    h->solve_graphs++;
+    h->launch_count += h->outer_kernels;
     if ((rc = read_state(h, &nactive))) return rc;
     on_device = true;
-    return finish_solve(h, on_device, res_hist, hist_cap, vcycles, final_rel, visible_cells);
+    rc = finish_solve(h, on_device, res_hist, hist_cap, vcycles, final_rel, visible_cells);
+    if (!rc && *std::max_element(h->res_iters.begin(), h->res_iters.end()) > 0) h->launch_count += h->rhs_kernels;
+    return rc;
   }
   if (!mixed(h)) reset_force(h);
   for (int k = 1; k <= h->nlev; ++k) launch_fill(h, k);
@@ -3318,7 +3328,7 @@ int bsam_solve_cycles(bsam_hier h, double *res_hist, int hist_cap, int *vcycles,
   if (nactive && (rc = build_graph(h))) return rc;
   while (nactive) {
     CK(cudaGraphLaunch(h->gexec, h->stream));
-    h->graph_launches++;
+    h->launch_count += h->kernels_per_cycle;
     if ((rc = read_state(h, &nactive))) return rc;
   }
   launch_qc_refresh(h);
@@ -3340,7 +3350,7 @@ static int finish_solve(bsam_hier h, bool on_device, double *res_hist, int hist_
   CK(cudaMemcpyAsync(h->active.p, h->ones.p, sizeof(int) * h->ninst, cudaMemcpyDeviceToDevice, h->stream));
   if (h->act_mode == kActChunk) CK(cudaMemsetAsync(h->cact.p, 1, h->cact.n, h->stream));
   CK(cudaStreamSynchronize(h->stream));
-  if (on_device) h->while_bodies += *std::max_element(h->res_iters.begin(), h->res_iters.end());
+  if (on_device) h->launch_count += h->kernels_per_cycle * *std::max_element(h->res_iters.begin(), h->res_iters.end());
   return bsam_batch_result(h, 0, res_hist, hist_cap, vcycles, final_rel, visible_cells);
 }
 
@@ -3512,8 +3522,7 @@ int bsam_restore_state(bsam_hier h) {
 
 int bsam_launch_count(bsam_hier h, int64_t *count) {
   if (!h || !count) return fail(BSAM_ERR_ARG, "null argument");
-  *count = h->launch_count + h->graph_launches * h->kernels_per_cycle + h->while_bodies * h->kernels_per_cycle +
-           h->solve_graphs * (h->preamble_kernels + 1);
+  *count = h->launch_count;
   return BSAM_OK;
 }
 
