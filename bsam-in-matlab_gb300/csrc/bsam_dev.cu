@@ -3597,19 +3597,32 @@ int bsam_profile_vcycles(bsam_hier h, int ncycles, int level, double ms[BSAM_NKI
   int rc = set_device(h);
   if (rc) return rc;
   for (int i = 0; i < BSAM_NKINDS; ++i) { ms[i] = 0; launches[i] = 0; bytes[i] = 0; }
-  if ((rc = ensure_f32(h))) return rc;
+  if ((rc = ensure_f32(h)) || (rc = autotune(h))) return rc;
+  // the solve's own flow, every instance kept active
+  const Synced synced(h);
+  auto go_on = [&]() -> int {
+    CK(cudaMemcpyAsync(h->active.p, h->ones.p, sizeof(int) * h->ninst, cudaMemcpyDeviceToDevice, h->stream));
+    CK(cudaMemsetAsync(h->iters.p, 0, sizeof(int) * h->ninst, h->stream));
+    if (h->act_mode == kActChunk) CK(cudaMemsetAsync(h->cact.p, 1, h->cact.n, h->stream));
+    return BSAM_OK;
+  };
+  if (!mixed(h)) reset_force(h);
+  for (int k = 1; k <= h->nlev; ++k) launch_fill(h, k);
+  launch_residual(h, RES_START);
+  if ((rc = go_on())) return rc;
   if (mixed(h)) {
     launch_consistent(h);
     launch_residual(h, RES_RHS);
-  } else {
-    reset_force(h);
   }
-  if ((rc = autotune(h))) return rc;
-  h->profiling = true;
   h->profile_level = level;
   h->recs.clear();
-  for (int c = 0; c < ncycles && !rc; ++c) rc = launch_iteration(h, RES_REPORT);
-  h->profiling = false;
+  for (int c = 0; c < ncycles && !rc; ++c) {
+    h->profiling = true;
+    rc = launch_iteration(h, RES_STEP);
+    h->profiling = false;
+    if (!rc) rc = go_on();
+  }
+  launch_qc_refresh(h);
   cudaError_t e = cudaStreamSynchronize(h->stream);
   for (auto &r : h->recs) {
     float t = 0;

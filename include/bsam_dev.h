@@ -232,8 +232,9 @@ int bsam_mass_check(bsam_hier h, double out[4]);
 
 /* Measurement support (no reference counterpart): the CUDA stream the
  * hierarchy's kernels run on (a cudaStream_t), and per-kernel device times
- * of `ncycles` eagerly launched V-cycles, each kernel bracketed by CUDA
- * events on that stream, restricted to the kernels of one level (level 0:
+ * of `ncycles` V-cycles as a solve runs them (its fills and first residual
+ * before them, its launch forms), launched one by one, each kernel bracketed
+ * by CUDA events on that stream, restricted to the kernels of one level (level 0:
  * all; the residual counts as level 0 only).  kinds: 0 relax, 1 ghost fill,
  * 2 restrict, 3 ring, 4 coarse load, 5 flux corrections, 6 prolong-correct,
  * 7 coarsest, 8 residual; ms[k] = total ms, launches[k], bytes[k] =
