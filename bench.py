@@ -251,7 +251,8 @@ def mixed_form(backend, fl, opts, ref_Q, steps, warmup, flush, local):
     return {'value': steps / (ms.sum() / 1e3), 'unit': 'solves/s', 'ms_per_solve': float(ms.mean()),
             'p50_ms': float(np.percentile(ms, 50)), 'p99_ms': float(np.percentile(ms, 99)),
             'vcycles': r[0], 'final_rel': r[2], 'rel_l2_vs_fp64': l2, 'rel_max_vs_fp64': mx,
-            'relax_cells_per_thread': dh.relax_tuning(1).tolist(), 'kernels_per_vcycle': dh.kernels_per_vcycle(),
+            'relax_cells_per_thread': dh.relax_tuning(1).tolist(), 'relax_tiles': dh.relax_tiles(1).tolist(),
+            'kernels_per_vcycle': dh.kernels_per_vcycle(),
             'dtype': 'f32 smoothing / f64 defect correction',
             'note': 'error against the FP64 path, which equals the C oracle bit for bit'}
 
@@ -330,7 +331,8 @@ def batched_form(backend, n, steps, warmup, flush, local, dist=None):
         d = {'value': rate, 'unit': 'solves/s', 'ms_per_batch': 1e3 * tmax / steps,
              'p50_ms': float(np.percentile(ms, 50)), 'p99_ms': float(np.percentile(ms, 99)),
              'vcycles_slowest': maxit, 'kernels_per_vcycle': bh.kernels_per_vcycle(),
-             'relax_cells_per_thread': bh.relax_tuning(1 if prec == 'mixed' else 0).tolist()}
+             'relax_cells_per_thread': bh.relax_tuning(1 if prec == 'mixed' else 0).tolist(),
+             'relax_tiles': bh.relax_tiles(1 if prec == 'mixed' else 0).tolist()}
         # smoother roofline per merged level (levels larger than L2 here)
         peak, peak_kind = load_peaks()
         from bsam.device import fp64_rate
@@ -518,11 +520,12 @@ def main():
         dh.restore_state()
         torch.cuda.synchronize()
         torch.cuda.profiler.start()
-        dh.vcycle()
+        dh.profile(1)            # the solve's V-cycle, launch by launch
         torch.cuda.synchronize()
         torch.cuda.profiler.stop()
         print(json.dumps({'eager_vcycle': 'done', 'precision': args.eager_vcycle, 'levels': H.nlev,
                           'kernels': dh.kernels_per_vcycle(), 'relax_forms': dh.relax_tuning(
+                              1 if args.eager_vcycle == 'mixed' else 0).tolist(), 'relax_tiles': dh.relax_tiles(
                               1 if args.eager_vcycle == 'mixed' else 0).tolist()}), flush=True)
         return
     dh.save_state()
@@ -657,7 +660,8 @@ def main():
                        'final_rel': rel, 'visible_cells': vis, 'stored_cells': int(fl.F.size - 0),
                        'p50_ms': float(np.percentile(per, 50)), 'p99_ms': float(np.percentile(per, 99)),
                        'kernels_per_vcycle': dh.kernels_per_vcycle(), 'per_kernel': per_kind,
-                       'relax_cells_per_thread': dh.relax_tuning(0).tolist()},
+                       'relax_cells_per_thread': dh.relax_tuning(0).tolist(),
+                       'relax_tiles': dh.relax_tiles(0).tolist()},
             'e2e': {'value': e2e_value, 'unit': 'solves/s',
                     'h2d_bytes_per_step': int(8 * (Q0.size + F0.size)),
                     'd2h_bytes_per_step': int(8 * Qout.size + hist_bytes),

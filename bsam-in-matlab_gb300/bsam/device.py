@@ -96,6 +96,7 @@ def lib():
         L.bsam_restore_state.argtypes = [P]
         L.bsam_launch_count.argtypes = [P, C.POINTER(I64)]
         L.bsam_relax_tuning.argtypes = [P, C.c_int, P, C.c_int]
+        L.bsam_relax_tiles.argtypes = [P, C.c_int, P, C.c_int]
         L.bsam_batch_result.argtypes = [P, C.c_int, P, C.c_int, C.POINTER(C.c_int), C.POINTER(D), C.POINTER(I64)]
         L.bsam_batch_set_stop.argtypes = [P, C.c_int, C.c_int, D]
         L.bsam_polygon_dist2.argtypes = [P, P, C.c_int, P, P, P, I64]
@@ -352,11 +353,18 @@ class DevHier:
 
     def relax_tuning(self, precision=0):
         """Smoother launch form per level 1..nlev as tuned: colour cells per
-        thread (1, 2, 4), 3 persistent blocks, 0 the single-cluster launch, 5
+        thread (1, 2, 4; 1 on tiles too, see relax_tiles), 3 persistent blocks, 0 the single-cluster launch, 5
         the single-cluster launch with the level's solution in distributed
         shared memory, -1 not yet run."""
         out = np.zeros(int(self.fl.nlev), np.int32)
         check(lib().bsam_relax_tuning(self.h, int(precision), out.ctypes.data, out.size))
+        return out
+
+    def relax_tiles(self, precision=0):
+        """Per level 1..nlev: 1 where a solve's relaxations run on tiles, -1
+        not yet run."""
+        out = np.zeros(int(self.fl.nlev), np.int32)
+        check(lib().bsam_relax_tiles(self.h, int(precision), out.ctypes.data, out.size))
         return out
 
     def kernels_per_vcycle(self):

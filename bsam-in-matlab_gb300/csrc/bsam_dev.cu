@@ -3535,6 +3535,15 @@ int bsam_relax_tuning(bsam_hier h, int precision, int32_t *cells_per_thread, int
   return BSAM_OK;
 }
 
+int bsam_relax_tiles(bsam_hier h, int precision, int32_t *on_tiles, int cap) {
+  if (!h || !on_tiles) return fail(BSAM_ERR_ARG, "null argument");
+  if (precision != 0 && precision != 1) return fail(BSAM_ERR_ARG, "precision must be 0 or 1");
+  const Synced synced(h);
+  for (int k = 1; k <= h->nlev && k <= cap; ++k)
+    on_tiles[k - 1] = !h->tuned[precision] ? -1 : k >= 2 && (precision ? tile_cycle<float>(h, k) : tile_cycle<double>(h, k));
+  return BSAM_OK;
+}
+
 int bsam_stream(bsam_hier h, void **stream) {
   if (!h || !stream) return fail(BSAM_ERR_ARG, "null argument");
   *stream = (void *)h->stream;

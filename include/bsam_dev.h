@@ -284,6 +284,12 @@ int bsam_launch_count(bsam_hier h, int64_t *count);
  * order).                                                                 */
 int bsam_relax_tuning(bsam_hier h, int precision, int32_t *cells_per_thread, int cap);
 
+/* on_tiles[k-1]: 1 where level k's relaxations run on tiles in a solve with
+ * the present options (the tuner's choice or BSAM_RELAX_N=6, the tables there,
+ * sweeps on either side), else 0; -1 where that cycle has not run yet.  No
+ * reference counterpart.                                                  */
+int bsam_relax_tiles(bsam_hier h, int precision, int32_t *on_tiles, int cap);
+
 /* Number of kernels one V-cycle (+ fill-down + residual) launches. */
 int bsam_kernels_per_vcycle(bsam_hier h, int64_t *count);
 
