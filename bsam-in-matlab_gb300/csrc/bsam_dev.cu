@@ -2310,7 +2310,9 @@ CorrRec corr_rec(const int32_t *r, const int32_t *win, int fc, int j) {
 }
 
 // room for the second copies of the levels below kTuneMinCells cells (a
-// uniform 1024^2 hierarchy: 6% of Q, the starfish: 30%)
+// uniform 1024^2 hierarchy: 6% of Q, the starfish: 30%), a whole number of
+// lines from the first copies, so that a level's rows meet the same lines in
+// both (starfish solve 3.137 ms with any distance, 3.120 with this)
 void second_copies(bsam_hier h, const bsam_hier_desc *d) {
   int64_t lo = INT64_MAX, hi = 0;
   for (int k = 2; k <= d->nlev; ++k) {
@@ -2322,9 +2324,11 @@ void second_copies(bsam_hier h, const bsam_hier_desc *d) {
       hi = std::max<int64_t>(hi, r[PD_QOFF] + (int64_t)(r[PD_MX] + 2) * (r[PD_MY] + 2));
     }
   }
-  if (hi <= lo || d->n_q + (hi - lo) > INT32_MAX || d->n_q == lo) return;
-  h->second_n = hi - lo;
-  h->second_home = (int)(d->n_q - lo);
+  if (hi <= lo || d->n_q == lo) return;
+  const int64_t home = (d->n_q - lo + 31) & ~(int64_t)31;
+  if (home + hi > INT32_MAX) return;
+  h->second_n = home + hi - d->n_q;
+  h->second_home = (int)home;
 }
 
 int do_upload(bsam_hier h, const bsam_hier_desc *d) {
